@@ -45,8 +45,9 @@ typedef struct tfim_ctx tfim_ctx;
 #define TFIM_COUNTER_AUTO    0   /* chosen per job from its shape */
 #define TFIM_COUNTER_LOP3    1   /* AND + popc on CUDA cores */
 #define TFIM_COUNTER_TENSOR  2   /* b1 AND+POPC tensor-core MMA */
-#define TFIM_COUNTER_I8      4   /* tcgen05.mma kind::i8 on the bits expanded to bytes
-                                    (tfim_count_wave only) */
+#define TFIM_COUNTER_I8      4   /* tcgen05 tensor-core tiles: waves and the empty prefix's family
+                                    on the bits expanded to 4-bit values (kind::mxf4), other
+                                    families expanded to bytes (kind::i8) */
 #define TFIM_COUNTER_PROJ    3   /* resident engine: projected counting (prefix transactions x
                                     the reduced transaction list) wherever it applies, else auto */
 
@@ -335,10 +336,10 @@ typedef struct {
     double  rate_b1_bitops;     /* cost model of the empty-prefix family: b1 bit-ops/s, */
     double  rate_lop3_bitops;   /*   LOP3 bit-ops/s, */
     double  rate_pair_incr;     /*   pair co-occurrence increments/s */
-    int32_t i8_min_rows;        /* automatic choice: the tcgen05 kind::i8 counter for count jobs */
+    int32_t i8_min_rows;        /* automatic choice: the tcgen05 wave counter for count jobs */
     int32_t i8_min_cols;        /*   of at least i8_min_rows x i8_min_cols (tfim_count_wave and
                                      the empty-prefix family's bitmap Gram) */
-    double  rate_i8_bitops;     /* cost model: tcgen05 kind::i8 bit-ops/s */
+    double  rate_i8_bitops;     /* cost model: tcgen05 wave counter bit-ops/s */
     int32_t tc_min_work;        /* automatic choice: the tcgen05 family counter for family jobs of
                                    at most 128 columns with rows x columns >= tc_min_work and a */
     float   tc_min_density;     /*   prefix holding at least this fraction of 128-bit positions */

@@ -12,8 +12,8 @@ Parameters (the tfim_tuning table of include/tfim.h):
   * rate_b1_bitops, rate_lop3_bitops, rate_i8_bitops: bit-ops/s of one 256-node x 512-item
     counting wave over a random half-dense bitmap of 2^18 transactions, each counter forced
     (tensorfim_b200.countbench);
-  * i8_min_rows = i8_min_cols: the square wave size from which the tcgen05 kind::i8 counter
-    beats the b1 counter (waves of m x m over 2^20 transactions);
+  * i8_min_rows: the wave size from which the tcgen05 counter beats the CUDA-core and b1
+    counters (waves of m prefixes x 512 items over 2^20 transactions; i8_min_cols = 1);
   * rate_pair_incr: pair increments/s of the empty-prefix family counted by pair
     co-occurrence on configuration 4 (sum over reduced rows of len^2/2 over its time).
 Every mine of the sweep is checked against the first one: the table changes speed, never
@@ -74,16 +74,16 @@ def _bit_rates(reps: int) -> dict:
 
 
 def _i8_crossover(reps: int) -> tuple[int, list]:
-    """Smallest square wave size m (b = d = m nodes x items, 2^20 transactions) from which the
-    tcgen05 kind::i8 counter beats the b1 counter at every larger size measured."""
+    """Smallest wave of m nodes (x 512 items over 2^20 transactions) from which the tcgen05
+    counter beats the CUDA-core and b1 counters at every larger size measured."""
     from . import countbench
     rec = []
-    for m in (32, 64, 96, 128, 192, 256, 384):
-        r = countbench.run(m, m, 1 << 20, counters=("tensor", "i8"), reps=reps)["counters"]
-        rec.append([m, r["tensor"]["seconds"], r["i8"]["seconds"]])
+    for m in (1, 2, 3, 4, 8, 16, 32, 64, 128, 256):
+        r = countbench.run(m, 512, 1 << 20, counters=("lop3", "tensor", "i8"), reps=reps)["counters"]
+        rec.append([m, r["lop3"]["seconds"], r["tensor"]["seconds"], r["i8"]["seconds"]])
     best = rec[-1][0] * 2
-    for m, t_b1, t_i8 in reversed(rec):
-        if t_i8 < t_b1:
+    for m, t_l3, t_b1, t_i8 in reversed(rec):
+        if t_i8 < min(t_l3, t_b1):
             best = m
         else:
             break
@@ -148,7 +148,7 @@ def main() -> None:
              "b1_tiles_per_sm": float(best["b1_tiles_per_sm"]), "b1_min_rows": int(best["b1_min"]),
              "b1_min_cols": int(best["b1_min"]), "proj_auto": int(start["proj_auto"]),
              "rate_b1_bitops": float(rates["rate_b1_bitops"]), "rate_lop3_bitops": float(rates["rate_lop3_bitops"]),
-             "rate_pair_incr": float(rates["rate_pair_incr"]), "i8_min_rows": int(i8_min), "i8_min_cols": int(i8_min),
+             "rate_pair_incr": float(rates["rate_pair_incr"]), "i8_min_rows": int(i8_min), "i8_min_cols": 1,
              "rate_i8_bitops": float(rates["rate_i8_bitops"]),
              "l3_dense_slices_per_sm": float(best["l3_dense_slices_per_sm"])}
     for k in ("tc_min_work", "tc_min_density", "tc_tiles_per_sm", "gram_min_rows"):   # not swept here
@@ -161,7 +161,7 @@ def main() -> None:
     doc["sweep_columns"] = ["value", "sum_ms"] + [n for n, _ in dbs]
     for k, rec in sweeps.items():
         doc["sweep:" + k] = rec
-    doc["sweep:i8_crossover"] = {"columns": ["m", "b1_seconds", "i8_seconds"], "rows": i8_rec}
+    doc["sweep:i8_crossover"] = {"columns": ["m", "lop3_seconds", "b1_seconds", "i8_seconds"], "rows": i8_rec}
     doc["seconds"] = round(time.time() - t0, 1)
     with open(a.out, "w") as f:
         json.dump(doc, f, indent=1)

@@ -95,8 +95,13 @@ int count_wave_impl(tfim_ctx* c, int32_t b, int32_t min_count, const int32_t* d_
     // host-built job/tile tables (independent of the list contents)
     const int32_t counter = c->counter_pref;
     const tfim_tuning tn = tuning();
+    // One or two rows over a long bitmap stay on the CUDA-core tiles: the tensor tiles read every
+    // column word whatever the row masks hold (1 row x 6,162 long-tail items x 1M transactions:
+    // 377 us against 130), while up to 2^14 words the call is launch-bound and the tensor tiles are
+    // the shorter launch (1 row x 69 items x 262,144 transactions: 49 us against 80).
     const bool i8 = counter == TFIM_COUNTER_I8 ||
-                    (counter == TFIM_COUNTER_AUTO && b >= tn.i8_min_rows && d >= tn.i8_min_cols);
+                    (counter == TFIM_COUNTER_AUTO && d >= tn.i8_min_cols &&
+                     (b >= tn.i8_min_rows || c->W <= (1 << 14)));
     const bool b1 = !i8 && (counter == TFIM_COUNTER_TENSOR ||
                             (counter == TFIM_COUNTER_AUTO && b >= tn.b1_min_rows && d >= tn.b1_min_cols));
     std::vector<JobDesc> jobs(1);
@@ -110,17 +115,7 @@ int count_wave_impl(tfim_ctx* c, int32_t b, int32_t min_count, const int32_t* d_
     std::vector<TileDesc> tiles;
     const int64_t W = c->W;
     if (i8) {
-        // 128 x 128 tiles, word slices of 64-word multiples
-        const int64_t base = (int64_t)((b + 127) / 128) * ((d + 127) / 128);
-        const int64_t want = (int64_t)(tn.b1_tiles_per_sm * 148);
-        int64_t ks = std::max<int64_t>(1, (want + base - 1) / base);
-        ks = std::min<int64_t>(ks, W / 64);
-        const int64_t kslice = ((W / 64 + ks - 1) / ks) * 64;
-        for (int64_t w0 = 0; w0 < W; w0 += kslice)
-            for (int32_t r0 = 0; r0 < b; r0 += 128)
-                for (int32_t c0 = 0; c0 < d; c0 += 128)
-                    tiles.push_back(TileDesc{0, r0, std::min(128, b - r0), c0, std::min(d, c0 + 128), (int32_t)w0,
-                                             (int32_t)std::min<int64_t>(W, w0 + kslice), 0});
+        tiles_f4(0, b, d, W, 148, tiles);
     } else if (b1) {
         const int64_t base = (int64_t)((b + kB1Rows - 1) / kB1Rows) * ((d + kB1Cols - 1) / kB1Cols);
         const int64_t want = (int64_t)(tn.b1_tiles_per_sm * 148);
@@ -162,13 +157,14 @@ int count_wave_impl(tfim_ctx* c, int32_t b, int32_t min_count, const int32_t* d_
     a.bitmap = c->d_bitmap; a.W = W; a.masks = c->d_masks.as<uint32_t>();
     a.jobs = (const JobDesc*)dp; a.rows = (const RowDesc*)(dp + o_rows); a.cols = (const int32_t*)(dp + o_cols);
     a.tiles = (const TileDesc*)(dp + o_tiles); a.n_tiles = (int32_t)tiles.size(); a.out = d_counts;
-    c->used_i8 = i8;
-    TFIM_TRY(i8 ? launch_count_i8(a, s) : b1 ? launch_count_b1(a, s) : launch_count_lop3(a, s));
+    if (i8) TFIM_TRY(c->h_flags.reserve(64));
+    TFIM_TRY(i8 ? launch_count_f4(a, s) : b1 ? launch_count_b1(a, s) : launch_count_lop3(a, s));
     TFIM_TRY(group_reduce(c, d_counts, (int64_t)b * d, TFIM_DT_I32, TFIM_RED_SUM, s));
     TFIM_TRY(launch_nfreq(d_counts, b, d, min_count, d_nfreq, s));
+    if (i8) TFIM_TRY(count_f4_status_fetch(c->h_flags.as<int32_t>(), s));
     // the host staging buffer may be reused by the next call only after this copy ran
     TFIM_CUDA(cudaStreamSynchronize(s));
-    return TFIM_OK;
+    return i8 ? count_f4_status_check(*c->h_flags.as<int32_t>()) : TFIM_OK;
 }
 
 namespace {
@@ -418,7 +414,6 @@ int tfim_count_wave(tfim_ctx* c, const int32_t* item_lists, const int64_t* list_
     TFIM_CUDA(cudaMemcpyAsync(counts_out, dp + o_counts, (size_t)b * d * 4, cudaMemcpyDeviceToHost, s));
     TFIM_CUDA(cudaMemcpyAsync(nfreq_out, dp + o_nfreq, (size_t)b * 4, cudaMemcpyDeviceToHost, s));
     TFIM_CUDA(cudaStreamSynchronize(s));
-    if (c->used_i8) TFIM_TRY(count_i8_status(true));
     return TFIM_OK;
 }
 
@@ -630,6 +625,7 @@ void tfim_close(tfim_ctx* c) {
     tfim::dev_free(c->d_red_items, c->stream);
     for (auto& b : c->d_scratch) b.release();
     for (auto& b : c->h_scratch) b.release();
+    c->h_flags.release();
     c->d_masks.release();
     c->d_group.release();
     if (c->stream) cudaStreamSynchronize(c->stream);

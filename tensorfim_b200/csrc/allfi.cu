@@ -94,7 +94,6 @@ int tfim_mine_all(tfim_ctx* c, int32_t min_count, int32_t max_len, int64_t max_i
     TFIM_CUDA(cudaEventCreate(&e0));
     TFIM_CUDA(cudaEventCreate(&e1));
     int rc = TFIM_OK;
-    bool any_i8 = false;
     for (int32_t k = 2; k <= max_len && !cur.empty() && rc == TFIM_OK; k++) {
         const int32_t plen = k - 1;
         const int64_t n_pref = (int64_t)cur.size() / plen;
@@ -118,7 +117,6 @@ int tfim_mine_all(tfim_ctx* c, int32_t min_count, int32_t max_len, int64_t max_i
             int64_t* doff = (int64_t*)(d_aux.as<unsigned char>() + (((size_t)b * 4 + 15) & ~size_t(15)));
             cudaEventRecord(e0, s);
             if ((rc = count_wave_impl(c, b, min_count, di, dm, dc, dn, s))) break;
-            any_i8 |= c->used_i8;
             cudaEventRecord(e1, s);
             const unsigned grid = (unsigned)(((int64_t)b * 32 + 255) / 256);
             k_ext_count<<<grid, 256, 0, s>>>(dc, b, d, min_count, dm, di, dn);
@@ -164,7 +162,6 @@ int tfim_mine_all(tfim_ctx* c, int32_t min_count, int32_t max_len, int64_t max_i
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    if (rc == TFIM_OK && any_i8) rc = count_i8_status(true);
     if (rc != TFIM_OK) {
         if (rc == TFIM_E_CUDA) set_error("all-itemset mining: %s", cudaGetErrorString(cudaGetLastError()));
         A.clear();

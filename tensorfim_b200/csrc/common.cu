@@ -156,9 +156,9 @@ void tuning_builtin(tfim_tuning* t) {
     t->rate_b1_bitops = kTuneB1BitOps;
     t->rate_lop3_bitops = kTuneLop3BitOps;
     t->rate_pair_incr = kTunePairIncrements;
-    t->i8_min_rows = 128;
-    t->i8_min_cols = 128;
-    t->rate_i8_bitops = 3.0e14;
+    t->i8_min_rows = 3;
+    t->i8_min_cols = 1;
+    t->rate_i8_bitops = 2.0e15;
     t->tc_min_work = 1536;
     t->tc_min_density = 0.5f;
     t->tc_tiles_per_sm = 8.f;

@@ -1,0 +1,441 @@
+// Tensor-core wave counter on the 5th-generation tensor cores: tcgen05.mma kind::mxf4 on the
+// bits expanded to 4-bit values.
+//
+// The AND+popc block of a count job, popc(A_r & B_c), is the dot product of the rows' 0/1
+// vectors.  This counter expands bits to e2m1 values in shared memory and multiplies them
+// with tcgen05.mma.cta_group::1.kind::mxf4 into a 128 x 256 accumulator in tensor memory.  The
+// arithmetic is the reference's (a support is a popcount of ANDed bit rows,
+// code/engine/src/kernel_bmma.cu:636-768, there computed by WMMA b1).  It is exact: every product
+// is 0 or 1, the accumulator is FP32, and a tile covers at most 2^23 transactions, so every
+// partial sum is an integer below 2^24; partial sums of different tiles meet in int32.
+//
+// Expansion without shifts per bit: the nibble masks 0x1, 0x2 and 0x4 of a word pick bits as
+// the e2m1 values 0.5, 1 and 2, and (word >> 1) & 0x4 picks the last bit as 2.  All 16-byte
+// chunks of one MMA (K = 64) hold the same value, and the block scale factors (2, 1, 1/2 on
+// both operands) bring its products back to 0 or 1.  A scale region of tensor memory holds
+// one value in every byte, so it does not depend on the scale factors' layout.
+//
+// Tile (TileDesc): columns [c0, c1) (at most 128, the accumulator's lanes) x rows
+// [r0, r0 + nr) (at most 256, its columns) over words [w0, w1), one CTA.  A chunk is 512 bits of
+// K: two K blocks of (columns + N) rows x 128 bytes in the K-major 128-byte-swizzle layout.  A
+// stage is 1, 2 or 4 chunks: a narrow tile's chunk is little work, and its time would be the
+// latency of the stage hand-over (measured: 8.4M transactions x 69 items x 1 row, 78 us with one
+// chunk per stage, XX us with four).
+// Warp roles (544 threads):
+//   warps 0..15: expansion.  A unit is 8 rows x 512 bits; a lane loads one 16-byte piece (a warp's
+//                load covers 64 contiguous bytes of each row) two to six stages ahead into
+//                registers and stores its four words as four chunks; lanes are placed so that
+//                the eight lanes of a store phase hit different banks;
+//   warp 16    : one lane issues the stage's 8 MMAs and commits them to its `empty` barrier.
+// Then all expansion warps read the accumulator (lane = column of the job, so the int32
+// atomics of a row are coalesced).  Every mbarrier wait is bounded; on expiry the kernel
+// records an error, stops issuing, drains what it issued and frees its tensor memory.
+#include <algorithm>
+#include <atomic>
+
+#include "tfim_internal.h"
+
+namespace tfim {
+namespace {
+
+constexpr int kQM = kF4Cols, kQN = kF4Rows;
+constexpr int kQChunkWords = 16;                 // a chunk: 512 bits of K
+constexpr int kQBlocks = 2;                      // K blocks (256 bits, 128 bytes of nibbles) per chunk
+constexpr int kQExpWarps = 16;
+constexpr int kQThreads = 32 * (kQExpWarps + 1);
+constexpr int kQUnits = 3;                       // units of 8 rows per warp and stage, at most
+constexpr int kQFlight = 6;                      // 16-byte loads in flight per lane: units x stages ahead
+constexpr int kQMaxStages = 6;
+constexpr int kQStaged = 2 * (kQM + kQN) * 128 * kQBlocks;   // two stages of the widest tile
+// The A operand spans 128 rows from its block's start whatever the tile's width; past a narrow
+// tile's columns it runs into the rows behind them (what it adds is not read), and past the
+// last block into a guard of 16 KiB.  Tiles of more than kQNarrow units hold 128 A rows instead
+// (the space behind a narrow tile's columns stays unwritten), so that two of their stages fit
+// without a guard: what shared memory leaves is the L1 cache that the loads in flight need
+// (16 KiB less of it cost the widest tiles 6%).
+constexpr int kQGuard = kQM * 128;
+constexpr int kQNarrow = 22;
+static_assert(2 * 2 * kQNarrow * 2048 + kQGuard <= kQStaged, "two stages of a narrow tile and the guard fit");
+constexpr int kQSmem = kQStaged + 1024;
+constexpr uint32_t kQTmemCols = 512;
+constexpr uint32_t kQScale = 256;                // first scale column; three regions of 32 columns
+constexpr uint32_t kQSpin = 1u << 22;
+static_assert((kQM + kQN) / 8 <= kQUnits * kQExpWarps, "units fit the expansion warps");
+
+__device__ int g_f4_status;   // 0 ok, 1 an mbarrier wait expired
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+
+// K-major, 128-byte swizzle shared-memory matrix descriptor: start address, leading byte
+// offset 16 (unused by swizzled K-major layouts), stride byte offset 1024 (8-row groups),
+// version 1, layout SWIZZLE_128B.
+__device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
+    uint64_t d = 0;
+    d |= (uint64_t)((addr >> 4) & 0x3FFF);
+    d |= (uint64_t)1 << 16;
+    d |= (uint64_t)(1024 >> 4) << 32;
+    d |= (uint64_t)1 << 46;
+    d |= (uint64_t)2 << 61;
+    return d;
+}
+
+// Instruction descriptor of kind::mxf4: A and B e2m1 (format 1), both K-major, UE8M0 scales,
+// scale ids 0, N columns, M = 128.
+__device__ __forceinline__ uint32_t idesc_mxf4(int n) {
+    return (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | (1u << 23) | ((uint32_t)(kQM >> 4) << 24);
+}
+
+__device__ __forceinline__ void mma_mxf4(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t sf,
+                                         uint32_t accumulate) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        "setp.ne.b32 p, %5, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::mxf4.block_scale.scale_vec::2X [%0], %1, %2, %3, [%4], [%4], p;\n\t"
+        "}\n" ::"r"(tmem_d),
+        "l"(da), "l"(db), "r"(idesc), "r"(sf), "r"(accumulate));
+}
+
+__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+    asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.shared::cta.b64 st, [%0];\n\t}" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t"
+        "}\n"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+// Bounded wait on phase `parity`; false when the limit expired.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
+    for (uint32_t k = 0; k < kQSpin; k++)
+        if (mbar_try_wait(bar, parity)) return true;
+    return false;
+}
+__device__ __forceinline__ void tc_commit(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+
+// One value into 32 columns of this warp's 32 lanes.
+__device__ __forceinline__ void tmem_fill32(uint32_t taddr, uint32_t v) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {"
+        "%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, "
+        "%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1};" ::"r"(taddr),
+        "r"(v)
+        : "memory");
+}
+
+// The accumulator's registers are written asynchronously by tcgen05.ld and are valid only
+// after tcgen05.wait::ld; both sit in one asm statement, so nothing reads them in between.
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {"
+        "%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15"
+        "}, [%16];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+        : "r"(taddr)
+        : "memory");
+}
+
+// The expansion of one warp: U units of 8 rows (an A unit holds columns of the job, a B unit
+// rows), kQFlight / U stages of raw words ahead.  Returns false when a wait expired.
+template <int U>
+__device__ __forceinline__ bool f4_expand(const CountArgs& a, const TileDesc& t, const JobDesc& j, int units_a, int units_b,
+                                          int rb, int kc, uint32_t base, int S, int n_st, uint64_t* full, uint64_t* empty,
+                                          int warp, int lane) {
+    constexpr int kAhead = kQFlight / U;
+    const int64_t W = a.W;
+    const int units = units_a + units_b;
+    const uint32_t kb_bytes = (uint32_t)(rb + units_b) * 1024u, stage_bytes = (uint32_t)kc * kQBlocks * kb_bytes;
+    const int stage_words = kc * kQChunkWords;
+    // Lane -> (row of the unit, 16-byte piece): the eight lanes of a store phase hold rows of one
+    // parity and the two pieces of one K block, so chunk ^ row takes eight different values
+    const int q = lane >> 3, i = lane & 7;
+    const int row = 2 * (i >> 1) + (q >> 1), piece = 2 * (q & 1) + (i & 1);
+    const uint32_t* src[U];
+    uint32_t dst[U];
+    bool on[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        const int ch = (warp + u * kQExpWarps) / units, un = (warp + u * kQExpWarps) - ch * units;
+        on[u] = ch < kc;
+        // rows past the tile repeat its last one: their results are not read
+        const uint32_t* p = nullptr;   // null: all ones
+        if (on[u]) {
+            if (un < units_a) {
+                const int c = min(t.c0 + un * 8 + row, t.c1 - 1);
+                const int32_t col = c == j.self_col ? -1 : a.cols[j.col_off + c];
+                if (col >= 0) p = a.bitmap + (int64_t)col * W;
+            } else {
+                const RowDesc rd = a.rows[j.row_off + t.r0 + min((un - units_a) * 8 + row, t.nr - 1)];
+                if (rd.slot >= 0) p = a.masks + (int64_t)rd.slot * W;
+                else if (rd.item >= 0) p = a.bitmap + (int64_t)rd.item * W;
+            }
+        }
+        src[u] = p ? p + t.w0 + ch * kQChunkWords + piece * 4 : nullptr;
+        dst[u] = base + (uint32_t)(ch * kQBlocks + (piece >> 1)) * kb_bytes +
+                 (uint32_t)((un < units_a ? un : rb + un - units_a) * 8 + row) * 128u;
+    }
+    const uint32_t c0 = (uint32_t)(piece & 1), rx = (uint32_t)row;
+    uint4 pf[kAhead][U];
+    auto load = [&](int st, uint4 (&v)[U]) {
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            v[u] = make_uint4(~0u, ~0u, ~0u, ~0u);
+            if (on[u] && src[u] && st < n_st)
+                v[u] = __ldg(reinterpret_cast<const uint4*>(src[u] + (int64_t)st * stage_words));
+        }
+    };
+#pragma unroll
+    for (int d = 0; d < kAhead; d++) load(d, pf[d]);
+    int s = 0;
+    uint32_t ph = 1;   // parity to wait for on `empty`: the first pass over the stages waits for nothing
+    bool ok = true;
+    for (int st0 = 0; st0 < n_st && ok; st0 += kAhead) {
+#pragma unroll
+        for (int d = 0; d < kAhead; d++) {
+            const int st = st0 + d;
+            if (st >= n_st) break;
+            if (st >= S) ok = mbar_wait(smem_u32(&empty[s]), ph);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            const uint32_t off = (uint32_t)s * stage_bytes;
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                if (!on[u]) continue;
+                const uint4 x = pf[d][u];
+                const uint32_t o = dst[u] + off;
+                st_shared_v4(o + (((0 + c0) ^ rx) << 4), x.x & 0x11111111u, x.y & 0x11111111u, x.z & 0x11111111u,
+                             x.w & 0x11111111u);
+                st_shared_v4(o + (((2 + c0) ^ rx) << 4), x.x & 0x22222222u, x.y & 0x22222222u, x.z & 0x22222222u,
+                             x.w & 0x22222222u);
+                st_shared_v4(o + (((4 + c0) ^ rx) << 4), x.x & 0x44444444u, x.y & 0x44444444u, x.z & 0x44444444u,
+                             x.w & 0x44444444u);
+                st_shared_v4(o + (((6 + c0) ^ rx) << 4), (x.x >> 1) & 0x44444444u, (x.y >> 1) & 0x44444444u,
+                             (x.z >> 1) & 0x44444444u, (x.w >> 1) & 0x44444444u);
+            }
+            load(st + kAhead, pf[d]);
+            // generic-proxy stores -> visible to the tensor cores' async proxy
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&full[s]));
+            if (++s == S) {
+                s = 0;
+                ph ^= 1u;
+            }
+        }
+    }
+    return ok;
+}
+
+__global__ void __launch_bounds__(kQThreads, 1) k_count_f4(CountArgs a) {
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ __align__(8) uint64_t full[kQMaxStages], empty[kQMaxStages], done;
+    __shared__ uint32_t s_tmem;
+    __shared__ int32_t s_abort;
+    const TileDesc t = a.tiles[blockIdx.x];
+    const JobDesc j = a.jobs[t.job];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    const int N = (t.nr + 15) & ~15;
+    // 8-row units of a K block: the columns', the rows'; rb: where the rows' units begin
+    const int units_a = (t.c1 - t.c0 + 7) >> 3, units_b = N >> 3, units = units_a + units_b;
+    const bool narrow = units <= kQNarrow;
+    const int rb = narrow ? units_a : kQM / 8;
+    const int kc = units <= kQNarrow / 2 ? 4 : narrow ? 2 : 1;   // chunks per stage
+    const uint32_t kb_bytes = (uint32_t)(rb + units_b) * 1024u;
+    const uint32_t stage_bytes = (uint32_t)kc * kQBlocks * kb_bytes;
+    const int S = min(kQMaxStages, (kQStaged - (narrow ? kQGuard : 0)) / (int)stage_bytes);   // at least 2
+    const int n_st = (t.w1 - t.w0) / (kc * kQChunkWords);      // word slices are multiples of 64 words
+
+    if (tid == 0) {
+        for (int s = 0; s < kQMaxStages; s++) {
+            mbar_init(smem_u32(&full[s]), kQExpWarps);
+            mbar_init(smem_u32(&empty[s]), 1);
+        }
+        mbar_init(smem_u32(&done), 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        s_abort = 0;
+    }
+    if (warp == kQExpWarps) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)),
+                     "r"(kQTmemCols));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = s_tmem;
+    if (warp < 4) {   // the scale regions: every byte 2, 1 and 1/2 (UE8M0)
+        const uint32_t lanes = tmem + ((uint32_t)(32 * warp) << 16) + kQScale;
+        tmem_fill32(lanes, 0x80808080u);
+        tmem_fill32(lanes + 32, 0x7F7F7F7Fu);
+        tmem_fill32(lanes + 64, 0x7E7E7E7Eu);
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+
+    if (warp == kQExpWarps) {
+        if (lane == 0) {
+            bool ok = true;
+            const uint32_t idesc = idesc_mxf4(N);
+            const uint32_t to_b = (uint32_t)rb * 1024u;
+            auto chunk = [&](uint32_t blk, bool first) {
+#pragma unroll
+                for (int kb = 0; kb < kQBlocks; kb++) {
+                    const uint32_t at = blk + (uint32_t)kb * kb_bytes;
+#pragma unroll
+                    for (int k = 0; k < 4; k++)
+                        mma_mxf4(tmem, smem_desc(at + k * 32), smem_desc(at + to_b + k * 32), idesc,
+                                 tmem + kQScale + 32u * (uint32_t)min(k, 2), (!first || kb > 0 || k > 0) ? 1u : 0u);
+                }
+            };
+            for (int st = 0; st < n_st; st++) {
+                const int s = st % S;
+                if (!mbar_wait(smem_u32(&full[s]), (uint32_t)(st / S) & 1u)) {
+                    ok = false;
+                    break;
+                }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t stage = base + (uint32_t)s * stage_bytes;
+                chunk(stage, st == 0);
+                for (int c = 1; c < kc; c++) chunk(stage + (uint32_t)c * kQBlocks * kb_bytes, false);
+                tc_commit(smem_u32(&empty[s]));
+            }
+            if (!ok) {
+                atomicExch(&s_abort, 1);
+                atomicExch(&g_f4_status, 1);
+            }
+            tc_commit(smem_u32(&done));   // tracks every MMA issued so far
+        }
+        __syncwarp();
+    } else {
+        bool ok;
+        if (kc * units <= kQExpWarps) ok = f4_expand<1>(a, t, j, units_a, units_b, rb, kc, base, S, n_st, full, empty, warp, lane);
+        else if (kc * units <= 2 * kQExpWarps)
+            ok = f4_expand<2>(a, t, j, units_a, units_b, rb, kc, base, S, n_st, full, empty, warp, lane);
+        else ok = f4_expand<3>(a, t, j, units_a, units_b, rb, kc, base, S, n_st, full, empty, warp, lane);
+        if (!ok && lane == 0) {
+            atomicExch(&s_abort, 1);
+            atomicExch(&g_f4_status, 1);
+        }
+        // ---- epilogue: warp w reads lanes 32 * (w % 4) (columns of the job), accumulator columns
+        // 16 * (w / 4) + 64 k (rows of the job)
+        const bool fin = mbar_wait(smem_u32(&done), 0);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const bool all_fin = __all_sync(0xffffffffu, fin);
+        if (!all_fin && lane == 0) {
+            atomicExch(&s_abort, 1);
+            atomicExch(&g_f4_status, 1);
+        }
+        if (all_fin && !*(volatile int32_t*)&s_abort && n_st > 0) {
+            const int quad = warp & 3, c = t.c0 + 32 * quad + lane;
+            for (int n0 = 16 * (warp >> 2); n0 < N; n0 += 64) {
+                uint32_t v[16];
+                tmem_ld16(tmem + ((uint32_t)(32 * quad) << 16) + (uint32_t)n0, v);
+                if (c < t.c1) {
+                    int32_t* out = a.out + j.out_off + (int64_t)(t.r0 + n0) * j.n_cols + c;
+#pragma unroll
+                    for (int k = 0; k < 16; k++) {
+                        const int32_t n = __float2int_rn(__uint_as_float(v[k]));
+                        if (n && n0 + k < t.nr) atomicAdd(out + (int64_t)k * j.n_cols, n);
+                    }
+                }
+            }
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == kQExpWarps)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kQTmemCols));
+}
+
+}  // namespace
+
+// Tiles of one job of nr rows x nc columns.  The word slices are chosen so that the tiles fill
+// whole waves of one CTA per SM: the cheapest count by (waves of CTAs) x (chunks per tile + the
+// fixed cost of a tile, about 16 chunks' time: set-up, first loads and epilogue).  A slice holds
+// at most 2^18 words (2^23 transactions), so that FP32 sums stay exact.  `upper`: rows and
+// columns are the same list and tiles wholly below the diagonal are left out.
+void tiles_f4(int32_t job, int32_t nr, int32_t nc, int64_t W, int sms, std::vector<TileDesc>& out, bool upper) {
+    if (nr <= 0 || nc <= 0 || W <= 0) return;
+    std::vector<TileDesc> tl;
+    // equal row groups of at most kF4Rows, multiples of 16
+    const int32_t groups = (nr + kF4Rows - 1) / kF4Rows;
+    const int32_t step = ((nr + groups - 1) / groups + 15) & ~15;
+    for (int32_t r0 = 0; r0 < nr; r0 += step)
+        for (int32_t c0 = 0; c0 < nc; c0 += kF4Cols) {
+            const int32_t c1 = std::min(nc, c0 + kF4Cols);
+            if (upper && c1 <= r0) continue;
+            tl.push_back(TileDesc{job, r0, std::min(step, nr - r0), c0, c1, 0, 0, 0});
+        }
+    const int64_t blocks = W / kRowAlignWords, base = (int64_t)tl.size();
+    int64_t best = 1;
+    double best_cost = 1e300;
+    const int64_t max_ks = std::min<int64_t>(blocks, std::max<int64_t>(1, 4 * sms / std::max<int64_t>(base, 1)) + (W >> 18) + 1);
+    for (int64_t ks = 1; ks <= max_ks; ks++) {
+        const int64_t per = (blocks + ks - 1) / ks;
+        if (per * kRowAlignWords > (1 << 18)) continue;
+        const int64_t n = (blocks + per - 1) / per;
+        const double cost = (double)((base * n + sms - 1) / sms) * (double)(per * (kRowAlignWords / kQChunkWords) + 16);
+        if (cost < best_cost) {
+            best_cost = cost;
+            best = per;
+        }
+    }
+    if (best_cost == 1e300) best = (1 << 18) / kRowAlignWords;
+    for (int64_t b0 = 0; b0 < blocks; b0 += best)
+        for (TileDesc t : tl) {
+            t.w0 = (int32_t)(b0 * kRowAlignWords);
+            t.w1 = (int32_t)(std::min(blocks, b0 + best) * kRowAlignWords);
+            out.push_back(t);
+        }
+}
+
+int launch_count_f4(const CountArgs& a, cudaStream_t s) {
+    if (a.n_tiles <= 0) return TFIM_OK;
+    static std::atomic<bool> configured[64];
+    int dev = 0;
+    TFIM_CUDA(cudaGetDevice(&dev));
+    if (dev >= 0 && dev < 64 && !configured[dev].load()) {
+        TFIM_CUDA(cudaFuncSetAttribute(k_count_f4, cudaFuncAttributeMaxDynamicSharedMemorySize, kQSmem));
+        configured[dev].store(true);
+    }
+    k_count_f4<<<a.n_tiles, kQThreads, kQSmem, s>>>(a);
+    TFIM_CUDA(cudaGetLastError());
+    return TFIM_OK;
+}
+
+int count_f4_status_fetch(int32_t* pinned, cudaStream_t s) {
+    TFIM_CUDA(cudaMemcpyFromSymbolAsync(pinned, g_f4_status, sizeof(int32_t), 0, cudaMemcpyDeviceToHost, s));
+    return TFIM_OK;
+}
+
+int count_f4_status_check(int32_t v) {
+    if (v) {
+        const int z = 0;
+        TFIM_CUDA(cudaMemcpyToSymbol(g_f4_status, &z, sizeof z));
+    }
+    TFIM_CHECK(v == 0, TFIM_E_TIMEOUT, "tensor-memory counter: an mbarrier wait expired");
+    return TFIM_OK;
+}
+
+}  // namespace tfim

@@ -379,10 +379,13 @@ int launch_count_fam_persistent(const CountArgs* d_args, const int32_t* d_n_tile
     return TFIM_OK;
 }
 
-int count_fam_status(bool reset) {
-    int v = 0;
-    TFIM_CUDA(cudaMemcpyFromSymbol(&v, g_fam_status, sizeof v));
-    if (reset && v) {
+int count_fam_status_fetch(int32_t* pinned, cudaStream_t s) {
+    TFIM_CUDA(cudaMemcpyFromSymbolAsync(pinned, g_fam_status, sizeof(int32_t), 0, cudaMemcpyDeviceToHost, s));
+    return TFIM_OK;
+}
+
+int count_fam_status_check(int32_t v) {
+    if (v) {
         const int z = 0;
         TFIM_CUDA(cudaMemcpyToSymbol(g_fam_status, &z, sizeof z));
     }

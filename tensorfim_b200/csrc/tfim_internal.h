@@ -174,10 +174,15 @@ int launch_count_proj_persistent(const CountArgs* d_args, const int32_t* d_n_job
 // blocks of each persistent kernel resident per SM
 int persistent_occupancy(int* lop3, int* b1, int* proj);
 int configure_count_kernels();
-// tcgen05 kind::i8 counter (count_tc.cu): 128 x 128 tiles; the status reads (and with
-// `reset` clears) the device flag the kernel sets when an mbarrier wait expired.
-int launch_count_i8(const CountArgs& a, cudaStream_t s);
-int count_i8_status(bool reset);
+// tcgen05 kind::mxf4 wave counter (count_f4.cu): tiles of up to kF4Cols columns x kF4Rows rows of
+// one job without a base whose rows have one source each.  The device flag the kernel sets when
+// an mbarrier wait expired is copied to pinned memory in stream order and checked (and
+// cleared) once the stream has been waited for anyway.
+constexpr int kF4Cols = 128, kF4Rows = 256;
+int launch_count_f4(const CountArgs& a, cudaStream_t s);
+int count_f4_status_fetch(int32_t* pinned, cudaStream_t s);
+int count_f4_status_check(int32_t v);
+void tiles_f4(int32_t job, int32_t nr, int32_t nc, int64_t W, int sms, std::vector<TileDesc>& out, bool upper = false);
 // tcgen05 kind::i8 family counter (count_fam.cu): a tile is one family job (rows a run of its
 // columns, at most kFamMaxCols columns) over a word slice, TileDesc.pad = the F position of
 // the tile's first row; one CTA per SM.  The persistent form reads its arguments and tile
@@ -186,7 +191,8 @@ constexpr int kFamMaxCols = 128;
 int launch_count_fam(const CountArgs& a, cudaStream_t s);
 int launch_count_fam_persistent(const CountArgs* d_args, const int32_t* d_n_tiles, int32_t* d_next, int32_t grid,
                                 cudaStream_t s);
-int count_fam_status(bool reset);
+int count_fam_status_fetch(int32_t* pinned, cudaStream_t s);
+int count_fam_status_check(int32_t v);
 int configure_fam_kernel();   // opt into its shared memory (once per device, before any capture)
 // CUDA-core Gram counter for dense family jobs (count_gram.cu): a tile is one family job of at
 // most kGramMaxCols columns and at most 128 blocks of 4 x 4 (row, column) pairs, over a word
@@ -282,7 +288,7 @@ struct tfim_ctx {
     bool all_mined = false;
     bool mined = false;
     int32_t counter_pref = TFIM_COUNTER_AUTO;   // counter used by tfim_count_wave
-    bool used_i8 = false;                       // the last counting wave ran the tcgen05 i8 counter
+    tfim::HostBuf h_flags;                      // pinned copies of the tcgen05 counters' device flags
     tfim_mine_stats last_stats{};
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     tfim::EngineState* engine = nullptr;
