@@ -107,7 +107,7 @@ int count_wave_impl(tfim_ctx* c, int32_t b, int32_t min_count, const int32_t* d_
     std::vector<JobDesc> jobs(1);
     jobs[0].base_slot = -1; jobs[0].base_item = -1;
     jobs[0].n_rows = b; jobs[0].n_cols = d; jobs[0].row_off = 0; jobs[0].col_off = 0; jobs[0].out_off = 0;
-    jobs[0].self_col = -1; jobs[0].pad = 0;
+    jobs[0].self_col = -1; jobs[0].words = 0;
     std::vector<RowDesc> rows(b);
     for (int32_t i = 0; i < b; i++) rows[i] = RowDesc{i, -1};
     std::vector<int32_t> cols(d);

@@ -154,7 +154,7 @@ struct Wave {
         j.self_col = -1;   // a -1 column id is the all-ones column: tell the counters its index
         for (int32_t q = 0; q < j.n_cols; q++)
             if (cs[q] < 0) { j.self_col = q; break; }
-        j.pad = 0;
+        j.words = 0;
         const int32_t id = (int32_t)jobs.size();
         jobs.push_back(j);
         use_b1.push_back(b1);

@@ -28,7 +28,7 @@
 namespace tfim {
 namespace {
 
-struct DFam {
+struct alignas(16) DFam {
     int32_t slot, item;        // base mask = masks[slot] & B[item] (either optional)
     int32_t head_off, head_len;
     int32_t F_off, nF, nT;     // F list in the item pool, tail = its first nT entries
@@ -37,6 +37,8 @@ struct DFam {
     int32_t rows_done;         // rows expanded
     int32_t state;             // 0 ready, 1 waiting on its lookahead, 2 finished
     int32_t top;               // 1: the family of the empty prefix
+    int32_t W, n;              // its transactions: words per bitmap row, and their number
+    int32_t pad[2];
 };
 
 struct DLook {
@@ -52,15 +54,15 @@ struct MaskJob {
 enum { kJobFam = 0, kJobLook = 1 };
 struct DJob {
     int32_t fam, kind, r0, nr, slot, log;
-    int32_t b3, b1;            // exclusive prefix of CUDA-core / tensor-core tiles over the wave's jobs
-    int32_t cls, sl3;          // counter class (kCls*); word slices of its CUDA-core tiles
-    int32_t b3l, heavy;        // CUDA-core tiles: heavy jobs' tiles come first (prefix b3), then the light
-                               // jobs' (prefix b3l after all heavy tiles)
-    int32_t btc;               // exclusive prefix of the tcgen05 family counter's jobs
-    int32_t bgr;               // exclusive prefix of the CUDA-core Gram counter's jobs
-    int32_t b3d;               // CUDA-core tiles of dense families (heavy == 2): they come before all
-                               // others (prefix b3d), for the register-blocked dense launch
+    int32_t cls, sl3;          // tile group (kGrp*, or kGrps: the projected counter's); word slices
+    // exclusive prefixes of the tile groups over the wave's jobs.  CUDA-core tiles: dense
+    // families' first (the register-blocked launch), then heavy jobs', then the light ones'
+    int32_t pre[6];
+    int32_t sup, pad;          // its family's support
 };
+
+// Tile groups of a wave: the order of DJob::pre.
+enum { kGrpDense = 0, kGrpHeavy, kGrpLight, kGrpB1, kGrpTc, kGrpGram, kGrps };
 
 // Phases of a wave (device-time stamps) and counter classes of a count job.
 enum { kPhPack = 0, kPhZero, kPhLop3, kPhB1, kPhTc, kPhProj, kPhGram, kPhExpand, kPhMasks, kPhases };
@@ -216,7 +218,7 @@ constexpr int kPackCand = kPackThreads * kPackItems;
 // most kFamMaxCols columns: always when that counter is asked for, and in the automatic choice
 // when the job is large enough and its prefix dense enough that skipping zero words (which
 // the CUDA-core tiles do and the tensor tiles do not) saves little.
-__device__ __forceinline__ bool use_tc(const ResPtrs& p, const JobDesc& jd, int32_t sup) {
+__device__ __forceinline__ bool use_tc(const ResPtrs& p, const JobDesc& jd, int32_t sup, int32_t n) {
     if (jd.n_cols < 1 || jd.n_cols > kFamMaxCols || jd.n_rows < 1) return false;
     if (p.counter == TFIM_COUNTER_I8) return true;
     if (p.counter != TFIM_COUNTER_AUTO) return false;
@@ -224,7 +226,7 @@ __device__ __forceinline__ bool use_tc(const ResPtrs& p, const JobDesc& jd, int3
     // shape there); wider ones take the tensor tiles when large enough to fill their MMAs
     if (jd.n_cols <= kGramMaxCols) return false;
     if ((int64_t)jd.n_rows * jd.n_cols < p.tc_min_work) return false;
-    const float d = p.n_bits > 0 ? fminf(1.f, 128.f * (float)sup / (float)p.n_bits) : 1.f;
+    const float d = n > 0 ? fminf(1.f, 128.f * (float)sup / (float)n) : 1.f;
     return d >= p.tc_min_density;
 }
 
@@ -232,13 +234,13 @@ __device__ __forceinline__ bool use_tc(const ResPtrs& p, const JobDesc& jd, int3
 // most 128 blocks of 4 x 4 pairs): a dense prefix has no zero word for the general tiles to
 // skip, and at these widths the register-tiled Gram block (86-91% of the POPC ceiling at 32
 // and 64 columns) beats the tensor tiles, whose narrow MMAs cost about 50 cycles each.
-__device__ __forceinline__ bool use_gram(const ResPtrs& p, const JobDesc& jd, int32_t sup) {
+__device__ __forceinline__ bool use_gram(const ResPtrs& p, const JobDesc& jd, int32_t sup, int32_t n) {
     // tails of 1 or 2 rows are memory-bound in any kernel (8 bit-ops per byte and row); the
     // general tiles handle them as well, and measured faster on the dense benchmark
     if (jd.n_cols < 1 || jd.n_cols > kGramMaxCols || jd.n_rows < p.gram_min_rows) return false;
     if (((jd.n_rows + 3) / 4) * ((jd.n_cols + 3) / 4) > 128) return false;
     if (p.counter != TFIM_COUNTER_AUTO) return false;
-    const float d = p.n_bits > 0 ? fminf(1.f, 128.f * (float)sup / (float)p.n_bits) : 1.f;
+    const float d = n > 0 ? fminf(1.f, 128.f * (float)sup / (float)n) : 1.f;
     return d >= p.tc_min_density;
 }
 
@@ -254,54 +256,102 @@ __device__ __forceinline__ int64_t b1_tiles(int nr, int nc) { return (int64_t)((
 // One block.  Phases: (0) recycle the mask slots released by the last expand; (1) one job
 // per queued lookahead; (2) families from the top of the stack, 4096 candidates per pass,
 // with block scans deciding how many fit the wave's row and output budgets; (3) the counted
-// rows and row->job maps; (4) tiles (split-k slices chosen from the wave's base tile count).
-// Every phase is block-parallel; jobs are ordered by their row offsets, which the row and
-// tile writers binary-search.
-__device__ __forceinline__ int find_job_by_row(const JobDesc* jobs, int nj, int32_t g) {
-    int lo = 0, hi = nj - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (jobs[mid].row_off <= g) lo = mid; else hi = mid - 1;
+// rows and row->job maps; (4) tiles.  Every phase is block-parallel; jobs are ordered by their
+// row offsets, which the row writer binary-searches, as the tile writers do the prefixes of
+// their group.
+//
+// The kernel is a chain of latencies on one SM while the other 147 wait, so each phase scans
+// all its quantities in one pass of warp shuffles (two barriers) and the binary searches run
+// on prefixes held in shared memory.  Measured per launch: 10,000-row dense database 39 -> 18
+// us, 1M-row sparse one 60 -> 38 us, 6.3M-row dense one 147 -> 100 us.
+constexpr int kPackSearch = 5120;   // jobs whose prefixes fit the shared search arrays
+
+// Exclusive prefixes of N values per thread over the block, and their totals.  `sm` holds
+// N * 33 values; `any` = false: this warp's values are all zero.
+template <int N, typename T>
+__device__ __forceinline__ void block_scan(T (&v)[N], T (&ex)[N], T (&tot)[N], T* sm, bool any) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    T inc[N];
+#pragma unroll
+    for (int k = 0; k < N; k++) inc[k] = v[k];
+    if (any) {
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1)
+#pragma unroll
+            for (int k = 0; k < N; k++) {
+                const T x = __shfl_up_sync(0xffffffffu, inc[k], o);
+                if (lane >= o) inc[k] += x;
+            }
     }
-    return lo;
+    if (lane == 31)
+#pragma unroll
+        for (int k = 0; k < N; k++) sm[k * 33 + warp] = inc[k];
+    __syncthreads();
+    if (warp < N) {   // warp k scans value k's warp totals
+        const T own = sm[warp * 33 + lane];
+        T x = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const T y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        sm[warp * 33 + lane] = x - own;
+        if (lane == 31) sm[warp * 33 + 32] = x;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < N; k++) {
+        ex[k] = sm[k * 33 + warp] + inc[k] - v[k];
+        tot[k] = sm[k * 33 + 32];
+    }
+    __syncthreads();   // sm is reused
 }
-// The last job whose prefix (0: b3, 1: b1, 2: b3l) is <= t: the job owning tile t, since a
-// job with no tiles of that kind shares its prefix with the next job that has some.
-template <int K>
-__device__ __forceinline__ int find_job_by_tile(const DJob* dj, int nj, int64_t t) {
-    int lo = 0, hi = nj - 1;
+
+// The last entry of the ascending a[0 .. n) that is <= t (a[0] <= t).
+template <typename A>
+__device__ __forceinline__ int last_le(const A& at, int n, int32_t t) {
+    int lo = 0, hi = n - 1;
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
-        const int32_t v = K == 0   ? dj[mid].b3
-                          : K == 1 ? dj[mid].b1
-                          : K == 2 ? dj[mid].b3l
-                          : K == 3 ? dj[mid].btc
-                          : K == 4 ? dj[mid].bgr
-                                   : dj[mid].b3d;
-        if (v <= t) lo = mid; else hi = mid - 1;
+        if (at(mid) <= t) lo = mid; else hi = mid - 1;
     }
     return lo;
 }
 
+// Word slices of `n` tiles of `words` words each when a wave's tiles hold `total` words in all
+// and should make about `want` slices: the slice length in words, a multiple of 64.
+__device__ __forceinline__ int64_t slice_words(int64_t total, int64_t want) {
+    return lmax(1, (total / lmax(want, 1) + 63) / 64) * 64;
+}
+
 __device__ __forceinline__ void res_pack(const ResPtrs& p) {
-    typedef cub::BlockScan<int64_t, kPackThreads> Scan;
-    typedef cub::BlockReduce<int64_t, kPackThreads> Red;
-    __shared__ union {
-        typename Scan::TempStorage scan;
-        typename Red::TempStorage red;
-    } tmp;
-    __shared__ int32_t s_fam[kPackCand];
+    __shared__ int64_t sm64[2 * 33];
+    __shared__ int32_t sm32[6 * 33];
+    __shared__ int32_t s_pre[kPackSearch];
+    __shared__ int32_t s_src[kPackSearch];
     __shared__ int32_t s_n_jobs, s_rows_total, s_done, s_max_cols, s_max_head, s_stack_after, s_kstop, s_fit;
-    __shared__ int64_t s_out_total, s_agg;
+    __shared__ int64_t s_out_total;
+    __shared__ float s_cost;
+    __shared__ unsigned long long s_words[3];   // words of the wave's b1 / tcgen05 / Gram tiles
     ResStatus* st = p.st;
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31;
     // (0) recycle
     const int32_t taken = min(st->free_taken, st->free_n);
     const int32_t fn = st->free_n - taken, dn = st->defer_n;
+    const int32_t n_look = st->look_n;
     for (int k = tid; k < dn; k += kPackThreads) p.free_slots[fn + k] = p.defer[k];
-    if (tid == 0) {
-        s_n_jobs = 0; s_rows_total = 0; s_out_total = 0; s_max_cols = 0; s_max_head = 0; s_done = 0;
+    if (tid < kPhases) {
+        // the last wave's phases: add their durations, clear the stamps, stamp this pack
+        const unsigned long long s0 = st->ph_s[tid], e0 = st->ph_e[tid];
+        if (s0 != ~0ull && e0 > s0) st->ph_ns[tid] += e0 - s0;
+        st->ph_s[tid] = tid == kPhPack ? globaltimer() : ~0ull;
+        st->ph_e[tid] = 0;
+    }
+    if (tid == 32) {
+        s_n_jobs = n_look; s_rows_total = n_look; s_out_total = 0; s_max_cols = 0; s_max_head = 0; s_done = 0;
         s_stack_after = st->stack_n;
+        s_cost = 0.f;
+        s_words[0] = s_words[1] = s_words[2] = 0;
         st->n_proj = 0;
         st->n_mjobs = 0;
         st->grow = 0;
@@ -312,14 +362,6 @@ __device__ __forceinline__ void res_pack(const ResPtrs& p) {
             st->launch_id = p.launch_id;
             st->launch_t0 = globaltimer();
         }
-        // the last wave's phases: add their durations, clear the stamps, stamp this pack
-        for (int k = 0; k < kPhases; k++) {
-            const unsigned long long s0 = st->ph_s[k], e0 = st->ph_e[k];
-            if (s0 != ~0ull && e0 > s0) st->ph_ns[k] += e0 - s0;
-            st->ph_s[k] = ~0ull;
-            st->ph_e[k] = 0;
-        }
-        st->ph_s[kPhPack] = globaltimer();
     }
     __syncthreads();
     if (tid == 0) {
@@ -328,49 +370,36 @@ __device__ __forceinline__ void res_pack(const ResPtrs& p) {
         st->defer_n = 0;
     }
     // (1) lookahead jobs
-    const int32_t n_look = st->look_n;
-    for (int base = 0; base < n_look; base += kPackCand) {
-        int64_t v[kPackItems], ex[kPackItems];
-        int64_t mc = 0;
-        for (int q = 0; q < kPackItems; q++) {
-            const int k = base + tid * kPackItems + q;
-            v[q] = 0;
-            if (k < n_look) {
-                const DFam f = p.fams[p.looks[k].fam];
-                v[q] = f.nF - f.nT + 1;
-                mc = max(mc, v[q]);
-            }
+    for (int base = 0; base < n_look; base += kPackThreads) {
+        const int k = base + tid;
+        int64_t v[1] = {0}, ex[1], tot[1];
+        DLook L{};
+        DFam f{};
+        if (k < n_look) {
+            L = p.looks[k];
+            f = p.fams[L.fam];
+            v[0] = f.nF - f.nT + 1;
+            atomicMax(&s_max_cols, (int32_t)v[0]);
         }
-        Scan(tmp.scan).ExclusiveSum(v, ex, s_agg);
-        __syncthreads();
-        const int64_t agg = s_agg;
-        const int64_t mcb = Red(tmp.red).Reduce(mc, cub::Max());
-        for (int q = 0; q < kPackItems; q++) {
-            const int k = base + tid * kPackItems + q;
-            if (k >= n_look) continue;
-            const DLook L = p.looks[k];
-            const DFam f = p.fams[L.fam];
-            DJob dj;
-            dj.fam = L.fam; dj.kind = kJobLook; dj.r0 = 0; dj.nr = 1; dj.slot = L.slot; dj.log = L.log; dj.b3 = 0; dj.b1 = 0;
-            dj.cls = 0; dj.sl3 = 1; dj.b3l = 0; dj.heavy = 0; dj.btc = 0; dj.bgr = 0; dj.b3d = 0;
+        block_scan<1>(v, ex, tot, sm64, base + (tid & ~31) < n_look);
+        if (k < n_look) {
+            DJob dj{};
+            dj.fam = L.fam; dj.kind = kJobLook; dj.nr = 1; dj.slot = L.slot; dj.log = L.log; dj.sl3 = 1; dj.sup = f.sup;
             p.djobs[k] = dj;
             JobDesc jd;
-            jd.base_slot = -1; jd.base_item = -1; jd.n_rows = 1; jd.n_cols = f.nF - f.nT + 1;
-            jd.row_off = k; jd.col_off = f.F_off + f.nT; jd.out_off = s_out_total + ex[q]; jd.self_col = f.nF - f.nT; jd.pad = 0;
+            jd.base_slot = -1; jd.base_item = -1; jd.n_rows = 1; jd.n_cols = (int32_t)v[0];
+            jd.row_off = k; jd.col_off = f.F_off + f.nT; jd.out_off = s_out_total + ex[0]; jd.self_col = f.nF - f.nT;
+            jd.words = f.W;
             p.jobs[k] = jd;
+            if (k < kPackSearch) {
+                s_pre[k] = k;
+                s_src[k] = -1 - L.slot;
+            }
         }
         __syncthreads();
-        if (tid == 0) {
-            s_out_total += agg;
-            s_max_cols = max(s_max_cols, (int32_t)mcb);
-        }
+        if (tid == 0) s_out_total += tot[0];
         __syncthreads();
     }
-    if (tid == 0) {
-        s_rows_total = n_look;
-        s_n_jobs = n_look;
-    }
-    __syncthreads();
     // (2) families from the top of the stack
     while (!s_done) {
         const int32_t avail = s_stack_after;
@@ -378,18 +407,23 @@ __device__ __forceinline__ void res_pack(const ResPtrs& p) {
         if (n_c == 0) break;
         const int64_t rows_left = (int64_t)p.wave_rows - s_rows_total;
         const int64_t out_left = p.cap_out - s_out_total;
-        const bool wave_empty = s_n_jobs == 0;
-        int64_t rv[kPackItems], ov[kPackItems], rc[kPackItems], oc[kPackItems];
+        const int64_t out_base = s_out_total;
+        const int32_t rows_base = s_rows_total, jobs_base = s_n_jobs;
+        const bool any = (tid & ~31) * kPackItems < n_c;
+        int32_t fid[kPackItems];
+        int64_t rv[kPackItems], ov[kPackItems];
         int32_t nf[kPackItems], hl[kPackItems];
+#pragma unroll
         for (int q = 0; q < kPackItems; q++) {
             const int k = tid * kPackItems + q;
+            fid[q] = k < n_c ? p.stack[avail - 1 - k] : -1;
+        }
+#pragma unroll
+        for (int q = 0; q < kPackItems; q++) {
             rv[q] = ov[q] = 0;
-            nf[q] = 0;
-            hl[q] = 0;
-            if (k < n_c) {
-                const int32_t fid = p.stack[avail - 1 - k];
-                const DFam f = p.fams[fid];
-                s_fam[k] = fid;
+            nf[q] = hl[q] = 0;
+            if (fid[q] >= 0) {
+                const DFam f = p.fams[fid[q]];
                 const int32_t rem = f.state == 0 ? f.nT - f.next_row : 0;
                 rv[q] = rem;
                 ov[q] = (int64_t)rem * f.nF;
@@ -397,182 +431,179 @@ __device__ __forceinline__ void res_pack(const ResPtrs& p) {
                 hl[q] = f.head_len;
             }
         }
-        Scan(tmp.scan).InclusiveSum(rv, rc);
-        __syncthreads();
-        Scan(tmp.scan).InclusiveSum(ov, oc);
-        __syncthreads();
+        if (tid == 0) s_kstop = n_c;
+        int64_t tr[2] = {0, 0}, ex[2], tot[2];
+#pragma unroll
+        for (int q = 0; q < kPackItems; q++) {
+            tr[0] += rv[q];
+            tr[1] += ov[q];
+        }
+        block_scan<2>(tr, ex, tot, sm64, any);
         // take per candidate and the first stop point
         int32_t take[kPackItems];
-        int64_t kstop_local = n_c;
+        int64_t o_at[kPackItems];
+        int kstop = n_c;
+        int64_t rb = ex[0], ob = ex[1];
+#pragma unroll
         for (int q = 0; q < kPackItems; q++) {
             const int k = tid * kPackItems + q;
             take[q] = -1;
-            if (k >= n_c) continue;
-            const int64_t r_before = rc[q] - rv[q], o_before = oc[q] - ov[q];
-            if (rc[q] <= rows_left && oc[q] <= out_left) {
-                take[q] = (int32_t)rv[q];
-            } else if (r_before < rows_left && o_before < out_left) {
-                int64_t t_rows = min(rows_left - r_before, (out_left - o_before) / max(1, nf[q]));
-                take[q] = (int32_t)min(t_rows, rv[q]);
-                if (take[q] == 0 && r_before == 0 && o_before == 0 && wave_empty) atomicExch(&st->starved, 1);
+            o_at[q] = ob;
+            if (k < n_c) {
+                const int64_t r1 = rb + rv[q], o1 = ob + ov[q];
+                if (r1 <= rows_left && o1 <= out_left) {
+                    take[q] = (int32_t)rv[q];
+                } else if (rb < rows_left && ob < out_left) {
+                    take[q] = (int32_t)lmin(lmin(rows_left - rb, (out_left - ob) / max(1, nf[q])), rv[q]);
+                    if (take[q] == 0 && rb == 0 && ob == 0 && jobs_base == 0) atomicExch(&st->starved, 1);
+                }
+                if (take[q] < 0 || (rv[q] > 0 && take[q] < rv[q])) kstop = min(kstop, k);
+                rb = r1;
+                ob = o1;
             }
-            const bool stop = take[q] < 0 || (rv[q] > 0 && take[q] < rv[q]);
-            if (stop) kstop_local = min(kstop_local, (int64_t)k);
         }
-        const int64_t kstop = Red(tmp.red).Reduce(kstop_local, cub::Min());
-        if (tid == 0) s_kstop = (int32_t)kstop;
+        if (kstop < n_c) atomicMin(&s_kstop, kstop);
         __syncthreads();
         const int32_t ks = s_kstop;
         // jobs: candidates before the stop point with rows left, and the stop point if it takes rows
-        int64_t hj[kPackItems], hx[kPackItems], tr[kPackItems];
-        int64_t mcol = 0, mhead = 0;
+        bool hj[kPackItems];
+        int32_t jv[2] = {0, 0}, jx[2], jt[2];
+        int32_t mcol = 0, mhead = 0;
+        int64_t contrib = 0;
+#pragma unroll
         for (int q = 0; q < kPackItems; q++) {
             const int k = tid * kPackItems + q;
-            hj[q] = 0;
-            tr[q] = 0;
-            if (k < n_c && ((k < ks && rv[q] > 0) || (k == ks && take[q] > 0))) {
-                hj[q] = 1;
-                tr[q] = take[q];
-                mcol = max(mcol, (int64_t)nf[q]);
-                mhead = max(mhead, (int64_t)hl[q]);
+            hj[q] = k < n_c && ((k < ks && rv[q] > 0) || (k == ks && take[q] > 0));
+            if (hj[q]) {
+                jv[0] += 1;
+                jv[1] += take[q];
+                mcol = max(mcol, nf[q]);
+                mhead = max(mhead, hl[q]);
+                contrib += (int64_t)take[q] * nf[q];
             }
         }
-        Scan(tmp.scan).ExclusiveSum(hj, hx, s_agg);
-        __syncthreads();
-        const int64_t n_new = s_agg;
-        int64_t trx[kPackItems];
-        Scan(tmp.scan).ExclusiveSum(tr, trx, s_agg);
-        __syncthreads();
-        const int64_t rows_new = s_agg;
-        const int64_t mcb = Red(tmp.red).Reduce(mcol, cub::Max());
-        __syncthreads();
-        const int64_t mhb = Red(tmp.red).Reduce(mhead, cub::Max());
+        block_scan<2>(jv, jx, jt, sm32, any);
+        if (any) {
+            mcol = __reduce_max_sync(0xffffffffu, mcol);
+            mhead = __reduce_max_sync(0xffffffffu, mhead);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) contrib += __shfl_xor_sync(0xffffffffu, contrib, o);
+            if (lane == 0) {
+                atomicMax(&s_max_cols, mcol);
+                atomicMax(&s_max_head, mhead);
+                if (contrib) atomicAdd((unsigned long long*)&s_out_total, (unsigned long long)contrib);
+            }
+        }
+        int32_t jid = jobs_base + jx[0], row = rows_base + jx[1];
+#pragma unroll
         for (int q = 0; q < kPackItems; q++) {
-            const int k = tid * kPackItems + q;
             if (!hj[q]) continue;
-            const int32_t fid = s_fam[k];
-            DFam* fp = p.fams + fid;
-            const DFam f = *fp;
-            const int32_t jid = s_n_jobs + (int32_t)hx[q];
-            DJob dj;
-            dj.fam = fid; dj.kind = kJobFam; dj.r0 = f.next_row; dj.nr = take[q]; dj.slot = -1; dj.log = -1; dj.b3 = 0; dj.b1 = 0;
-            dj.cls = 0; dj.sl3 = 1; dj.b3l = 0; dj.heavy = 0; dj.btc = 0; dj.bgr = 0; dj.b3d = 0;
-            p.djobs[jid] = dj;
+            const DFam f = p.fams[fid[q]];
+            DJob dj{};
+            dj.fam = fid[q]; dj.kind = kJobFam; dj.r0 = f.next_row; dj.nr = take[q]; dj.slot = -1; dj.log = -1; dj.sl3 = 1;
+            dj.sup = f.sup;
+            p.djobs[jid] = dj;   // next_row advances when the wave is committed
             JobDesc jd;
             jd.base_slot = f.slot; jd.base_item = f.item; jd.n_rows = take[q]; jd.n_cols = f.nF;
-            jd.row_off = s_rows_total + (int32_t)trx[q];
+            jd.row_off = row;
             jd.col_off = f.F_off;
             // outputs: every candidate before this one contributed rv * nF, this one take * nF
-            jd.out_off = s_out_total + (oc[q] - ov[q]);
-            jd.self_col = -1; jd.pad = 0;
+            jd.out_off = out_base + o_at[q];
+            jd.self_col = -1; jd.words = f.W;
             p.jobs[jid] = jd;
-            (void)fp;   // next_row advances when the wave is committed
+            if (jid < kPackSearch) {
+                s_pre[jid] = row;
+                s_src[jid] = f.F_off + f.next_row;
+            }
+            jid++;
+            row += take[q];
         }
         __syncthreads();
-        // outputs of this pass: every job's taken rows x its columns
-        int64_t contrib = 0;
-        for (int q = 0; q < kPackItems; q++) contrib += (int64_t)(hj[q] ? (int64_t)tr[q] * nf[q] : 0);
-        const int64_t out_pass = Red(tmp.red).Sum(contrib);
         if (tid == 0) {
-            s_n_jobs += (int32_t)n_new;
-            s_rows_total += (int32_t)rows_new;
-            s_out_total += out_pass;
-            s_max_cols = max(s_max_cols, (int32_t)mcb);
-            s_max_head = max(s_max_head, (int32_t)mhb);
-            s_stack_after -= ks;   // candidates before the stop point are consumed
+            s_n_jobs = jobs_base + jt[0];
+            s_rows_total = rows_base + jt[1];
+            s_stack_after = avail - ks;   // candidates before the stop point are consumed
             if (ks < n_c || s_rows_total >= p.wave_rows || n_c < kPackCand || s_stack_after == 0) s_done = 1;
         }
         __syncthreads();
     }
-    __syncthreads();
     const int32_t nj = s_n_jobs, rows_total = s_rows_total;
+    const bool in_sm = nj <= kPackSearch;
     // (3) rows
     for (int32_t g = tid; g < rows_total; g += kPackThreads) {
-        const int j = find_job_by_row(p.jobs, nj, g);
-        const JobDesc jd = p.jobs[j];
-        const DJob dj = p.djobs[j];
-        const int32_t r = g - jd.row_off;
-        if (dj.kind == kJobFam) p.rows[g] = RowDesc{-1, p.items[jd.col_off + dj.r0 + r]};
-        else p.rows[g] = RowDesc{dj.slot, -1};
+        int j, r;
+        int32_t src;
+        if (in_sm) {
+            j = last_le([&](int k) { return s_pre[k]; }, nj, g);
+            r = g - s_pre[j];
+            src = s_src[j];
+        } else {
+            j = last_le([&](int k) { return p.jobs[k].row_off; }, nj, g);
+            r = g - p.jobs[j].row_off;
+            const DJob dj = p.djobs[j];
+            src = dj.kind == kJobFam ? p.jobs[j].col_off + dj.r0 : -1 - dj.slot;
+        }
+        p.rows[g] = src >= 0 ? RowDesc{-1, p.items[src + r]} : RowDesc{-1 - src, -1};
         p.row_job[g] = j;
         p.row_local[g] = r;
     }
-    // (4) tiles.  Pass 1 picks each job's counter and sums the estimated cost of its
-    // CUDA-core tiles; pass 2 gives every CUDA-core job its own number of word slices (a
-    // heavy job -- dense prefix, many rows and columns -- is split so that no tile runs
-    // far longer than the wave's average) and forms the prefix sums the tile writers
-    // search.  Tensor-core jobs share one split-k factor.
-    const int64_t W = p.W;
-    const float P4 = (float)(W >> 2);
-    auto l3_cost = [&](const JobDesc& jd, const DJob& dj) -> float {
+    // (4) tiles.  Pass 1 picks each job's counter and sums the estimated cost of its CUDA-core
+    // tiles and the words of the others; pass 2 gives every job its own number of word slices (a
+    // heavy job -- dense prefix, many rows and columns, long rows -- is split so that no tile
+    // runs far longer than the wave's average) and forms the prefix sums the tile writers search.
+    auto l3_cost = [&](const JobDesc& jd, const DJob& dj, int32_t n) -> float {
         float d = 1.f;   // fraction of 128-bit base positions that are nonzero
-        if (dj.kind == kJobFam && (jd.base_slot >= 0 || jd.base_item >= 0) && p.n_bits > 0)
-            d = fminf(1.f, 128.f * (float)p.fams[dj.fam].sup / (float)p.n_bits);
+        if (dj.kind == kJobFam && (jd.base_slot >= 0 || jd.base_item >= 0) && n > 0)
+            d = fminf(1.f, 128.f * (float)dj.sup / (float)n);
         const float nr = (float)min(jd.n_rows, kLop3Rows), nc = (float)min(jd.n_cols, 64);
-        return P4 * (1.f + d * (2.f + nr + nr * nc / 32.f));
+        return (float)(jd.words >> 2) * (1.f + d * (2.f + nr + nr * nc / 32.f));
     };
-    float cost_local = 0.f;
-    int64_t tot1 = 0, tottc = 0, totgr = 0;
-    for (int base = 0; base < nj; base += kPackCand) {
-        int64_t a1[kPackItems], x1[kPackItems], at[kPackItems], xt[kPackItems], ag[kPackItems], xg[kPackItems];
-        for (int q = 0; q < kPackItems; q++) {
-            const int j = base + tid * kPackItems + q;
-            a1[q] = 0;
-            at[q] = 0;
-            ag[q] = 0;
-            if (j < nj) {
-                const JobDesc jd = p.jobs[j];
-                DJob* djp = p.djobs + j;
-                const bool fam = djp->kind == kJobFam;
-                const int32_t fsup = p.fams[djp->fam].sup;
-                int cls = kClsLop3;
-                if (fam && use_proj(p, jd, fsup)) {
-                    cls = kClsProj;
-                    const int32_t k = atomicAdd(&p.st->n_proj, 1);
-                    p.proj_list[k] = j;
-                } else if (fam && use_gram(p, jd, fsup)) {
-                    cls = kClsGram;
-                    ag[q] = 1;
-                } else if (fam && use_tc(p, jd, fsup)) {
-                    cls = kClsTc;
-                    at[q] = 1;
-                } else if (use_b1_shape(p, jd.n_rows, jd.n_cols) && fam) {
-                    cls = kClsB1;
-                    a1[q] = b1_tiles(jd.n_rows, jd.n_cols);
-                } else {
-                    cost_local += (float)l3_tiles(jd.n_rows, jd.n_cols) * l3_cost(jd, *djp);
-                }
-                djp->cls = cls;
-            }
-        }
-        Scan(tmp.scan).ExclusiveSum(a1, x1, s_agg);
-        __syncthreads();
-        const int64_t g1 = s_agg;
-        Scan(tmp.scan).ExclusiveSum(at, xt, s_agg);
-        __syncthreads();
-        const int64_t gt = s_agg;
-        Scan(tmp.scan).ExclusiveSum(ag, xg, s_agg);
-        __syncthreads();
-        const int64_t gg = s_agg;
-        for (int q = 0; q < kPackItems; q++) {
-            const int j = base + tid * kPackItems + q;
-            if (j < nj) {
-                p.djobs[j].b1 = (int32_t)(tot1 + x1[q]);
-                p.djobs[j].btc = (int32_t)(tottc + xt[q]);
-                p.djobs[j].bgr = (int32_t)(totgr + xg[q]);
-            }
-        }
-        tot1 += g1;
-        tottc += gt;
-        totgr += gg;
-        __syncthreads();
-    }
-    __shared__ float s_cost;
     {
-        typedef cub::BlockReduce<float, kPackThreads> RedF;
-        __shared__ typename RedF::TempStorage redf;
-        const float c = RedF(redf).Sum(cost_local);
-        if (tid == 0) s_cost = c;
+        float cost = 0.f;
+        unsigned long long w1 = 0, wt = 0, wg = 0;
+        for (int j = tid; j < nj; j += kPackThreads) {
+            const JobDesc jd = p.jobs[j];
+            const DJob dj = p.djobs[j];
+            const bool fam = dj.kind == kJobFam;
+            const int32_t n = p.fams[dj.fam].n;
+            int cls;
+            if (fam && use_proj(p, jd, dj.sup)) {
+                cls = kGrps;
+                p.proj_list[atomicAdd(&st->n_proj, 1)] = j;
+            } else if (fam && use_gram(p, jd, dj.sup, n)) {
+                cls = kGrpGram;
+                wg += (unsigned long long)jd.words;
+            } else if (fam && use_tc(p, jd, dj.sup, n)) {
+                cls = kGrpTc;
+                wt += (unsigned long long)jd.words;
+            } else if (fam && use_b1_shape(p, jd.n_rows, jd.n_cols)) {
+                cls = kGrpB1;
+                w1 += (unsigned long long)(b1_tiles(jd.n_rows, jd.n_cols) * jd.words);
+            } else {
+                // Tiles of dense families and of their lookaheads (the family's prefix holds at
+                // least 1/16 of its transactions, so no 128-bit position is zero to skip) come
+                // first, for the register-blocked dense launch
+                cls = 16 * (int64_t)dj.sup >= n ? kGrpDense : kGrpLight;
+                cost += (float)l3_tiles(jd.n_rows, jd.n_cols) * l3_cost(jd, dj, n);
+            }
+            p.djobs[j].cls = cls;
+            p.djobs[j].pad = n;
+        }
+        if ((tid & ~31) < nj) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                cost += __shfl_xor_sync(0xffffffffu, cost, o);
+                w1 += __shfl_xor_sync(0xffffffffu, w1, o);
+                wt += __shfl_xor_sync(0xffffffffu, wt, o);
+                wg += __shfl_xor_sync(0xffffffffu, wg, o);
+            }
+            if (lane == 0) {
+                atomicAdd(&s_cost, cost);
+                if (w1) atomicAdd(&s_words[0], w1);
+                if (wt) atomicAdd(&s_words[1], wt);
+                if (wg) atomicAdd(&s_words[2], wg);
+            }
+        }
         __syncthreads();
     }
     // the wave's estimated CUDA-core cost over (slices per SM x SMs): the cost of one tile
@@ -580,84 +611,50 @@ __device__ __forceinline__ void res_pack(const ResPtrs& p) {
     // launch's tail on large dense databases
     const float target = fmaxf(s_cost / (p.l3_slices_per_sm * (float)p.sm_count), 1.f);
     const float target_d = fmaxf(s_cost / (p.l3_dense_slices_per_sm * (float)p.sm_count), 1.f);
-    const int64_t max_sl = lmax(1, W / 256);
-    // Tiles of dense families and of their lookaheads (the family's prefix holds at least 1/16
-    // of the transactions, so no 128-bit position is zero to skip) come first, for the
-    // register-blocked dense launch;
-    // then heavy jobs (cost at least half the slice target), so that the longest tiles are
-    // dispatched first and the light ones fill in behind them.
-    int64_t tot3d = 0, tot3h = 0, tot3l = 0;
-    for (int base = 0; base < nj; base += kPackCand) {
-        int64_t ad[kPackItems], ah[kPackItems], al[kPackItems], xd[kPackItems], xh[kPackItems], xl[kPackItems];
-        for (int q = 0; q < kPackItems; q++) {
-            const int j = base + tid * kPackItems + q;
-            ad[q] = ah[q] = al[q] = 0;
-            if (j < nj) {
-                const JobDesc jd = p.jobs[j];
-                DJob* djp = p.djobs + j;
-                if (djp->cls == 0) {
-                    const float cost = l3_cost(jd, *djp);
-                    // a family job, or the lookahead of a family (its head-union-tail mask is a subset
-                    // of the family's prefix, and on a dense family almost never zero per 128 bits)
-                    const bool dense = 16 * (int64_t)p.fams[djp->fam].sup >= p.n_bits;
-                    int64_t sl = lmin(max_sl, lmax(1, (int64_t)ceilf(cost / (dense ? target_d : target))));
-                    const int64_t wsl = ((W / 64 + sl - 1) / sl) * 64;
-                    sl = wsl > 0 ? (W + wsl - 1) / wsl : 1;
-                    djp->sl3 = (int32_t)sl;
-                    djp->heavy = dense ? 2 : cost >= 0.5f * target ? 1 : 0;
-                    const int64_t nt = l3_tiles(jd.n_rows, jd.n_cols) * sl;
-                    if (djp->heavy == 2) ad[q] = nt;
-                    else if (djp->heavy) ah[q] = nt;
-                    else al[q] = nt;
-                }
+    const int64_t sw_b1 = slice_words((int64_t)s_words[0], (int64_t)(p.b1_tiles_per_sm * (float)p.sm_count));
+    const int64_t sw_tc = slice_words((int64_t)s_words[1], (int64_t)(p.tc_tiles_per_sm * (float)p.sm_count));
+    const int64_t sw_gr = slice_words((int64_t)s_words[2], (int64_t)(p.l3_slices_per_sm * (float)p.sm_count));
+    int32_t tot[kGrps] = {0, 0, 0, 0, 0, 0};
+    for (int base = 0; base < nj; base += kPackThreads) {
+        const int j = base + tid;
+        int32_t v[kGrps] = {0, 0, 0, 0, 0, 0}, ex[kGrps], t[kGrps];
+        if (j < nj) {
+            const JobDesc jd = p.jobs[j];
+            DJob* djp = p.djobs + j;
+            const DJob dj = *djp;
+            const int64_t W = jd.words;
+            int64_t sl = 1, per = 1;   // word slices, tiles per slice
+            int cls = dj.cls;
+            if (cls <= kGrpLight) {
+                const float cost = l3_cost(jd, dj, dj.pad);
+                sl = lmin(lmax(1, W / 256), lmax(1, (int64_t)ceilf(cost / (cls == kGrpDense ? target_d : target))));
+                // heavy jobs (cost at least half the slice target) before the light ones, so that the
+                // longest tiles are dispatched first and the light ones fill in behind them
+                if (cls == kGrpLight && cost >= 0.5f * target) cls = kGrpHeavy;
+                per = l3_tiles(jd.n_rows, jd.n_cols);
+            } else if (cls < kGrps) {
+                const int64_t sw = cls == kGrpB1 ? sw_b1 : cls == kGrpTc ? sw_tc : sw_gr;
+                sl = (W + sw - 1) / sw;
+                if (cls == kGrpB1) per = b1_tiles(jd.n_rows, jd.n_cols);
+            }
+            if (cls < kGrps) {
+                const int64_t wsl = ((W / 64 + sl - 1) / sl) * 64;
+                sl = wsl > 0 ? (W + wsl - 1) / wsl : 1;
+                djp->sl3 = (int32_t)sl;
+                djp->cls = cls;
+#pragma unroll
+                for (int k = 0; k < kGrps; k++) v[k] = k == cls ? (int32_t)lmin(per * sl, 1 << 30) : 0;
             }
         }
-        Scan(tmp.scan).ExclusiveSum(ad, xd, s_agg);
-        __syncthreads();
-        const int64_t gd = s_agg;
-        Scan(tmp.scan).ExclusiveSum(ah, xh, s_agg);
-        __syncthreads();
-        const int64_t gh = s_agg;
-        Scan(tmp.scan).ExclusiveSum(al, xl, s_agg);
-        __syncthreads();
-        const int64_t gl = s_agg;
-        for (int q = 0; q < kPackItems; q++) {
-            const int j = base + tid * kPackItems + q;
-            if (j < nj) {
-                p.djobs[j].b3d = (int32_t)(tot3d + xd[q]);
-                p.djobs[j].b3 = (int32_t)(tot3h + xh[q]);
-                p.djobs[j].b3l = (int32_t)(tot3l + xl[q]);
-            }
-        }
-        tot3d += gd;
-        tot3h += gh;
-        tot3l += gl;
-        __syncthreads();
+        block_scan<kGrps>(v, ex, t, sm32, base + (tid & ~31) < nj);
+        if (j < nj)
+#pragma unroll
+            for (int k = 0; k < kGrps; k++) p.djobs[j].pre[k] = tot[k] + ex[k];
+#pragma unroll
+        for (int k = 0; k < kGrps; k++) tot[k] += t[k];
     }
-    const int64_t tot3 = tot3d + tot3h + tot3l;
-    const int64_t want1 = lmax(1, (int64_t)(p.b1_tiles_per_sm * (float)p.sm_count));
-    int64_t ks1 = tot1 > 0 ? lmax(1, (want1 + tot1 - 1) / tot1) : 1;
-    ks1 = lmin(ks1, lmax(1, W / 64));
-    int64_t kslice = ((W / 64 + ks1 - 1) / ks1) * 64;
-    if (kslice <= 0) kslice = 64;
-    const int64_t nk = W > 0 ? (W + kslice - 1) / kslice : 1;
-    const int64_t T3 = tot3, T1 = tot1 * nk;
-    // tcgen05 family tiles: every job whole, over `sltc` word slices (multiples of 64 words)
-    const int64_t want_tc = lmax(1, (int64_t)(p.tc_tiles_per_sm * (float)p.sm_count));
-    int64_t sltc = tottc > 0 ? lmax(1, (want_tc + tottc - 1) / tottc) : 1;
-    sltc = lmin(sltc, lmax(1, W / 64));
-    int64_t wsltc = ((W / 64 + sltc - 1) / sltc) * 64;
-    if (wsltc <= 0) wsltc = 64;
-    const int64_t ntc = W > 0 ? (W + wsltc - 1) / wsltc : 1;
-    const int64_t TT = tottc * ntc;
-    // CUDA-core Gram tiles: every job whole, over `slgr` word slices (multiples of 64 words)
-    const int64_t want_gr = lmax(1, (int64_t)(p.l3_slices_per_sm * (float)p.sm_count));
-    int64_t slgr = totgr > 0 ? lmax(1, (want_gr + totgr - 1) / totgr) : 1;
-    slgr = lmin(slgr, lmax(1, W / 64));
-    int64_t wslgr = ((W / 64 + slgr - 1) / slgr) * 64;
-    if (wslgr <= 0) wslgr = 64;
-    const int64_t ngr = W > 0 ? (W + wslgr - 1) / wslgr : 1;
-    const int64_t TG = totgr * ngr;
+    const int64_t T3 = (int64_t)tot[kGrpDense] + tot[kGrpHeavy] + tot[kGrpLight], T1 = tot[kGrpB1], TT = tot[kGrpTc],
+                  TG = tot[kGrpGram];
     // the wave is committed only when the worst case of its expand fits the pools
     if (tid == 0) {
         const bool fit = s_out_total <= p.cap_out && T1 <= p.cap_tiles && T3 <= p.cap_tiles && TT <= p.cap_tiles &&
@@ -672,115 +669,106 @@ __device__ __forceinline__ void res_pack(const ResPtrs& p) {
             st->g_max_head = s_max_head;
             st->g_max_cols = s_max_cols;
             st->g_tiles = lmax(lmax(lmax(T1, T3), TT), TG);
-        }
-    }
-    __syncthreads();
-    if (!s_fit) {
-        if (tid == 0) {
             st->jobs = 0; st->rows = 0; st->tiles_l3 = 0; st->tiles_l3d = 0; st->tiles_b1 = 0; st->tiles_tc = 0;
             st->tiles_gr = 0; st->n_proj = 0;
             st->out_total = 0;
             st->ph_e[kPhPack] = globaltimer();
         }
-        return;
     }
-    // commit: the families hand out their rows
-    for (int j = n_look + tid; j < nj; j += kPackThreads) {
-        const DJob dj = p.djobs[j];
-        p.fams[dj.fam].next_row = dj.r0 + dj.nr;
-    }
-    // the wave's work per counter class (warp sums, one atomic per warp and class)
+    __syncthreads();   // s_fit; s_pre is free
+    if (!s_fit) return;
+    // commit: the families hand out their rows; the wave's work per counter class (warp sums, one
+    // atomic per warp and class)
     {
         unsigned long long cb[kClasses], cbo[kClasses], cs[kClasses], cj[kClasses];
 #pragma unroll
         for (int k = 0; k < kClasses; k++) cb[k] = cbo[k] = cs[k] = cj[k] = 0;
         for (int j = tid; j < nj; j += kPackThreads) {
             const JobDesc jd = p.jobs[j];
-            const int cls = p.djobs[j].cls;
+            const DJob dj = p.djobs[j];
+            if (dj.kind == kJobFam) p.fams[dj.fam].next_row = dj.r0 + dj.nr;
+            const int cls = dj.cls <= kGrpLight ? kClsLop3
+                            : dj.cls == kGrpB1  ? kClsB1
+                            : dj.cls == kGrpTc  ? kClsTc
+                            : dj.cls == kGrpGram ? kClsGram
+                                                 : kClsProj;
             const unsigned long long nbase = (jd.base_slot >= 0) + (jd.base_item >= 0);
             const unsigned long long sup = (unsigned long long)jd.n_rows * (unsigned long long)jd.n_cols;
-            const unsigned long long by =
-                (unsigned long long)p.row_bytes * ((unsigned long long)jd.n_rows + jd.n_cols + nbase) + 4ull * sup;
+            const unsigned long long by = (unsigned long long)((dj.pad + 7) / 8) *
+                                              ((unsigned long long)jd.n_rows + jd.n_cols + nbase) + 4ull * sup;
 #pragma unroll
             for (int k = 0; k < kClasses; k++)
                 if (cls == k) {
                     cb[k] += by;
-                    cbo[k] += sup * (unsigned long long)p.n_bits;
+                    cbo[k] += sup * (unsigned long long)dj.pad;
                     cs[k] += sup;
                     cj[k] += 1;
                 }
         }
+        if ((tid & ~31) < nj) {
 #pragma unroll
-        for (int k = 0; k < kClasses; k++) {
+            for (int k = 0; k < kClasses; k++) {
+                if (!__any_sync(0xffffffffu, cj[k] != 0)) continue;
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                cb[k] += __shfl_xor_sync(0xffffffffu, cb[k], o);
-                cbo[k] += __shfl_xor_sync(0xffffffffu, cbo[k], o);
-                cs[k] += __shfl_xor_sync(0xffffffffu, cs[k], o);
-                cj[k] += __shfl_xor_sync(0xffffffffu, cj[k], o);
-            }
-            if ((tid & 31) == 0 && cj[k]) {
-                atomicAdd(&st->cls_bytes[k], cb[k]);
-                atomicAdd(&st->cls_bitops[k], cbo[k]);
-                atomicAdd(&st->cls_sup[k], cs[k]);
-                atomicAdd(&st->cls_jobs[k], cj[k]);
+                for (int o = 16; o > 0; o >>= 1) {
+                    cb[k] += __shfl_xor_sync(0xffffffffu, cb[k], o);
+                    cbo[k] += __shfl_xor_sync(0xffffffffu, cbo[k], o);
+                    cs[k] += __shfl_xor_sync(0xffffffffu, cs[k], o);
+                    cj[k] += __shfl_xor_sync(0xffffffffu, cj[k], o);
+                }
+                if (lane == 0) {
+                    atomicAdd(&st->cls_bytes[k], cb[k]);
+                    atomicAdd(&st->cls_bitops[k], cbo[k]);
+                    atomicAdd(&st->cls_sup[k], cs[k]);
+                    atomicAdd(&st->cls_jobs[k], cj[k]);
+                }
             }
         }
     }
-    if (T3 <= p.cap_tiles)
-        for (int64_t t = tid; t < T3; t += kPackThreads) {
-            const int grp = t < tot3d ? 0 : t < tot3d + tot3h ? 1 : 2;   // dense, heavy, light
-            const int j = grp == 0   ? find_job_by_tile<5>(p.djobs, nj, t)
-                          : grp == 1 ? find_job_by_tile<0>(p.djobs, nj, t - tot3d)
-                                     : find_job_by_tile<2>(p.djobs, nj, t - tot3d - tot3h);
+    // the tiles of one group: `base` = the group's first entry of its tile list
+    auto emit = [&](int grp, TileDesc* out, int64_t first) {
+        const int32_t n = tot[grp];
+        if (n == 0) return;
+        if (in_sm) {
+            for (int j = tid; j < nj; j += kPackThreads) s_pre[j] = p.djobs[j].pre[grp];
+            __syncthreads();
+        }
+        for (int32_t t = tid; t < n; t += kPackThreads) {
+            // the job owning tile t: jobs of other groups share the prefix of the next one of this group
+            const int j = in_sm ? last_le([&](int k) { return s_pre[k]; }, nj, t)
+                                : last_le([&](int k) { return p.djobs[k].pre[grp]; }, nj, t);
             const JobDesc jd = p.jobs[j];
             const DJob dj = p.djobs[j];
-            const int64_t local = grp == 0 ? t - dj.b3d : grp == 1 ? t - tot3d - dj.b3 : t - tot3d - tot3h - dj.b3l;
-            const int64_t bt = l3_tiles(jd.n_rows, jd.n_cols);
-            const int64_t slice = local / bt, within = local % bt;
-            const int64_t wsl = ((W / 64 + dj.sl3 - 1) / dj.sl3) * 64;
-            const int cg = (jd.n_cols + 63) / 64;
-            const int rg = (int)(within / cg), cc = (int)(within % cg);
-            const int64_t w0 = slice * wsl;
-            p.tiles_l3[t] = TileDesc{j, rg * kLop3Rows, min(kLop3Rows, jd.n_rows - rg * kLop3Rows), cc * 64,
-                                     min(jd.n_cols, cc * 64 + 64), (int32_t)w0, (int32_t)lmin(W, w0 + wsl), grp == 0 ? 1 : 0};
+            const int32_t local = t - dj.pre[grp];
+            const int64_t W = jd.words, wsl = ((W / 64 + dj.sl3 - 1) / dj.sl3) * 64;
+            if (grp >= kGrpTc) {
+                // rows 0 .. n_rows of the job are its columns dj.r0 .. dj.r0 + n_rows
+                const int64_t w0 = local * wsl;
+                out[first + t] = TileDesc{j, 0, jd.n_rows, 0, jd.n_cols, (int32_t)w0, (int32_t)lmin(W, w0 + wsl), dj.r0};
+            } else {
+                const int tr = grp == kGrpB1 ? kB1Rows : kLop3Rows, tc = grp == kGrpB1 ? kB1Cols : 64;
+                const int cg = (jd.n_cols + tc - 1) / tc;
+                const int bt = cg * ((jd.n_rows + tr - 1) / tr);
+                const int slice = local / bt, within = local - slice * bt;
+                const int rg = within / cg, cc = within - rg * cg;
+                const int64_t w0 = slice * wsl;
+                out[first + t] = TileDesc{j, rg * tr, min(tr, jd.n_rows - rg * tr), cc * tc, min(jd.n_cols, cc * tc + tc),
+                                          (int32_t)w0, (int32_t)lmin(W, w0 + wsl), grp == kGrpDense ? 1 : 0};
+            }
         }
-    if (T1 <= p.cap_tiles)
-        for (int64_t t = tid; t < T1; t += kPackThreads) {
-            const int64_t slice = t / tot1, local = t % tot1;
-            const int j = find_job_by_tile<1>(p.djobs, nj, local);
-            const JobDesc jd = p.jobs[j];
-            const int64_t within = local - p.djobs[j].b1;
-            const int cg = (jd.n_cols + kB1Cols - 1) / kB1Cols;
-            const int rg = (int)(within / cg), cc = (int)(within % cg);
-            const int64_t w0 = slice * kslice;
-            p.tiles_b1[t] = TileDesc{j, rg * kB1Rows, min(kB1Rows, jd.n_rows - rg * kB1Rows), cc * kB1Cols,
-                                     min(jd.n_cols, cc * kB1Cols + kB1Cols), (int32_t)w0, (int32_t)lmin(W, w0 + kslice), 0};
-        }
-    if (TT <= p.cap_tiles)
-        for (int64_t t = tid; t < TT; t += kPackThreads) {
-            const int64_t slice = t / tottc, local = t % tottc;
-            const int j = find_job_by_tile<3>(p.djobs, nj, local);
-            const JobDesc jd = p.jobs[j];
-            const int64_t w0 = slice * wsltc;
-            // rows 0 .. n_rows of the job are its columns dj.r0 .. dj.r0 + n_rows
-            p.tiles_tc[t] = TileDesc{j, 0, jd.n_rows, 0, jd.n_cols, (int32_t)w0, (int32_t)lmin(W, w0 + wsltc),
-                                     p.djobs[j].r0};
-        }
-    if (TG <= p.cap_tiles)
-        for (int64_t t = tid; t < TG; t += kPackThreads) {
-            const int64_t slice = t / totgr, local = t % totgr;
-            const int j = find_job_by_tile<4>(p.djobs, nj, local);
-            const JobDesc jd = p.jobs[j];
-            const int64_t w0 = slice * wslgr;
-            p.tiles_gr[t] = TileDesc{j, 0, jd.n_rows, 0, jd.n_cols, (int32_t)w0, (int32_t)lmin(W, w0 + wslgr),
-                                     p.djobs[j].r0};
-        }
+        __syncthreads();   // s_pre is reused
+    };
+    emit(kGrpDense, p.tiles_l3, 0);
+    emit(kGrpHeavy, p.tiles_l3, tot[kGrpDense]);
+    emit(kGrpLight, p.tiles_l3, (int64_t)tot[kGrpDense] + tot[kGrpHeavy]);
+    emit(kGrpB1, p.tiles_b1, 0);
+    emit(kGrpTc, p.tiles_tc, 0);
+    emit(kGrpGram, p.tiles_gr, 0);
     if (tid == 0) {
         st->jobs = nj;
         st->rows = rows_total;
         st->tiles_l3 = (int32_t)T3;
-        st->tiles_l3d = (int32_t)tot3d;
+        st->tiles_l3d = tot[kGrpDense];
         st->tiles_b1 = (int32_t)T1;
         st->tiles_tc = (int32_t)TT;
         st->tiles_gr = (int32_t)TG;
@@ -1256,6 +1244,7 @@ __device__ void expand_row(const ResPtrs& p, int64_t g, int lane) {
         ch.slot = cslot; ch.item = citem; ch.head_off = hoff; ch.head_len = head_len;
         ch.F_off = foff; ch.nF = n_rest; ch.nT = n_tail; ch.sup = supc;
         ch.next_row = 0; ch.rows_done = 0; ch.state = issue ? 1 : 0; ch.top = 0;
+        ch.W = f.W; ch.n = f.n;
         p.fams[fid] = ch;
     }
     if (issue) {
@@ -1926,6 +1915,7 @@ int mine_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt) {
     DFam top;
     top.slot = -1; top.item = -1; top.head_off = 0; top.head_len = 0; top.F_off = 0; top.nF = n0; top.nT = n0;
     top.sup = 0; top.next_row = n0; top.rows_done = 0; top.state = 0; top.top = 1;
+    top.W = (int32_t)W; top.n = (int32_t)c->n_bits;
     ResStatus hs;
     memset(&hs, 0, sizeof hs);
     for (int k = 0; k < kPhases; k++) hs.ph_s[k] = ~0ull;
@@ -1964,8 +1954,12 @@ int mine_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt) {
             memcpy(at(p_freq), c->dense_freq.data(), c->dense_freq.size() * 4);
             memcpy(at(p_fam), &top, sizeof top);
             memcpy(at(p_F), F0.data(), (size_t)n0 * 4);
-            *(DJob*)at(p_dj) = DJob{0, kJobFam, 0, n0, -1, -1, 0, 0, 0, 1, 0, 0, 0, 0};
-            *(JobDesc*)at(p_jd) = JobDesc{-1, -1, n0, n0, 0, 0, 0, -1, 0};
+            {
+                DJob dj{};
+                dj.kind = kJobFam; dj.nr = n0; dj.slot = -1; dj.log = -1; dj.sl3 = 1;
+                *(DJob*)at(p_dj) = dj;
+            }
+            *(JobDesc*)at(p_jd) = JobDesc{-1, -1, n0, n0, 0, 0, 0, -1, (int32_t)W};
             RowDesc* rows = (RowDesc*)at(p_rows);
             int32_t* rj = (int32_t*)at(p_rj);
             int32_t* rl = (int32_t*)at(p_rl);

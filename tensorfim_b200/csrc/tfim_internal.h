@@ -90,7 +90,7 @@ struct JobDesc {
     int32_t col_off;      // into the column table
     int64_t out_off;      // into the counts buffer
     int32_t self_col;     // column index that stands for all ones (not read from the table), or -1
-    int32_t pad;
+    int32_t words;        // words per row of the job's transactions (resident pack)
 };
 struct RowDesc {
     int32_t slot;
