@@ -78,7 +78,7 @@ __device__ void b1_tile(const CountArgs& a, const TileDesc t, unsigned char* sme
         if (r < t.nr) {
             const RowDesc rd = a.rows[j.row_off + t.r0 + r];
             if (rd.slot >= 0) { row_src[r] = a.masks + (int64_t)rd.slot * W; row_kind[r] = 0; }
-            else if (rd.item >= 0) { row_src[r] = a.bitmap + (int64_t)rd.item * W; row_kind[r] = 0; }
+            else if (rd.item >= 0) { row_src[r] = item_row(a, rd.item); row_kind[r] = 0; }
             else { row_src[r] = nullptr; row_kind[r] = 1; }
         } else {
             row_src[r] = nullptr;
@@ -88,7 +88,7 @@ __device__ void b1_tile(const CountArgs& a, const TileDesc t, unsigned char* sme
         const int c = tid - 64;
         if (t.c0 + c < t.c1) {
             const int32_t col = (t.c0 + c) == j.self_col ? -1 : a.cols[j.col_off + t.c0 + c];
-            if (col >= 0) { col_src[c] = a.bitmap + (int64_t)col * W; col_kind[c] = 0; }
+            if (col >= 0) { col_src[c] = item_row(a, col); col_kind[c] = 0; }
             else { col_src[c] = nullptr; col_kind[c] = 1; }
         } else {
             col_src[c] = nullptr;
@@ -96,7 +96,7 @@ __device__ void b1_tile(const CountArgs& a, const TileDesc t, unsigned char* sme
         }
     }
     const uint32_t* base_m = j.base_slot >= 0 ? a.masks + (int64_t)j.base_slot * W : nullptr;
-    const uint32_t* base_i = j.base_item >= 0 ? a.bitmap + (int64_t)j.base_item * W : nullptr;
+    const uint32_t* base_i = j.base_item >= 0 ? item_row(a, j.base_item) : nullptr;
     const bool has_base = base_m || base_i;
     __syncthreads();
 

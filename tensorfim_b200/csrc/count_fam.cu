@@ -254,9 +254,9 @@ __global__ void __launch_bounds__(kFThreads, 1) k_count_fam(CountArgs a_val, con
             const bool active = lane < (nrw << kb_log);
             const int q = lane >> kb_log, kb = lane & (KB - 1);
             const int r = e + q * kFExpWarps;
-            const uint32_t* src = active ? a.bitmap + (int64_t)a.cols[j.col_off + r] * W : nullptr;
+            const uint32_t* src = active ? item_row(a, a.cols[j.col_off + r]) : nullptr;
             const uint32_t* bm = j.base_slot >= 0 ? a.masks + (int64_t)j.base_slot * W : nullptr;
-            const uint32_t* bi = j.base_item >= 0 ? a.bitmap + (int64_t)j.base_item * W : nullptr;
+            const uint32_t* bi = j.base_item >= 0 ? item_row(a, j.base_item) : nullptr;
             const int64_t w_unit = t.w0 + (int64_t)kb * 4;   // + st * stage_words
             const uint4 ones = make_uint4(~0u, ~0u, ~0u, ~0u);
             uint4 pr[kFAhead], pm[kFAhead], pi[kFAhead];

@@ -69,9 +69,9 @@ __device__ void gram_tile_t(const CountArgs& a, const TileDesc t, uint8_t* smem,
     // the staged rows' sources (shared: the columns, then the base's)
     for (int q = tid; q < rows; q += kGThreads) {
         const uint32_t* src;
-        if (q < nF) src = a.bitmap + (int64_t)a.cols[j.col_off + q] * W;
+        if (q < nF) src = item_row(a, a.cols[j.col_off + q]);
         else if (q == nF && j.base_slot >= 0) src = a.masks + (int64_t)j.base_slot * W;
-        else src = a.bitmap + (int64_t)j.base_item * W;
+        else src = item_row(a, j.base_item);
         rowp[q] = src;
     }
     __syncthreads();

@@ -52,11 +52,11 @@ __device__ void lop3_tile_impl(const CountArgs& a, const TileDesc t, Lop3Shared&
     if (tid < kLop3Rows && tid < nr) {
         const RowDesc rd = a.rows[j.row_off + t.r0 + tid];
         sh.rsrc[tid][0] = rd.slot >= 0 ? reinterpret_cast<const uint4*>(a.masks + (int64_t)rd.slot * W) : nullptr;
-        sh.rsrc[tid][1] = rd.item >= 0 ? reinterpret_cast<const uint4*>(a.bitmap + (int64_t)rd.item * W) : nullptr;
+        sh.rsrc[tid][1] = rd.item >= 0 ? reinterpret_cast<const uint4*>(item_row(a, rd.item)) : nullptr;
     }
     for (int q = tid; q < kLop3Rows * 64; q += blockDim.x) sh.acc[q] = 0;
     const uint4* base_m = j.base_slot >= 0 ? reinterpret_cast<const uint4*>(a.masks + (int64_t)j.base_slot * W) : nullptr;
-    const uint4* base_i = j.base_item >= 0 ? reinterpret_cast<const uint4*>(a.bitmap + (int64_t)j.base_item * W) : nullptr;
+    const uint4* base_i = j.base_item >= 0 ? reinterpret_cast<const uint4*>(item_row(a, j.base_item)) : nullptr;
     // flush layout: G staged positions per pass, lane -> (position offset, column(s))
     constexpr bool wide = WIDE;
     constexpr int NC = WIDE ? 2 : 1;   // columns per lane
@@ -76,7 +76,7 @@ __device__ void lop3_tile_impl(const CountArgs& a, const TileDesc t, Lop3Shared&
             if (col < 0) ck[ci] = 1;   // the all-ones column
             else {
                 ck[ci] = 0;
-                cp[ci] = reinterpret_cast<const uint4*>(a.bitmap + (int64_t)col * W);
+                cp[ci] = reinterpret_cast<const uint4*>(item_row(a, col));
             }
         }
     }
@@ -214,7 +214,7 @@ __device__ void lop3_dense_impl(const CountArgs& a, const TileDesc t, int32_t* s
     const int br = busy ? (b / cb) * BR : 0, bc = busy ? (b % cb) * BC : 0;
     for (int q = tid; q < kLop3Rows * 64; q += blockDim.x) sacc[q] = 0;
     const uint4* base_m = j.base_slot >= 0 ? reinterpret_cast<const uint4*>(a.masks + (int64_t)j.base_slot * W) : nullptr;
-    const uint4* base_i = j.base_item >= 0 ? reinterpret_cast<const uint4*>(a.bitmap + (int64_t)j.base_item * W) : nullptr;
+    const uint4* base_i = j.base_item >= 0 ? reinterpret_cast<const uint4*>(item_row(a, j.base_item)) : nullptr;
     // sources of the block's rows and columns, clamped to the tile's last row / column (pairs
     // outside the tile are computed on valid rows and discarded); a null source is all ones
     const uint4* rsl[BR];
@@ -224,13 +224,13 @@ __device__ void lop3_dense_impl(const CountArgs& a, const TileDesc t, int32_t* s
     for (int x = 0; x < BR; x++) {
         const RowDesc rd = a.rows[j.row_off + t.r0 + min(br + x, nr - 1)];
         rsl[x] = rd.slot >= 0 ? reinterpret_cast<const uint4*>(a.masks + (int64_t)rd.slot * W) : nullptr;
-        rit[x] = rd.item >= 0 ? reinterpret_cast<const uint4*>(a.bitmap + (int64_t)rd.item * W) : nullptr;
+        rit[x] = rd.item >= 0 ? reinterpret_cast<const uint4*>(item_row(a, rd.item)) : nullptr;
     }
 #pragma unroll
     for (int y = 0; y < BC; y++) {
         const int c = t.c0 + min(bc + y, nc - 1);
         const int32_t col = c == j.self_col ? -1 : a.cols[j.col_off + c];
-        csrc[y] = col >= 0 ? reinterpret_cast<const uint4*>(a.bitmap + (int64_t)col * W) : nullptr;
+        csrc[y] = col >= 0 ? reinterpret_cast<const uint4*>(item_row(a, col)) : nullptr;
     }
     uint32_t acc[BR][BC];
 #pragma unroll

@@ -137,11 +137,19 @@ struct CountArgs {
     int32_t n_tiles;
     int32_t* out;
     const int32_t* job_list;   // projected counter: the jobs it counts
+    // Rows of projected families (resident engine): ids from n_base on are vrows[id - n_base]
+    const uint32_t* const* vrows = nullptr;
+    int32_t n_base = 0x7fffffff;
     // phase stamps of the launch (or nullptr): the earliest block start and the latest block
     // end, in %globaltimer nanoseconds (phase_begin / phase_end)
     unsigned long long* ph_s = nullptr;
     unsigned long long* ph_e = nullptr;
 };
+
+// The bitmap row of an item id (or of a projected family's row).
+__device__ __forceinline__ const uint32_t* item_row(const CountArgs& a, int32_t id) {
+    return id < a.n_base ? a.bitmap + (int64_t)id * a.W : a.vrows[id - a.n_base];
+}
 
 __device__ __forceinline__ unsigned long long dev_globaltimer() {
     unsigned long long t;
