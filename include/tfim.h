@@ -45,9 +45,8 @@ typedef struct tfim_ctx tfim_ctx;
 #define TFIM_COUNTER_AUTO    0   /* chosen per job from its shape */
 #define TFIM_COUNTER_LOP3    1   /* AND + popc on CUDA cores */
 #define TFIM_COUNTER_TENSOR  2   /* b1 AND+POPC tensor-core MMA */
-#define TFIM_COUNTER_I8      4   /* tcgen05 tensor-core tiles: waves and the empty prefix's family
-                                    on the bits expanded to 4-bit values (kind::mxf4), other
-                                    families expanded to bytes (kind::i8) */
+#define TFIM_COUNTER_I8      4   /* tcgen05 tensor-core tiles on the bits expanded to 4-bit values
+                                    (kind::mxf4) */
 #define TFIM_COUNTER_PROJ    3   /* resident engine: projected counting (prefix transactions x
                                     the reduced transaction list) wherever it applies, else auto */
 

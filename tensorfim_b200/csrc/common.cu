@@ -159,7 +159,7 @@ void tuning_builtin(tfim_tuning* t) {
     t->i8_min_rows = 3;
     t->i8_min_cols = 1;
     t->rate_i8_bitops = 2.0e15;
-    t->tc_min_work = 1536;
+    t->tc_min_work = 64;
     t->tc_min_density = 0.5f;
     t->tc_tiles_per_sm = 8.f;
     t->gram_min_rows = 32;

@@ -18,6 +18,7 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstring>
@@ -89,7 +90,7 @@ struct ResStatus {
     int64_t g_out, g_tiles;
     int32_t launch_id, next3, next1;         // next3 / next1: tile counters of the persistent counters
     int32_t tiles_l3d;                       // the first tiles_l3d CUDA-core tiles are dense families'
-    int32_t tiles_tc, next_tc;               // tcgen05 family counter: tiles, tile counter
+    int32_t tiles_tc, pad3;                  // packed tcgen05 family counter: tiles
     int32_t tiles_gr, next_gr;               // CUDA-core Gram counter: tiles, tile counter
     unsigned long long launch_t0;
     unsigned long long supports, nodes, lookaheads, hits, skipped, pep;
@@ -143,6 +144,7 @@ struct ResPtrs {
     TileDesc* tiles_b1;
     TileDesc* tiles_tc;
     TileDesc* tiles_gr;
+    int32_t* pk_list;             // jobs of each packed tile (kPkJobs entries)
     int32_t* counts;
     // constants
     const uint32_t* bitmap;
@@ -233,35 +235,53 @@ __device__ __forceinline__ bool use_proj(const ResPtrs& p, const JobDesc& jd, in
 __host__ __device__ __forceinline__ int64_t lmin(int64_t a, int64_t b) { return a < b ? a : b; }
 __host__ __device__ __forceinline__ int64_t lmax(int64_t a, int64_t b) { return a > b ? a : b; }
 
+// Packed tcgen05 counter, automatic choice: a 128-column tile costs about 128 cycles per 64
+// transactions whatever its jobs' tail rows, a register-blocked CUDA-core tile about 0.17 per
+// row and column; on the 6.3M-row dense database the counting of the later waves took 20.1 / 18.1
+// ms from 4 / 8 tail rows on.  Short rows stay with the CUDA cores, whose launch is the
+// shorter one (10,000 rows, W = 320: 0.71 against 0.66 ms a mine).
+constexpr int kPkMinRows = 8, kPkMinWords = 1024;
+// and, over the wave, rows x columns x words, below which the second launch and its packing cost more
+// than they save (a 1M-row sparse mine 1.69 / 1.72 ms with its one packed wave on the CUDA cores /
+// packed; a 49,000-row dense one 2.62 / 2.56 ms with its waves below 2e8 / 5e7 on the CUDA cores).
+constexpr float kPkMinWork = 1e8f;
+// Narrow dense families of short rows stay with the Gram counter: 49,000 / 98,000 / 196,000 rows of
+// the dense database mine in 2.57 / 3.27 / 3.50 ms with it and 2.56 / 3.25 / 3.49 ms with their jobs in
+// packed tiles, the same within a launch.
+constexpr int kGramMaxWords = 4096;
+
 constexpr int kPackThreads = 1024;
 constexpr int kPackItems = 4;
 constexpr int kPackCand = kPackThreads * kPackItems;
 
-// The tcgen05 family counter takes a family job (its rows are a run of its columns) of at
-// most kFamMaxCols columns: always when that counter is asked for, and in the automatic choice
-// when the job is large enough and its prefix dense enough that skipping zero words (which
-// the CUDA-core tiles do and the tensor tiles do not) saves little.
+// The packed tcgen05 counter takes a family job (its rows are a run of its columns) of at most
+// kPkMaxCols columns: always when that counter is asked for, and in the automatic choice from
+// kPkMinRows tail rows on when its prefix is dense enough that skipping zero words (which the
+// CUDA-core tiles do and the tensor tiles do not) saves little.
 __device__ __forceinline__ bool use_tc(const ResPtrs& p, const JobDesc& jd, int32_t sup, int32_t n) {
-    if (jd.n_cols < 1 || jd.n_cols > kFamMaxCols || jd.n_rows < 1) return false;
+    if (jd.n_cols < 1 || jd.n_cols > kPkMaxCols || jd.n_rows < 1) return false;
     if (p.counter == TFIM_COUNTER_I8) return true;
     if (p.counter != TFIM_COUNTER_AUTO) return false;
-    // families up to kGramMaxCols columns are the Gram counter's (measured faster at every
-    // shape there); wider ones take the tensor tiles when large enough to fill their MMAs
-    if (jd.n_cols <= kGramMaxCols) return false;
-    if ((int64_t)jd.n_rows * jd.n_cols < p.tc_min_work) return false;
+    if (jd.n_rows < kPkMinRows || jd.words < kPkMinWords || (int64_t)jd.n_rows * jd.n_cols < p.tc_min_work) return false;
     const float d = n > 0 ? fminf(1.f, 128.f * (float)sup / (float)n) : 1.f;
     return d >= p.tc_min_density;
 }
+// Jobs per packed tile by columns: 8, 16, 24, 32, 40, 64 or 128 rows of the tile each.
+constexpr int kPkClasses = 7;
+__device__ __forceinline__ int pk_class(int cols) {
+    return cols <= 40 ? max(0, (cols - 1) >> 3) : cols <= 64 ? 5 : 6;
+}
+__device__ __forceinline__ int pk_per(int cls) { return cls <= 3 ? 16 / (cls + 1) : cls == 4 ? 3 : cls == 5 ? 2 : 1; }
 
 // The CUDA-core Gram counter takes a dense family job of at most kGramMaxCols columns (and at
-// most 128 blocks of 4 x 4 pairs): a dense prefix has no zero word for the general tiles to
+// most 128 blocks of 4 x 4 pairs) that the packed tiles leave: a dense prefix has no zero word for the general tiles to
 // skip, and at these widths the register-tiled Gram block (86-91% of the POPC ceiling at 32
 // and 64 columns) beats the tensor tiles, whose narrow MMAs cost about 50 cycles each.
 __device__ __forceinline__ bool use_gram(const ResPtrs& p, const JobDesc& jd, int32_t sup, int32_t n) {
     // tails of 1 or 2 rows are memory-bound in any kernel (8 bit-ops per byte and row); the
     // general tiles handle them as well, and measured faster on the dense benchmark
     if (jd.n_cols < 1 || jd.n_cols > kGramMaxCols || jd.n_rows < p.gram_min_rows) return false;
-    if (((jd.n_rows + 3) / 4) * ((jd.n_cols + 3) / 4) > 128) return false;
+    if (((jd.n_rows + 3) / 4) * ((jd.n_cols + 3) / 4) > 128 || jd.words >= kGramMaxWords) return false;
     if (p.counter != TFIM_COUNTER_AUTO) return false;
     const float d = n > 0 ? fminf(1.f, 128.f * (float)sup / (float)n) : 1.f;
     return d >= p.tc_min_density;
@@ -349,12 +369,12 @@ __device__ __forceinline__ int64_t slice_words(int64_t total, int64_t want) {
 
 __device__ __forceinline__ void res_pack(const ResPtrs& p) {
     __shared__ int64_t sm64[2 * 33];
-    __shared__ int32_t sm32[6 * 33];
+    __shared__ int32_t sm32[kPkClasses * 33];
     __shared__ int32_t s_pre[kPackSearch];
     __shared__ int32_t s_src[kPackSearch];
     __shared__ int32_t s_n_jobs, s_rows_total, s_done, s_max_cols, s_max_head, s_stack_after, s_kstop, s_fit;
     __shared__ int64_t s_out_total;
-    __shared__ float s_cost;
+    __shared__ float s_cost, s_pk_work, s_pk_cost;
     __shared__ unsigned long long s_words[3];   // words of the wave's b1 / tcgen05 / Gram tiles
     ResStatus* st = p.st;
     const int tid = threadIdx.x, lane = tid & 31;
@@ -373,7 +393,7 @@ __device__ __forceinline__ void res_pack(const ResPtrs& p) {
     if (tid == 32) {
         s_n_jobs = n_look; s_rows_total = n_look; s_out_total = 0; s_max_cols = 0; s_max_head = 0; s_done = 0;
         s_stack_after = st->stack_n;
-        s_cost = 0.f;
+        s_cost = s_pk_work = s_pk_cost = 0.f;
         s_words[0] = s_words[1] = s_words[2] = 0;
         st->n_proj = 0;
         st->n_mjobs = 0;
@@ -532,7 +552,7 @@ __device__ __forceinline__ void res_pack(const ResPtrs& p) {
             jd.col_off = f.F_off;
             // outputs: every candidate before this one contributed rv * nF, this one take * nF
             jd.out_off = out_base + o_at[q];
-            jd.self_col = -1; jd.words = f.W;
+            jd.self_col = -1; jd.words = f.W; jd.r0 = f.next_row;
             p.jobs[jid] = jd;
             if (jid < kPackSearch) {
                 s_pre[jid] = row;
@@ -582,7 +602,7 @@ __device__ __forceinline__ void res_pack(const ResPtrs& p) {
         return (float)(jd.words >> 2) * (1.f + d * (2.f + nr + nr * nc / 32.f));
     };
     {
-        float cost = 0.f;
+        float cost = 0.f, pk_work = 0.f, pk_cost = 0.f;   // of the packed jobs: pairs x words; as CUDA-core tiles
         unsigned long long w1 = 0, wt = 0, wg = 0;
         for (int j = tid; j < nj; j += kPackThreads) {
             const JobDesc jd = p.jobs[j];
@@ -598,7 +618,9 @@ __device__ __forceinline__ void res_pack(const ResPtrs& p) {
                 wg += (unsigned long long)jd.words;
             } else if (fam && use_tc(p, jd, dj.sup, n)) {
                 cls = kGrpTc;
-                wt += (unsigned long long)jd.words;
+                wt += (unsigned long long)(jd.words / pk_per(pk_class(jd.n_cols)) + 1);
+                pk_work += (float)jd.n_rows * (float)jd.n_cols * (float)jd.words;
+                pk_cost += (float)l3_tiles(jd.n_rows, jd.n_cols) * l3_cost(jd, dj, n);
             } else if (fam && use_b1_shape(p, jd.n_rows, jd.n_cols)) {
                 cls = kGrpB1;
                 w1 += (unsigned long long)(b1_tiles(jd.n_rows, jd.n_cols) * jd.words);
@@ -616,6 +638,8 @@ __device__ __forceinline__ void res_pack(const ResPtrs& p) {
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
                 cost += __shfl_xor_sync(0xffffffffu, cost, o);
+                pk_work += __shfl_xor_sync(0xffffffffu, pk_work, o);
+                pk_cost += __shfl_xor_sync(0xffffffffu, pk_cost, o);
                 w1 += __shfl_xor_sync(0xffffffffu, w1, o);
                 wt += __shfl_xor_sync(0xffffffffu, wt, o);
                 wg += __shfl_xor_sync(0xffffffffu, wg, o);
@@ -623,9 +647,22 @@ __device__ __forceinline__ void res_pack(const ResPtrs& p) {
             if (lane == 0) {
                 atomicAdd(&s_cost, cost);
                 if (w1) atomicAdd(&s_words[0], w1);
-                if (wt) atomicAdd(&s_words[1], wt);
+                if (wt) {
+                    atomicAdd(&s_words[1], wt);
+                    atomicAdd(&s_pk_work, pk_work);
+                    atomicAdd(&s_pk_cost, pk_cost);
+                }
                 if (wg) atomicAdd(&s_words[2], wg);
             }
+        }
+        __syncthreads();
+    }
+    // a wave whose packed jobs are little work in all counts them on the CUDA cores instead
+    const bool few_pk = p.counter == TFIM_COUNTER_AUTO && s_words[1] > 0 && s_pk_work < kPkMinWork;
+    if (few_pk) {
+        if (tid == 0) {
+            s_cost += s_pk_cost;
+            s_words[1] = 0;
         }
         __syncthreads();
     }
@@ -648,6 +685,7 @@ __device__ __forceinline__ void res_pack(const ResPtrs& p) {
             const int64_t W = jd.words;
             int64_t sl = 1, per = 1;   // word slices, tiles per slice
             int cls = dj.cls;
+            if (few_pk && cls == kGrpTc) cls = 16 * (int64_t)dj.sup >= dj.pad ? kGrpDense : kGrpLight;
             if (cls <= kGrpLight) {
                 const float cost = l3_cost(jd, dj, dj.pad);
                 sl = lmin(lmax(1, W / 256), lmax(1, (int64_t)ceilf(cost / (cls == kGrpDense ? target_d : target))));
@@ -656,11 +694,11 @@ __device__ __forceinline__ void res_pack(const ResPtrs& p) {
                 if (cls == kGrpLight && cost >= 0.5f * target) cls = kGrpHeavy;
                 per = l3_tiles(jd.n_rows, jd.n_cols);
             } else if (cls < kGrps) {
-                const int64_t sw = cls == kGrpB1 ? sw_b1 : cls == kGrpTc ? sw_tc : sw_gr;
+                const int64_t sw = cls == kGrpB1 ? sw_b1 : sw_gr;
                 sl = (W + sw - 1) / sw;
                 if (cls == kGrpB1) per = b1_tiles(jd.n_rows, jd.n_cols);
             }
-            if (cls < kGrps) {
+            if (cls < kGrps && cls != kGrpTc) {
                 const int64_t wsl = ((W / 64 + sl - 1) / sl) * 64;
                 sl = wsl > 0 ? (W + wsl - 1) / wsl : 1;
                 djp->sl3 = (int32_t)sl;
@@ -676,8 +714,75 @@ __device__ __forceinline__ void res_pack(const ResPtrs& p) {
 #pragma unroll
         for (int k = 0; k < kGrps; k++) tot[k] += t[k];
     }
-    const int64_t T3 = (int64_t)tot[kGrpDense] + tot[kGrpHeavy] + tot[kGrpLight], T1 = tot[kGrpB1], TT = tot[kGrpTc],
-                  TG = tot[kGrpGram];
+    // packed tiles: the jobs of a class fill them in order; the tiles of class k follow those of
+    // class k - 1
+    int32_t n_pk = 0;          // packed tiles before slicing
+    int32_t TT = 0;            // and in word slices
+    int32_t pk_first[kPkClasses] = {0, 0, 0, 0, 0, 0, 0}, pk_jobs[kPkClasses] = {0, 0, 0, 0, 0, 0, 0};
+    // counts the word slices of the packed tiles and, with `write`, writes them; a slice holds at
+    // most 2^18 words, so that FP32 sums stay exact
+    auto pk_tiles = [&](bool write) -> int32_t {
+        int32_t run = 0;
+        for (int base = 0; base < n_pk; base += kPackThreads) {
+            const int b = base + tid;
+            int32_t n = 0, per = 1, v[1] = {0}, ex[1], t[1];
+            int64_t W = 0, wsl = 64;
+            if (b < n_pk) {
+#pragma unroll
+                for (int k = 0; k < kPkClasses; k++)
+                    if (pk_jobs[k] > 0 && b >= pk_first[k]) {   // the last such class holds tile b
+                        per = pk_per(k);
+                        n = min(per, pk_jobs[k] - (b - pk_first[k]) * per);
+                    }
+                for (int i = 0; i < n; i++) W = lmax(W, (int64_t)p.jobs[p.pk_list[b * kPkJobs + i]].words);
+                const int64_t sw = lmin(sw_tc, 1 << 18), sl = lmax(1, (W + sw - 1) / sw);
+                wsl = lmax(1, (W / 64 + sl - 1) / sl) * 64;
+                v[0] = (int32_t)((W + wsl - 1) / wsl);
+            }
+            block_scan<1>(v, ex, t, sm32, base + (tid & ~31) < n_pk);
+            if (write)
+                for (int32_t q = 0; q < v[0]; q++)
+                    p.tiles_tc[run + ex[0] + q] = TileDesc{b * kPkJobs, 0, n, per, 0, (int32_t)(q * wsl),
+                                                           (int32_t)lmin(W, (q + 1) * wsl), 0};
+            run += t[0];
+        }
+        return run;
+    };
+    if (s_words[1] > 0) {
+        for (int base = 0; base < nj; base += kPackThreads) {
+            const int j = base + tid;
+            int32_t v[kPkClasses] = {0, 0, 0, 0, 0, 0, 0}, ex[kPkClasses], t[kPkClasses];
+            const bool in = j < nj && p.djobs[j].cls == kGrpTc;
+            const int pc = in ? pk_class(p.jobs[j].n_cols) : 0;
+            if (in)
+#pragma unroll
+                for (int k = 0; k < kPkClasses; k++) v[k] = k == pc;
+            block_scan<kPkClasses>(v, ex, t, sm32, base + (tid & ~31) < nj);
+#pragma unroll
+            for (int k = 0; k < kPkClasses; k++) {
+                if (in && k == pc) p.djobs[j].pre[kGrpTc] = pk_jobs[k] + ex[k];
+                pk_jobs[k] += t[k];
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < kPkClasses; k++) {
+            pk_first[k] = n_pk;
+            n_pk += (pk_jobs[k] + pk_per(k) - 1) / pk_per(k);
+        }
+        for (int j = tid; j < nj; j += kPackThreads) {
+            const DJob dj = p.djobs[j];
+            if (dj.cls != kGrpTc) continue;
+            const int pc = pk_class(p.jobs[j].n_cols), per = pk_per(pc);
+            int32_t first = 0;
+#pragma unroll
+            for (int k = 0; k < kPkClasses; k++)
+                if (k == pc) first = pk_first[k];
+            p.pk_list[(first + dj.pre[kGrpTc] / per) * kPkJobs + dj.pre[kGrpTc] % per] = j;
+        }
+        __syncthreads();   // the lists are read below
+        TT = pk_tiles(false);
+    }
+    const int64_t T3 = (int64_t)tot[kGrpDense] + tot[kGrpHeavy] + tot[kGrpLight], T1 = tot[kGrpB1], TG = tot[kGrpGram];
     // the wave is committed only when the worst case of its expand fits the pools
     if (tid == 0) {
         const bool fit = s_out_total <= p.cap_out && T1 <= p.cap_tiles && T3 <= p.cap_tiles && TT <= p.cap_tiles &&
@@ -764,7 +869,7 @@ __device__ __forceinline__ void res_pack(const ResPtrs& p) {
             const DJob dj = p.djobs[j];
             const int32_t local = t - dj.pre[grp];
             const int64_t W = jd.words, wsl = ((W / 64 + dj.sl3 - 1) / dj.sl3) * 64;
-            if (grp >= kGrpTc) {
+            if (grp == kGrpGram) {
                 // rows 0 .. n_rows of the job are its columns dj.r0 .. dj.r0 + n_rows
                 const int64_t w0 = local * wsl;
                 out[first + t] = TileDesc{j, 0, jd.n_rows, 0, jd.n_cols, (int32_t)w0, (int32_t)lmin(W, w0 + wsl), dj.r0};
@@ -785,7 +890,7 @@ __device__ __forceinline__ void res_pack(const ResPtrs& p) {
     emit(kGrpHeavy, p.tiles_l3, tot[kGrpDense]);
     emit(kGrpLight, p.tiles_l3, (int64_t)tot[kGrpDense] + tot[kGrpHeavy]);
     emit(kGrpB1, p.tiles_b1, 0);
-    emit(kGrpTc, p.tiles_tc, 0);
+    if (TT > 0) pk_tiles(true);
     emit(kGrpGram, p.tiles_gr, 0);
     if (tid == 0) {
         st->jobs = nj;
@@ -793,7 +898,7 @@ __device__ __forceinline__ void res_pack(const ResPtrs& p) {
         st->tiles_l3 = (int32_t)T3;
         st->tiles_l3d = tot[kGrpDense];
         st->tiles_b1 = (int32_t)T1;
-        st->tiles_tc = (int32_t)TT;
+        st->tiles_tc = TT;
         st->tiles_gr = (int32_t)TG;
         st->out_total = s_out_total;
         st->max_cols = s_max_cols;
@@ -1302,18 +1407,21 @@ __global__ void __launch_bounds__(256) k_res_expand(ResPtrs p) {
 __device__ __forceinline__ void build_masks(const ResPtrs& p) {
     const int32_t n = p.st->n_mjobs;
     if (n <= 0) return;
-    const int64_t most = (p.W / 4 + 255) / 256;   // a part holds at least a block's width
-    const int64_t parts = lmax(1, lmin(most, (2 * (int64_t)gridDim.x + n - 1) / n));
+    // a part holds at least a block's width (rows of a bitmap are below 2^31 transactions)
+    const int32_t most = (int32_t)((p.W / 4 + 255) / 256);
+    const int32_t parts = max(1, min(most, (int32_t)((2 * gridDim.x + n - 1) / n)));
     const uint4 ones = make_uint4(~0u, ~0u, ~0u, ~0u);
-    for (int64_t u = blockIdx.x; u < n * parts; u += gridDim.x) {
-        const MaskJob mj = p.mjobs[u / parts];
-        const int64_t W4 = mj.W >> 2, per = (W4 + parts - 1) / parts;
-        const int64_t c0 = (u % parts) * per, c1 = lmin(W4, c0 + per);
+    const int64_t units = (int64_t)n * parts;
+    for (int64_t u = blockIdx.x; u < units; u += gridDim.x) {
+        const int32_t job = parts == 1 ? (int32_t)u : (int32_t)(u / parts), part = (int32_t)(u - (int64_t)job * parts);
+        const MaskJob mj = p.mjobs[job];
+        const int32_t W4 = mj.W >> 2, per = (W4 + parts - 1) / parts;
+        const int32_t c0 = part * per, c1 = min(W4, c0 + per);
         uint4* d = reinterpret_cast<uint4*>(p.masks + (int64_t)mj.dst * p.W);
         const uint4* sm = mj.slot >= 0 ? reinterpret_cast<const uint4*>(p.masks + (int64_t)mj.slot * p.W) : nullptr;
         const uint4* si = mj.item >= 0 ? reinterpret_cast<const uint4*>(row_of(p, mj.item)) : nullptr;
         const uint4* st = mj.t >= 0 ? reinterpret_cast<const uint4*>(row_of(p, mj.t)) : nullptr;
-        for (int64_t w = c0 + threadIdx.x; w < c1; w += blockDim.x) {
+        for (int32_t w = c0 + (int32_t)threadIdx.x; w < c1; w += blockDim.x) {
             uint4 v = ones;
             auto andv = [&](uint4 x) { v.x &= x.x; v.y &= x.y; v.z &= x.z; v.w &= x.w; };
             if (sm) andv(sm[w]);
@@ -1683,7 +1791,6 @@ __global__ void __launch_bounds__(256) k_res_zero(const ResArgs* __restrict__ ar
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         st->next3 = 0;
         st->next1 = 0;
-        st->next_tc = 0;
         st->next_gr = 0;
     }
     const int64_t n = st->out_total;
@@ -1835,7 +1942,7 @@ int build_wave_graph(WaveGraph& G, const ResArgs* d_args, ResStatus* d_status, b
     TFIM_CUDA(cudaGetDevice(&dev));
     TFIM_CUDA(cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, dev));
     TFIM_TRY(persistent_occupancy(&occ3, &occ1, &occp));
-    TFIM_TRY(configure_fam_kernel());
+    TFIM_TRY(configure_pk_kernel());
     TFIM_TRY(occupancy_gram(&occg));
     TFIM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occe, k_res_expand_g, 256, 0));
     TFIM_CUDA(cudaGraphCreate(&G.graph, 0));
@@ -1860,7 +1967,7 @@ int build_wave_graph(WaveGraph& G, const ResArgs* d_args, ResStatus* d_status, b
         if (with_proj &&
             (rc = launch_count_proj_persistent(&d_args->ap, &d_status->n_proj, sm * std::max(1, occp), red_off, red_items, s)))
             break;
-        if ((rc = launch_count_fam_persistent(&d_args->atc, &d_status->tiles_tc, &d_status->next_tc, sm, s))) break;
+        if ((rc = launch_count_pk_persistent(&d_args->atc, &d_status->tiles_tc, sm, s))) break;
         if ((rc = launch_count_gram_persistent(&d_args->agr, &d_status->tiles_gr, &d_status->next_gr, sm * std::max(1, occg),
                                                s)))
             break;
@@ -1888,6 +1995,7 @@ struct ResidentState {
     Pool fams, items, heads, stack, looks, free_slots, defer, mfi_off, mfi_len, mfi_sup, mfi_items, log_feat, log_label;
     Pool djobs, jobs, rows, row_job, row_local, tiles_l3, tiles_b1, tiles_tc, tiles_gr, counts, status, is_root, dense_freq, top_pos,
         top_diag, proj_list, args, top_sum, mjobs, sup_index;
+    Pool pk_list;
     Pool pjobs, pj_off, pj_pool, vrows, vitem;              // projected families
     Pool ord_keys, ord_idx, ord_meta, ord_items, ord_tmp;   // output order of the MFIs
     HostBuf h_status, h_args, h_res, h_setup;
@@ -1905,7 +2013,7 @@ struct ResidentState {
         for (Pool* b : {&fams, &items, &heads, &stack, &looks, &free_slots, &defer, &mfi_off, &mfi_len, &mfi_sup, &mfi_items,
                         &log_feat, &log_label, &djobs, &jobs, &rows, &row_job, &row_local, &tiles_l3, &tiles_b1, &tiles_tc, &tiles_gr, &counts,
                         &status, &is_root, &dense_freq, &top_pos, &top_diag, &proj_list, &args, &top_sum, &mjobs,
-                        &sup_index, &pjobs, &pj_off, &pj_pool, &vrows, &vitem, &ord_keys, &ord_idx, &ord_meta, &ord_items, &ord_tmp}) {
+                        &sup_index, &pk_list, &pjobs, &pj_off, &pj_pool, &vrows, &vitem, &ord_keys, &ord_idx, &ord_meta, &ord_items, &ord_tmp}) {
             dev_free(b->p, s);
             b->p = nullptr;
             b->bytes = 0;
@@ -2143,6 +2251,7 @@ int mine_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt) {
     TFIM_TRY(grow(R.row_job, cap_rows * 4, s));
     TFIM_TRY(grow(R.row_local, cap_rows * 4, s));
     TFIM_TRY(grow(R.proj_list, cap_rows * 4, s));
+    TFIM_TRY(grow(R.pk_list, cap_rows * kPkJobs * 4, s));   // at most one tile per job
     TFIM_TRY(grow(R.mjobs, (2 * cap_rows + 2) * sizeof(MaskJob), s));   // at most two masks per expanded row
     TFIM_TRY(grow(R.tiles_l3, cap_tiles * sizeof(TileDesc), s));
     TFIM_TRY(grow(R.tiles_b1, cap_tiles * sizeof(TileDesc), s));
@@ -2280,6 +2389,7 @@ int mine_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt) {
         P.row_job = (int32_t*)R.row_job.p; P.row_local = (int32_t*)R.row_local.p;
         P.tiles_l3 = (TileDesc*)R.tiles_l3.p; P.tiles_b1 = (TileDesc*)R.tiles_b1.p; P.tiles_tc = (TileDesc*)R.tiles_tc.p;
         P.tiles_gr = (TileDesc*)R.tiles_gr.p;
+        P.pk_list = (int32_t*)R.pk_list.p;
         P.counts = (int32_t*)R.counts.p;
         P.bitmap = c->d_bitmap; P.masks = c->d_masks.as<uint32_t>(); P.dense_freq = (const int32_t*)R.dense_freq.p;
         P.is_root = (const uint8_t*)R.is_root.p; P.st = (ResStatus*)R.status.p;
@@ -2420,9 +2530,14 @@ int mine_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt) {
         if (n_pj == 0) return TFIM_OK;
         // the compressed rows may take an eighth of the device's memory; without room for them
         // the families stay where they are
-        size_t mem_free = 0, mem_total = 0;
-        TFIM_CUDA(cudaMemGetInfo(&mem_free, &mem_total));
-        if ((size_t)words * 4 > mem_total / 8) return TFIM_OK;
+        static std::atomic<size_t> total_of[64];   // device memory, asked for once (the call is slow)
+        std::atomic<size_t>& total = total_of[c->device & 63];
+        if (!total.load()) {
+            size_t mem_free = 0, mem_total = 0;
+            TFIM_CUDA(cudaMemGetInfo(&mem_free, &mem_total));
+            total.store(mem_total);
+        }
+        if ((size_t)words * 4 > total.load() / 8) return TFIM_OK;
         if ((size_t)words * 4 > R.pj_pool.bytes) {   // its old contents are not needed
             dev_free(R.pj_pool.p, s);
             R.pj_pool = Pool{};
@@ -2540,7 +2655,7 @@ int mine_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt) {
             ha->p.launch_id = ++R.launch_id;
             ha->p.wave_limit = 0x7fffffff;
             CountArgs a;
-            a.vrows = P.vrows; a.n_base = P.n_base;
+            a.vrows = P.vrows; a.n_base = P.n_base; a.pk_list = P.pk_list;
             a.bitmap = c->d_bitmap; a.W = W; a.masks = P.masks; a.jobs = P.jobs; a.rows = P.rows;
             a.cols = P.items; a.out = P.counts; a.n_tiles = 0; a.job_list = P.proj_list;
             a.tiles = P.tiles_l3;
@@ -2600,7 +2715,7 @@ int mine_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt) {
         if (hst->jobs == 0) break;
         TFIM_CUDA(cudaMemsetAsync(R.counts.p, 0, (size_t)hst->out_total * 4, s));
         CountArgs a;
-        a.vrows = P.vrows; a.n_base = P.n_base;
+        a.vrows = P.vrows; a.n_base = P.n_base; a.pk_list = P.pk_list;
         a.bitmap = c->d_bitmap; a.W = W; a.masks = c->d_masks.as<uint32_t>(); a.jobs = P.jobs; a.rows = P.rows;
         a.cols = P.items; a.out = P.counts; a.job_list = P.proj_list;
         if (hst->tiles_l3) {
@@ -2635,7 +2750,7 @@ int mine_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt) {
             a.tiles = P.tiles_tc;
             a.n_tiles = hst->tiles_tc;
             a.ph_s = &d_st->ph_s[kPhTc]; a.ph_e = &d_st->ph_e[kPhTc];
-            TFIM_TRY(launch_count_fam(a, s));
+            TFIM_TRY(launch_count_pk(a, sm_count, s));
             launches++;
             count_launches++;
             path_launches[TFIM_PATH_TC]++;
@@ -2700,10 +2815,10 @@ int mine_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt) {
     int32_t* flags = c->h_flags.as<int32_t>();
     flags[0] = flags[1] = 0;
     if (used_f4) TFIM_TRY(count_f4_status_fetch(flags, s));
-    if (used_tc) TFIM_TRY(count_fam_status_fetch(flags + 1, s));
+    if (used_tc) TFIM_TRY(count_pk_status_fetch(flags + 1, s));
     TFIM_CUDA(cudaStreamSynchronize(s));
     TFIM_TRY(count_f4_status_check(flags[0]));
-    TFIM_TRY(count_fam_status_check(flags[1]));
+    TFIM_TRY(count_pk_status_check(flags[1]));
     {
         MfiSet& M = c->mfis;
         const bool fresh = M.size() == 0;

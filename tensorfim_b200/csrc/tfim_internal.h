@@ -91,6 +91,7 @@ struct JobDesc {
     int64_t out_off;      // into the counts buffer
     int32_t self_col;     // column index that stands for all ones (not read from the table), or -1
     int32_t words;        // words per row of the job's transactions (resident pack)
+    int32_t r0, pad;      // family jobs: the column that is the job's first row
 };
 struct RowDesc {
     int32_t slot;
@@ -140,6 +141,7 @@ struct CountArgs {
     // Rows of projected families (resident engine): ids from n_base on are vrows[id - n_base]
     const uint32_t* const* vrows = nullptr;
     int32_t n_base = 0x7fffffff;
+    const int32_t* pk_list = nullptr;   // packed family counter: the jobs of each tile
     // phase stamps of the launch (or nullptr): the earliest block start and the latest block
     // end, in %globaltimer nanoseconds (phase_begin / phase_end)
     unsigned long long* ph_s = nullptr;
@@ -191,17 +193,17 @@ int launch_count_f4(const CountArgs& a, cudaStream_t s);
 int count_f4_status_fetch(int32_t* pinned, cudaStream_t s);
 int count_f4_status_check(int32_t v);
 void tiles_f4(int32_t job, int32_t nr, int32_t nc, int64_t W, int sms, std::vector<TileDesc>& out, bool upper = false);
-// tcgen05 kind::i8 family counter (count_fam.cu): a tile is one family job (rows a run of its
-// columns, at most kFamMaxCols columns) over a word slice, TileDesc.pad = the F position of
-// the tile's first row; one CTA per SM.  The persistent form reads its arguments and tile
-// count from device memory and takes tiles from `d_next` (zero at launch).
-constexpr int kFamMaxCols = 128;
-int launch_count_fam(const CountArgs& a, cudaStream_t s);
-int launch_count_fam_persistent(const CountArgs* d_args, const int32_t* d_n_tiles, int32_t* d_next, int32_t grid,
-                                cudaStream_t s);
-int count_fam_status_fetch(int32_t* pinned, cudaStream_t s);
-int count_fam_status_check(int32_t v);
-int configure_fam_kernel();   // opt into its shared memory (once per device, before any capture)
+// Packed tcgen05 kind::mxf4 family counter (count_pk.cu): a tile holds the X rows of `nr` jobs of at
+// most kPkMaxCols columns, CountArgs::pk_list[job .. job + nr), of a class of c0 jobs per tile, over
+// a word slice of at most 2^18 words (its jobs may have fewer).  The persistent form reads its
+// arguments and tile count from device memory.
+constexpr int kPkMaxCols = 128;
+constexpr int kPkJobs = 16;         // list entries per tile
+int launch_count_pk(const CountArgs& a, int32_t sms, cudaStream_t s);
+int launch_count_pk_persistent(const CountArgs* d_args, const int32_t* d_n_tiles, int32_t grid, cudaStream_t s);
+int count_pk_status_fetch(int32_t* pinned, cudaStream_t s);
+int count_pk_status_check(int32_t v);
+int configure_pk_kernel();   // opt into its shared memory (once per device, before any capture)
 // CUDA-core Gram counter for dense family jobs (count_gram.cu): a tile is one family job of at
 // most kGramMaxCols columns and at most 128 blocks of 4 x 4 (row, column) pairs, over a word
 // slice; TileDesc.pad = the F position of the job's first row.

@@ -22,7 +22,7 @@ import time
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 PATHS = ["lop3", "b1", "tc", "pairs", "proj", "gram"]
-KERNELS = {"lop3": "k_count_lop3", "b1": "k_count_b1", "tc": "k_count_fam", "pairs": "k_pair_count",
+KERNELS = {"lop3": "k_count_lop3", "b1": "k_count_b1", "tc": "k_count_pk", "pairs": "k_pair_count",
            "proj": "k_count_proj", "gram": "k_count_gram"}
 PEAKS_FALLBACK = {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0, "bf16_tflops_sustained": 1400.0}
 
