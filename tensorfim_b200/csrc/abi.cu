@@ -37,7 +37,7 @@ int make_ctx(int32_t device, tfim_ctx** out) {
     c->device = device;
     static std::atomic<uint64_t> next_uid{1};
     c->uid = next_uid.fetch_add(1);
-    if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
+    if (stream_get(&c->stream) != cudaSuccess ||
         cudaEventCreate(&c->ev0) != cudaSuccess || cudaEventCreate(&c->ev1) != cudaSuccess ||
         cudaEventCreate(&c->ev_span0) != cudaSuccess || cudaEventCreate(&c->ev_span1) != cudaSuccess) {
         set_error("stream/event creation failed: %s", cudaGetErrorString(cudaGetLastError()));
@@ -84,14 +84,15 @@ int make_sharded_ctx(int32_t device, const tfim_group* g, bool args_ok, const st
 
 }  // namespace
 
-// Per-node masks + one count job over every counted row (the reference counting contract).
-int count_wave_impl(tfim_ctx* c, int32_t b, int32_t min_count, const int32_t* d_items, const MatDesc* d_mats,
-                    int32_t* d_counts, int32_t* d_nfreq, cudaStream_t s) {
+// Per-node masks + one count job over every counted row (the reference counting contract).  The
+// tables of the count job and, for lists on the host, the lists go up in one copy; one kernel
+// builds the masks and clears the counts, one counts the frequent columns and hands small
+// results and the counter's error flag to pinned host memory.
+int count_wave_impl(tfim_ctx* c, int32_t b, int32_t min_count, const WaveLists& L, int32_t* d_counts, int32_t* d_nfreq,
+                    cudaStream_t s, int32_t* out) {
     const int32_t d = c->n_counted;
     // masks: one pool row per node
     TFIM_TRY(c->d_masks.reserve((size_t)b * (size_t)c->W * 4));
-    TFIM_TRY(launch_materialize(c->d_bitmap, c->W, c->d_masks.as<uint32_t>(), d_mats, d_items, b, s));
-    if (d == 0) return launch_nfreq(d_counts, b, 0, min_count, d_nfreq, s);
     // host-built job/tile tables (independent of the list contents)
     const int32_t counter = c->counter_pref;
     const tfim_tuning tn = tuning();
@@ -104,7 +105,7 @@ int count_wave_impl(tfim_ctx* c, int32_t b, int32_t min_count, const int32_t* d_
                      (b >= tn.i8_min_rows || c->W <= (1 << 14)));
     const bool b1 = !i8 && (counter == TFIM_COUNTER_TENSOR ||
                             (counter == TFIM_COUNTER_AUTO && b >= tn.b1_min_rows && d >= tn.b1_min_cols));
-    std::vector<JobDesc> jobs(1);
+    std::vector<JobDesc> jobs(1, JobDesc{});
     jobs[0].base_slot = -1; jobs[0].base_item = -1;
     jobs[0].n_rows = b; jobs[0].n_cols = d; jobs[0].row_off = 0; jobs[0].col_off = 0; jobs[0].out_off = 0;
     jobs[0].self_col = -1; jobs[0].words = 0;
@@ -114,7 +115,8 @@ int count_wave_impl(tfim_ctx* c, int32_t b, int32_t min_count, const int32_t* d_
     std::iota(cols.begin(), cols.end(), 0);
     std::vector<TileDesc> tiles;
     const int64_t W = c->W;
-    if (i8) {
+    if (d == 0) {
+    } else if (i8) {
         tiles_f4(0, b, d, W, 148, tiles);
     } else if (b1) {
         const int64_t base = (int64_t)((b + kB1Rows - 1) / kB1Rows) * ((d + kB1Cols - 1) / kB1Cols);
@@ -135,16 +137,23 @@ int count_wave_impl(tfim_ctx* c, int32_t b, int32_t min_count, const int32_t* d_
                     tiles.push_back(TileDesc{0, r0, std::min(kLop3Rows, b - r0), c0, std::min(d, c0 + 64), (int32_t)w0,
                                              (int32_t)std::min<int64_t>(W, w0 + chunk), 0});
     }
+    const size_t n_items = L.h_off ? (size_t)L.h_off[b] : 0;
     const size_t o_rows = 64, o_cols = o_rows + ((rows.size() * sizeof(RowDesc) + 15) & ~size_t(15));
     const size_t o_tiles = o_cols + ((cols.size() * 4 + 15) & ~size_t(15));
-    const size_t total = o_tiles + tiles.size() * sizeof(TileDesc);
+    const size_t o_off = o_tiles + tiles.size() * sizeof(TileDesc);
+    const size_t o_items = o_off + (L.h_off ? (size_t)(b + 1) * 8 : 0), total = o_items + n_items * 4;
     TFIM_TRY(c->h_scratch[0].reserve(total));
     TFIM_TRY(c->d_scratch[0].reserve(total));
+    TFIM_TRY(c->h_flags.reserve(64));
     unsigned char* hp = c->h_scratch[0].as<unsigned char>();
     memcpy(hp, jobs.data(), sizeof(JobDesc));
     memcpy(hp + o_rows, rows.data(), rows.size() * sizeof(RowDesc));
     memcpy(hp + o_cols, cols.data(), cols.size() * 4);
     memcpy(hp + o_tiles, tiles.data(), tiles.size() * sizeof(TileDesc));
+    if (L.h_off) {
+        memcpy(hp + o_off, L.h_off, (size_t)(b + 1) * 8);
+        if (n_items) memcpy(hp + o_items, L.h_items, n_items * 4);
+    }
     unsigned char* dp = c->d_scratch[0].as<unsigned char>();
     if (s != c->stream) {
         // buffers are allocated in the context stream's order: the caller's stream waits
@@ -152,30 +161,28 @@ int count_wave_impl(tfim_ctx* c, int32_t b, int32_t min_count, const int32_t* d_
         TFIM_CUDA(cudaStreamWaitEvent(s, c->ev0, 0));
     }
     TFIM_CUDA(cudaMemcpyAsync(dp, hp, total, cudaMemcpyHostToDevice, s));
-    TFIM_CUDA(cudaMemsetAsync(d_counts, 0, (size_t)b * d * 4, s));
+    TFIM_TRY(launch_wave_begin(c->d_bitmap, W, c->d_masks.as<uint32_t>(), L.d_mats,
+                               L.h_off ? (const int64_t*)(dp + o_off) : L.d_off,
+                               L.h_off ? (const int32_t*)(dp + o_items) : L.d_items, b, d_counts, (int64_t)b * d, s));
     CountArgs a;
     a.bitmap = c->d_bitmap; a.W = W; a.masks = c->d_masks.as<uint32_t>();
     a.jobs = (const JobDesc*)dp; a.rows = (const RowDesc*)(dp + o_rows); a.cols = (const int32_t*)(dp + o_cols);
     a.tiles = (const TileDesc*)(dp + o_tiles); a.n_tiles = (int32_t)tiles.size(); a.out = d_counts;
-    if (i8) TFIM_TRY(c->h_flags.reserve(64));
-    TFIM_TRY(i8 ? launch_count_f4(a, s) : b1 ? launch_count_b1(a, s) : launch_count_lop3(a, s));
-    TFIM_TRY(group_reduce(c, d_counts, (int64_t)b * d, TFIM_DT_I32, TFIM_RED_SUM, s));
-    TFIM_TRY(launch_nfreq(d_counts, b, d, min_count, d_nfreq, s));
-    if (i8) TFIM_TRY(count_f4_status_fetch(c->h_flags.as<int32_t>(), s));
-    // the host staging buffer may be reused by the next call only after this copy ran
+    const int32_t* flag = nullptr;
+    volatile int32_t* flag_to = c->h_flags.as<int32_t>();
+    *flag_to = 0;
+    if (d > 0) {
+        if (i8) TFIM_TRY(count_f4_flag(&flag));
+        TFIM_TRY(i8 ? launch_count_f4(a, s) : b1 ? launch_count_b1(a, s) : launch_count_lop3(a, s));
+        TFIM_TRY(group_reduce(c, d_counts, (int64_t)b * d, TFIM_DT_I32, TFIM_RED_SUM, s));
+    }
+    TFIM_TRY(launch_nfreq(d_counts, b, d, min_count, d_nfreq, s, out, flag, flag ? (int32_t*)flag_to : nullptr));
+    // the host staging buffer may be reused by the next call only after its copy ran
     TFIM_CUDA(cudaStreamSynchronize(s));
-    return i8 ? count_f4_status_check(*c->h_flags.as<int32_t>()) : TFIM_OK;
+    return count_f4_status_check(*flag_to);
 }
 
 namespace {
-
-__global__ void k_mats_from_offsets(const int64_t* __restrict__ off, int32_t b, MatDesc* __restrict__ mats) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= b) return;
-    MatDesc m;
-    m.dst = i; m.src = -1; m.off = (int32_t)off[i]; m.n = (int32_t)(off[i + 1] - off[i]);
-    mats[i] = m;
-}
 
 std::string cpu_name() {
     std::ifstream f("/proc/cpuinfo");
@@ -280,7 +287,7 @@ int tfim_parse_text(const char* bytes, int64_t n_bytes, int32_t device, int64_t*
     TFIM_CHECK(device >= 0 && device < n_dev, TFIM_E_INVALID, "device %d out of range (%d devices)", device, n_dev);
     TFIM_CUDA(cudaSetDevice(device));
     cudaStream_t s = nullptr;
-    TFIM_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+    TFIM_CUDA(stream_get(&s));
     TextSource src;
     src.host = bytes ? bytes : "";
     src.n_bytes = n_bytes;
@@ -307,7 +314,7 @@ int tfim_parse_text(const char* bytes, int64_t n_bytes, int32_t device, int64_t*
     dev_free(d_off, s);
     dev_free(d_items, s);
     cudaStreamSynchronize(s);
-    cudaStreamDestroy(s);
+    stream_put(s);
     return rc;
 }
 
@@ -392,27 +399,33 @@ int tfim_count_wave(tfim_ctx* c, const int32_t* item_lists, const int64_t* list_
         for (int64_t q = list_offsets[i]; q < list_offsets[i + 1]; q++)
             TFIM_CHECK(item_lists[q] >= 0 && item_lists[q] < n_rows_total, TFIM_E_INVALID, "item %d out of range", item_lists[q]);
     }
-    const int64_t n_items = list_offsets[b];
     const int32_t d = c->n_counted;
     cudaStream_t s = c->stream;
-    // device staging: items, mats, counts, nfreq
-    const size_t o_items = 0;
-    const size_t o_mats = (((size_t)std::max<int64_t>(n_items, 1) * 4) + 15) & ~size_t(15);
-    const size_t o_counts = o_mats + (((size_t)b * sizeof(MatDesc) + 15) & ~size_t(15));
-    const size_t o_nfreq = o_counts + (((size_t)b * d * 4 + 15) & ~size_t(15));
-    const size_t total = o_nfreq + (size_t)b * 4;
-    TFIM_TRY(c->d_scratch[1].reserve(total));
-    TFIM_TRY(c->h_scratch[1].reserve(o_counts));
-    unsigned char* hp = c->h_scratch[1].as<unsigned char>();
-    if (n_items) memcpy(hp + o_items, item_lists, (size_t)n_items * 4);
-    MatDesc* hm = (MatDesc*)(hp + o_mats);
-    for (int32_t i = 0; i < b; i++) hm[i] = MatDesc{i, -1, (int32_t)list_offsets[i], (int32_t)(list_offsets[i + 1] - list_offsets[i])};
+    const size_t n_out = (size_t)b * d;
+    // device results: counts, nfreq
+    const size_t o_nfreq = (n_out * 4 + 15) & ~size_t(15);
+    TFIM_TRY(c->d_scratch[1].reserve(o_nfreq + (size_t)b * 4));
     unsigned char* dp = c->d_scratch[1].as<unsigned char>();
-    TFIM_CUDA(cudaMemcpyAsync(dp, hp, o_counts, cudaMemcpyHostToDevice, s));
-    TFIM_TRY(count_wave_impl(c, b, min_count, (const int32_t*)(dp + o_items), (const MatDesc*)(dp + o_mats),
-                             (int32_t*)(dp + o_counts), (int32_t*)(dp + o_nfreq), s));
-    TFIM_CUDA(cudaMemcpyAsync(counts_out, dp + o_counts, (size_t)b * d * 4, cudaMemcpyDeviceToHost, s));
-    TFIM_CUDA(cudaMemcpyAsync(nfreq_out, dp + o_nfreq, (size_t)b * 4, cudaMemcpyDeviceToHost, s));
+    int32_t* d_counts = (int32_t*)dp;
+    int32_t* d_nfreq = (int32_t*)(dp + o_nfreq);
+    WaveLists L;
+    L.h_items = item_lists;
+    L.h_off = list_offsets;
+    // up to 256 KiB of results come back through pinned memory that the last kernel writes itself (a
+    // copy into the caller's pageable arrays takes two more transfers and a second wait)
+    int32_t* out = nullptr;
+    if ((n_out + (size_t)b) * 4 <= (256u << 10)) {
+        TFIM_TRY(c->h_scratch[1].reserve((n_out + (size_t)b) * 4));
+        out = c->h_scratch[1].as<int32_t>();
+    }
+    TFIM_TRY(count_wave_impl(c, b, min_count, L, d_counts, d_nfreq, s, out));
+    if (out) {
+        memcpy(nfreq_out, out, (size_t)b * 4);
+        if (n_out) memcpy(counts_out, out + b, n_out * 4);
+        return TFIM_OK;
+    }
+    TFIM_CUDA(cudaMemcpyAsync(counts_out, d_counts, n_out * 4, cudaMemcpyDeviceToHost, s));
+    TFIM_CUDA(cudaMemcpyAsync(nfreq_out, d_nfreq, (size_t)b * 4, cudaMemcpyDeviceToHost, s));
     TFIM_CUDA(cudaStreamSynchronize(s));
     return TFIM_OK;
 }
@@ -425,15 +438,10 @@ int tfim_count_wave_device(tfim_ctx* c, const int32_t* d_item_lists, const int64
     if (b == 0) return TFIM_OK;
     TFIM_CUDA(cudaSetDevice(c->device));
     cudaStream_t s = stream ? (cudaStream_t)stream : c->stream;
-    TFIM_TRY(c->d_scratch[2].reserve((size_t)b * sizeof(MatDesc)));
-    TFIM_TRY(c->d_masks.reserve((size_t)b * (size_t)c->W * 4));
-    if (s != c->stream) {
-        TFIM_CUDA(cudaEventRecord(c->ev0, c->stream));
-        TFIM_CUDA(cudaStreamWaitEvent(s, c->ev0, 0));
-    }
-    k_mats_from_offsets<<<(b + 255) / 256, 256, 0, s>>>(d_list_offsets, b, c->d_scratch[2].as<MatDesc>());
-    TFIM_CUDA(cudaGetLastError());
-    return count_wave_impl(c, b, min_count, d_item_lists, c->d_scratch[2].as<MatDesc>(), d_counts_out, d_nfreq_out, s);
+    WaveLists L;
+    L.d_items = d_item_lists;
+    L.d_off = d_list_offsets;
+    return count_wave_impl(c, b, min_count, L, d_counts_out, d_nfreq_out, s);
 }
 
 int tfim_mine(tfim_ctx* c, const tfim_mine_opts* opts, tfim_mine_stats* stats) {
@@ -633,7 +641,7 @@ void tfim_close(tfim_ctx* c) {
     if (c->ev1) cudaEventDestroy(c->ev1);
     if (c->ev_span0) cudaEventDestroy(c->ev_span0);
     if (c->ev_span1) cudaEventDestroy(c->ev_span1);
-    if (c->stream) cudaStreamDestroy(c->stream);
+    stream_put(c->stream);
     delete c;
 }
 

@@ -116,7 +116,10 @@ int tfim_mine_all(tfim_ctx* c, int32_t min_count, int32_t max_len, int64_t max_i
             int32_t* dn = d_aux.as<int32_t>();   // nfreq of the count call, then the extension counts
             int64_t* doff = (int64_t*)(d_aux.as<unsigned char>() + (((size_t)b * 4 + 15) & ~size_t(15)));
             cudaEventRecord(e0, s);
-            if ((rc = count_wave_impl(c, b, min_count, di, dm, dc, dn, s))) break;
+            WaveLists L;
+            L.d_items = di;
+            L.d_mats = dm;
+            if ((rc = count_wave_impl(c, b, min_count, L, dc, dn, s))) break;
             cudaEventRecord(e1, s);
             const unsigned grid = (unsigned)(((int64_t)b * 32 + 255) / 256);
             k_ext_count<<<grid, 256, 0, s>>>(dc, b, d, min_count, dm, di, dn);

@@ -77,6 +77,49 @@ void dev_free(void* p, cudaStream_t s) {
     else cudaFree(p);
 }
 
+namespace {
+std::mutex g_stream_mu;
+std::vector<cudaStream_t> g_streams[64];
+constexpr size_t kIdleStreams = 16;   // kept per device: a context's and its eight upload workers', twice
+}  // namespace
+
+cudaError_t stream_get(cudaStream_t* s) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev >= 0 && dev < 64) {
+        std::lock_guard<std::mutex> lk(g_stream_mu);
+        if (!g_streams[dev].empty()) {
+            *s = g_streams[dev].back();
+            g_streams[dev].pop_back();
+            return cudaSuccess;
+        }
+    }
+    return cudaStreamCreateWithFlags(s, cudaStreamNonBlocking);
+}
+
+void stream_put(cudaStream_t s) {
+    if (!s) return;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (cudaStreamQuery(s) == cudaSuccess && dev >= 0 && dev < 64) {
+        std::lock_guard<std::mutex> lk(g_stream_mu);
+        if (g_streams[dev].size() < kIdleStreams) {
+            g_streams[dev].push_back(s);
+            return;
+        }
+    }
+    cudaStreamDestroy(s);   // too many, or not idle (an error)
+}
+
+void stream_release(int dev) {
+    std::vector<cudaStream_t> idle;
+    {
+        std::lock_guard<std::mutex> lk(g_stream_mu);
+        idle.swap(g_streams[dev]);
+    }
+    for (cudaStream_t s : idle) cudaStreamDestroy(s);
+}
+
 void* pinned_alloc(size_t bytes, size_t* got) {
     size_t cls = 4096;
     while (cls < bytes) cls <<= 1;

@@ -322,6 +322,21 @@ int count_f4_status_fetch(int32_t* pinned, cudaStream_t s) {
     return TFIM_OK;
 }
 
+int count_f4_flag(const int32_t** flag) {
+    static std::atomic<const int32_t*> at[64];
+    int dev = 0;
+    TFIM_CUDA(cudaGetDevice(&dev));
+    const int32_t* p = at[dev & 63].load();
+    if (!p) {
+        void* q = nullptr;
+        TFIM_CUDA(cudaGetSymbolAddress(&q, g_f4_status));
+        p = (const int32_t*)q;
+        at[dev & 63].store(p);
+    }
+    *flag = p;
+    return TFIM_OK;
+}
+
 int count_f4_status_check(int32_t v) {
     if (v) {
         const int z = 0;

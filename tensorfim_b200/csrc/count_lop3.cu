@@ -346,18 +346,45 @@ __global__ void k_materialize(const uint32_t* __restrict__ B, int64_t W, uint32_
     }
 }
 
-// one warp per row
+// The begin of a counting wave: prefix masks as in k_materialize (lists by descriptor or by
+// offset), and the count block's zeros.  grid = (word blocks, nodes)
+__global__ void k_wave_begin(const uint32_t* __restrict__ B, int64_t W, uint32_t* __restrict__ masks,
+                             const MatDesc* __restrict__ mats, const int64_t* __restrict__ off,
+                             const int32_t* __restrict__ items, int32_t* __restrict__ counts, int64_t n_zero) {
+    const int64_t t0 = (blockIdx.y * (int64_t)gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x;
+    for (int64_t i = t0; i < n_zero; i += (int64_t)gridDim.x * gridDim.y * blockDim.x) counts[i] = 0;
+    const int32_t node = blockIdx.y;
+    const int64_t first = mats ? mats[node].off : off[node];
+    const int32_t n = mats ? mats[node].n : (int32_t)(off[node + 1] - first);
+    const int64_t W4 = W >> 2;
+    uint4* dst = reinterpret_cast<uint4*>(masks + (int64_t)node * W);
+    for (int64_t w = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; w < W4; w += (int64_t)gridDim.x * blockDim.x) {
+        uint4 v = make_uint4(~0u, ~0u, ~0u, ~0u);
+        for (int q = 0; q < n; q++) v = and4(v, __ldg(reinterpret_cast<const uint4*>(B + (int64_t)items[first + q] * W) + w));
+        dst[w] = v;
+    }
+}
+
+// One warp per row.  `out` (pinned host memory): nfreq of every row, then the counts.
 __global__ void k_nfreq(const int32_t* __restrict__ counts, int64_t n_rows, int32_t n_cols, int32_t min_count,
-                        int32_t* __restrict__ nfreq) {
+                        int32_t* __restrict__ nfreq, int32_t* __restrict__ out, const int32_t* flag, int32_t* flag_to) {
     const int64_t g = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
+    if (flag_to && g == 0 && lane == 0) *flag_to = *flag;
     if (g >= n_rows) return;
     const int32_t* row = counts + g * n_cols;
     int32_t c = 0;
-    for (int e = lane; e < n_cols; e += 32) c += row[e] >= min_count;
+    for (int e = lane; e < n_cols; e += 32) {
+        const int32_t v = row[e];
+        c += v >= min_count;
+        if (out) out[n_rows + g * n_cols + e] = v;
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
-    if (lane == 0) nfreq[g] = c;
+    if (lane == 0) {
+        nfreq[g] = c;
+        if (out) out[g] = c;
+    }
 }
 
 // one warp per job row: count the entries >= min_count, reserve space, then write them
@@ -435,11 +462,22 @@ int launch_materialize(const uint32_t* bitmap, int64_t W, uint32_t* masks, const
     return TFIM_OK;
 }
 
+int launch_wave_begin(const uint32_t* bitmap, int64_t W, uint32_t* masks, const MatDesc* mats, const int64_t* off,
+                      const int32_t* items, int32_t b, int32_t* counts, int64_t n_zero, cudaStream_t s) {
+    if (b <= 0) return TFIM_OK;
+    int64_t bx = (W / 4 + 255) / 256;
+    bx = bx < 1 ? 1 : bx > 64 ? 64 : bx;
+    dim3 grid((unsigned)bx, (unsigned)b);
+    k_wave_begin<<<grid, 256, 0, s>>>(bitmap, W, masks, mats, off, items, counts, n_zero);
+    TFIM_CUDA(cudaGetLastError());
+    return TFIM_OK;
+}
+
 int launch_nfreq(const int32_t* counts, int64_t n_rows, int32_t n_cols, int32_t min_count, int32_t* nfreq,
-                 cudaStream_t s) {
+                 cudaStream_t s, int32_t* out, const int32_t* flag, int32_t* flag_to) {
     if (n_rows <= 0) return TFIM_OK;
     const int64_t threads = n_rows * 32;
-    k_nfreq<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(counts, n_rows, n_cols, min_count, nfreq);
+    k_nfreq<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(counts, n_rows, n_cols, min_count, nfreq, out, flag, flag_to);
     TFIM_CUDA(cudaGetLastError());
     return TFIM_OK;
 }

@@ -144,7 +144,8 @@ __global__ void k_parse_tail(int64_t* off, int64_t n_nl, int64_t n_ids, int64_t*
 // Copy the file bytes into d_text.  A pinned host buffer goes in one copy; otherwise worker
 // threads fill pinned chunks (memcpy from the host buffer, or pread from the file) and each
 // enqueues its chunk's copy on its own stream, so reading chunk k+1 overlaps copying chunk k.
-constexpr size_t kUploadChunk = 8u << 20;
+// 2 MiB chunks: an 18.8 MB file keeps eight workers busy (three with 8 MiB chunks).
+constexpr size_t kUploadChunk = 2u << 20;
 
 int upload_text(const TextSource& src, uint8_t* d_text, cudaStream_t s) {
     const int64_t n = src.n_bytes;
@@ -176,7 +177,7 @@ int upload_text(const TextSource& src, uint8_t* d_text, cudaStream_t s) {
             errs[wk] = what;
             failed.store(1);
         };
-        if (cudaStreamCreateWithFlags(&ws, cudaStreamNonBlocking) != cudaSuccess ||
+        if (stream_get(&ws) != cudaSuccess ||
             cudaEventCreateWithFlags(&ev[0], cudaEventDisableTiming) != cudaSuccess ||
             cudaEventCreateWithFlags(&ev[1], cudaEventDisableTiming) != cudaSuccess) {
             fail("stream or event creation failed");
@@ -220,7 +221,7 @@ int upload_text(const TextSource& src, uint8_t* d_text, cudaStream_t s) {
     work(0);
     for (auto& t : th) t.join();
     for (auto ws : streams)
-        if (ws) cudaStreamDestroy(ws);
+        stream_put(ws);
     if (failed.load()) {
         for (auto& e : errs)
             if (!e.empty()) { set_error("%s", e.c_str()); break; }

@@ -2084,6 +2084,7 @@ int release_cached(int dev) {
     std::lock_guard<std::mutex> lk(g_cache_mu);
     for (int d = 0; d < 64; d++) {
         if (dev >= 0 && d != dev) continue;
+        stream_release(d);
         if (!g_cached_res[d] && !g_cached_masks[d].p) continue;
         TFIM_CUDA(cudaSetDevice(d));
         if (g_cached_res[d]) free_resident(g_cached_res[d], nullptr);

@@ -57,6 +57,11 @@ int dev_alloc(void** p, size_t bytes, cudaStream_t s);
 void dev_free(void* p, cudaStream_t s);
 void* pinned_alloc(size_t bytes, size_t* got);
 void pinned_free(void* p, size_t bytes);
+// Non-blocking streams of the current device from a bounded free list (creating one takes 0.3 ms);
+// a stream goes back idle.  stream_release destroys the idle ones of a device.
+cudaError_t stream_get(cudaStream_t* s);
+void stream_put(cudaStream_t s);
+void stream_release(int dev);
 
 // A device buffer that grows on demand (stream-ordered on `stream`), freed with its owner.
 struct DevBuf {
@@ -191,6 +196,7 @@ int configure_count_kernels();
 constexpr int kF4Cols = 128, kF4Rows = 256;
 int launch_count_f4(const CountArgs& a, cudaStream_t s);
 int count_f4_status_fetch(int32_t* pinned, cudaStream_t s);
+int count_f4_flag(const int32_t** flag);   // the flag's address on the current device
 int count_f4_status_check(int32_t v);
 void tiles_f4(int32_t job, int32_t nr, int32_t nc, int64_t W, int sms, std::vector<TileDesc>& out, bool upper = false);
 // Packed tcgen05 kind::mxf4 family counter (count_pk.cu): a tile holds the X rows of `nr` jobs of at
@@ -224,9 +230,15 @@ int launch_count_proj(const CountArgs& a, const int32_t* job_ids, int32_t n_jobs
 constexpr int kProjMaxCols = 1024;  // longest column list the projected counter hashes
 int launch_materialize(const uint32_t* bitmap, int64_t W, uint32_t* masks, const MatDesc* mats,
                        const int32_t* items, int32_t n, cudaStream_t s);
-// nfreq[g] = #{c < n_cols : counts[g*n_cols + c] >= min_count} for g < n_rows
+// The begin of a counting wave: the b prefix masks (masks[i] = AND of node i's items, lists given by
+// descriptors or by offsets) and n_zero zeros in `counts`.
+int launch_wave_begin(const uint32_t* bitmap, int64_t W, uint32_t* masks, const MatDesc* mats, const int64_t* off,
+                      const int32_t* items, int32_t b, int32_t* counts, int64_t n_zero, cudaStream_t s);
+// nfreq[g] = #{c < n_cols : counts[g*n_cols + c] >= min_count} for g < n_rows.  With `out`, pinned host
+// memory takes nfreq (n_rows) and then the counts too; with flag_to, *flag_to = *flag.
 int launch_nfreq(const int32_t* counts, int64_t n_rows, int32_t n_cols, int32_t min_count,
-                 int32_t* nfreq, cudaStream_t s);
+                 int32_t* nfreq, cudaStream_t s, int32_t* out = nullptr, const int32_t* flag = nullptr,
+                 int32_t* flag_to = nullptr);
 // For each job row g (global row index over all jobs, row_job[g] = its job):
 // entries >= min_count are appended to `entries` (one atomic reservation per row) and
 // row_info[g] = (start, len).  counter[0] ends as the total entry count.
@@ -349,10 +361,19 @@ struct TextSource {
 // *d_off (n_rows + 1 int64) and *d_items (max(nnz, 1) int32), both from dev_alloc on `s`.
 int parse_text_device(const TextSource& src, cudaStream_t s, int64_t** d_off, int32_t** d_items, int64_t* n_rows,
                       int64_t* nnz);
+// The lists of a counting wave: on the device as descriptors or offsets, or on the host.
+struct WaveLists {
+    const int32_t* d_items = nullptr;
+    const MatDesc* d_mats = nullptr;
+    const int64_t* d_off = nullptr;
+    const int32_t* h_items = nullptr;
+    const int64_t* h_off = nullptr;
+};
 // Per-node prefix masks from item lists and one count job over every counted row (abi.cu):
 // counts[i][e] = popc(AND of node i's items & B[e]), nfreq[i] = #{e : counts >= min_count}.
-int count_wave_impl(tfim_ctx* c, int32_t b, int32_t min_count, const int32_t* d_items, const MatDesc* d_mats,
-                    int32_t* d_counts, int32_t* d_nfreq, cudaStream_t s);
+// Returns when they are there; with `out` (pinned), nfreq and counts are in it too.
+int count_wave_impl(tfim_ctx* c, int32_t b, int32_t min_count, const WaveLists& L, int32_t* d_counts, int32_t* d_nfreq,
+                    cudaStream_t s, int32_t* out = nullptr);
 // In-place all-reduce of `count` device elements over a sharded context's group, ordered on
 // `s`; nothing for an unsharded context (shard.cu).
 int group_reduce(tfim_ctx* c, void* d_buf, int64_t count, int32_t dtype, int32_t op, cudaStream_t s);
