@@ -90,12 +90,12 @@ struct ResStatus {
     int64_t g_out, g_tiles;
     int32_t launch_id, next3, next1;         // next3 / next1: tile counters of the persistent counters
     int32_t tiles_l3d;                       // the first tiles_l3d CUDA-core tiles are dense families'
-    int32_t tiles_tc, pad3;                  // packed tcgen05 family counter: tiles
+    int32_t tiles_tc, small;                  // packed tcgen05 family counter: tiles; the wave is the device loop's
     int32_t tiles_gr, next_gr;               // CUDA-core Gram counter: tiles, tile counter
     unsigned long long launch_t0;
     unsigned long long supports, nodes, lookaheads, hits, skipped, pep;
     // superset check: MFIs [0, sup_done) are in the item -> MFI index the expand reads
-    int32_t sup_done, pad2;
+    int32_t sup_done, loop_go;               // loop_go: 1 run the packed wave, 0 leave, 2 leave (time limit)
     unsigned long long sup_pruned;
     // phase stamps of the current wave (first block start, last block end; %globaltimer ns)
     // and their durations summed over the search; the pack folds and resets them
@@ -252,6 +252,10 @@ constexpr int kGramMaxWords = 4096;
 
 constexpr int kPackThreads = 1024;
 constexpr int kPackItems = 4;
+// A wave of at most this many rows x columns x words is counted inside the device loop (mines at
+// 3e7 / 1e8 / 2e8 / 6e8: 2M dense rows 0.395 / 0.314 / 0.314 / 0.313 ms, 196,000 rows of the dense
+// replicated database at 10% 1.03 / 0.91 / 0.90 / 1.02 ms).
+constexpr float kLoopMaxWork = 2e8f;
 constexpr int kPackCand = kPackThreads * kPackItems;
 
 // The packed tcgen05 counter takes a family job (its rows are a run of its columns) of at most
@@ -314,6 +318,7 @@ constexpr int kPackSearch = 5120;   // jobs whose prefixes fit the shared search
 template <int N, typename T>
 __device__ __forceinline__ void block_scan(T (&v)[N], T (&ex)[N], T (&tot)[N], T* sm, bool any) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int warps = blockDim.x >> 5;
     T inc[N];
 #pragma unroll
     for (int k = 0; k < N; k++) inc[k] = v[k];
@@ -331,14 +336,14 @@ __device__ __forceinline__ void block_scan(T (&v)[N], T (&ex)[N], T (&tot)[N], T
         for (int k = 0; k < N; k++) sm[k * 33 + warp] = inc[k];
     __syncthreads();
     if (warp < N) {   // warp k scans value k's warp totals
-        const T own = sm[warp * 33 + lane];
+        const T own = lane < warps ? sm[warp * 33 + lane] : T(0);
         T x = own;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const T y = __shfl_up_sync(0xffffffffu, x, o);
             if (lane >= o) x += y;
         }
-        sm[warp * 33 + lane] = x - own;
+        if (lane < warps) sm[warp * 33 + lane] = x - own;
         if (lane == 31) sm[warp * 33 + 32] = x;
     }
     __syncthreads();
@@ -367,14 +372,18 @@ __device__ __forceinline__ int64_t slice_words(int64_t total, int64_t want) {
     return lmax(1, (total / lmax(want, 1) + 63) / 64) * 64;
 }
 
+// NT: threads of the block.  LOOP: the wave loop on the device (k_res_loop), which counts waves of
+// at most kLoopMaxWork itself; these get no tiles.
+template <int NT, bool LOOP>
 __device__ __forceinline__ void res_pack(const ResPtrs& p) {
+    constexpr int kPackThreads = NT, kPackCand = NT * kPackItems;
     __shared__ int64_t sm64[2 * 33];
     __shared__ int32_t sm32[kPkClasses * 33];
     __shared__ int32_t s_pre[kPackSearch];
     __shared__ int32_t s_src[kPackSearch];
     __shared__ int32_t s_n_jobs, s_rows_total, s_done, s_max_cols, s_max_head, s_stack_after, s_kstop, s_fit;
     __shared__ int64_t s_out_total;
-    __shared__ float s_cost, s_pk_work, s_pk_cost;
+    __shared__ float s_cost, s_pk_work, s_pk_cost, s_work;
     __shared__ unsigned long long s_words[3];   // words of the wave's b1 / tcgen05 / Gram tiles
     ResStatus* st = p.st;
     const int tid = threadIdx.x, lane = tid & 31;
@@ -393,7 +402,7 @@ __device__ __forceinline__ void res_pack(const ResPtrs& p) {
     if (tid == 32) {
         s_n_jobs = n_look; s_rows_total = n_look; s_out_total = 0; s_max_cols = 0; s_max_head = 0; s_done = 0;
         s_stack_after = st->stack_n;
-        s_cost = s_pk_work = s_pk_cost = 0.f;
+        s_cost = s_pk_work = s_pk_cost = s_work = 0.f;
         s_words[0] = s_words[1] = s_words[2] = 0;
         st->n_proj = 0;
         st->n_mjobs = 0;
@@ -601,7 +610,26 @@ __device__ __forceinline__ void res_pack(const ResPtrs& p) {
         const float nr = (float)min(jd.n_rows, kLop3Rows), nc = (float)min(jd.n_cols, 64);
         return (float)(jd.words >> 2) * (1.f + d * (2.f + nr + nr * nc / 32.f));
     };
-    {
+    if (LOOP) {   // rows x columns x words of the wave
+        float work = 0.f;
+        for (int j = tid; j < nj; j += kPackThreads) {
+            const JobDesc jd = p.jobs[j];
+            work += (float)jd.n_rows * (float)jd.n_cols * (float)jd.words;
+        }
+        if ((tid & ~31) < nj) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) work += __shfl_xor_sync(0xffffffffu, work, o);
+            if (lane == 0) atomicAdd(&s_work, work);
+        }
+        __syncthreads();
+    }
+    const bool small = LOOP && s_work <= kLoopMaxWork;
+    if (small)
+        for (int j = tid; j < nj; j += kPackThreads) {
+            p.djobs[j].cls = kGrpLight;
+            p.djobs[j].pad = p.fams[p.djobs[j].fam].n;
+        }
+    if (!small) {
         float cost = 0.f, pk_work = 0.f, pk_cost = 0.f;   // of the packed jobs: pairs x words; as CUDA-core tiles
         unsigned long long w1 = 0, wt = 0, wg = 0;
         for (int j = tid; j < nj; j += kPackThreads) {
@@ -675,7 +703,7 @@ __device__ __forceinline__ void res_pack(const ResPtrs& p) {
     const int64_t sw_tc = slice_words((int64_t)s_words[1], (int64_t)(p.tc_tiles_per_sm * (float)p.sm_count));
     const int64_t sw_gr = slice_words((int64_t)s_words[2], (int64_t)(p.l3_slices_per_sm * (float)p.sm_count));
     int32_t tot[kGrps] = {0, 0, 0, 0, 0, 0};
-    for (int base = 0; base < nj; base += kPackThreads) {
+    for (int base = 0; base < (small ? 0 : nj); base += kPackThreads) {
         const int j = base + tid;
         int32_t v[kGrps] = {0, 0, 0, 0, 0, 0}, ex[kGrps], t[kGrps];
         if (j < nj) {
@@ -748,7 +776,7 @@ __device__ __forceinline__ void res_pack(const ResPtrs& p) {
         }
         return run;
     };
-    if (s_words[1] > 0) {
+    if (!small && s_words[1] > 0) {
         for (int base = 0; base < nj; base += kPackThreads) {
             const int j = base + tid;
             int32_t v[kPkClasses] = {0, 0, 0, 0, 0, 0, 0}, ex[kPkClasses], t[kPkClasses];
@@ -893,6 +921,7 @@ __device__ __forceinline__ void res_pack(const ResPtrs& p) {
     if (TT > 0) pk_tiles(true);
     emit(kGrpGram, p.tiles_gr, 0);
     if (tid == 0) {
+        st->small = small ? 1 : 0;
         st->jobs = nj;
         st->rows = rows_total;
         st->tiles_l3 = (int32_t)T3;
@@ -911,10 +940,10 @@ __device__ __forceinline__ void res_pack(const ResPtrs& p) {
     }
 }
 
-__global__ void __launch_bounds__(kPackThreads) k_res_pack(ResPtrs p) { res_pack(p); }
+__global__ void __launch_bounds__(kPackThreads) k_res_pack(ResPtrs p) { res_pack<kPackThreads, false>(p); }
 __global__ void __launch_bounds__(kPackThreads) k_res_pack_g(const ResArgs* __restrict__ args) {
     const ResPtrs p = args->p;
-    res_pack(p);
+    res_pack<kPackThreads, false>(p);
 }
 
 // ---------------------------------------------------------------------------------- expand helpers
@@ -1775,6 +1804,159 @@ __global__ void __launch_bounds__(128) k_proj_commit(ResPtrs p) {
     }
 }
 
+// ---------------------------------------------------------------------------------- device loop
+// Searches over short rows are chains of small waves: a 10,000-row dense database takes eight
+// waves of about 10 us of counting, and each cost a launch of every phase, a clear, a status copy
+// and a host wait, 85 us.  This kernel runs such waves back to back with its whole grid resident
+// (cooperative launch): block 0 packs, then all blocks count, expand and build masks, with a grid
+// barrier after each.  A wave of more than kLoopMaxWork, and one that needs larger pools, is left
+// to the host.  Measured: 10,000-row dense mine 0.70 -> 0.43 ms (31 us a wave), 2M-row one 0.43 ->
+// 0.31 ms, 500,000 rows at 82% 0.53 -> 0.33 ms.
+constexpr int kLoopThreads = 512;
+constexpr int kLoopMaxWords = 4096;     // rows of the databases that take it;
+constexpr int kLoopDenseWords = 1 << 16; // of dense ones (minimum support at least 1/64 of the transactions)
+constexpr int kLoopCols = 8;            // columns a warp counts at once
+constexpr uint32_t kLoopSpin = 1u << 22;
+
+// All blocks of the grid (`target` arrivals); false when the wait expired.  The fences order the
+// phases' plain loads and stores, as those of a grid-wide sync do.
+__device__ __forceinline__ bool grid_barrier(uint32_t* bar, uint32_t target) {
+    __shared__ int s_ok;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(bar, 1u);
+        uint32_t k = 0;
+        while (*(volatile uint32_t*)bar < target && ++k < kLoopSpin) __nanosleep(20);
+        s_ok = k < kLoopSpin;
+        __threadfence();
+    }
+    __syncthreads();
+    return s_ok != 0;
+}
+
+// Word slices of a wave's rows: enough for two tasks per warp, of at least 256 words.
+__device__ __forceinline__ int32_t loop_slices(const ResPtrs& p) {
+    const int64_t tasks = (int64_t)max(p.st->rows, 1) * max((p.st->max_cols + kLoopCols - 1) / kLoopCols, 1);
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+    return (int32_t)lmax(1, lmin((2 * warps + tasks - 1) / tasks, p.W / 256));
+}
+
+// Counts of the wave's rows: one warp per row, kLoopCols columns and word slice (several slices add
+// into cleared counts).  Masks, lists and counts are written during this kernel, so only bitmap
+// rows are read through the read-only path.
+__device__ __forceinline__ void loop_count(const ResPtrs& p, int32_t slices) {
+    const int32_t rows = p.st->rows, chunks = (p.st->max_cols + kLoopCols - 1) / kLoopCols;
+    const int lane = threadIdx.x & 31;
+    const int32_t warps = gridDim.x * (blockDim.x >> 5);
+    const int64_t tasks = (int64_t)rows * chunks;
+    for (int64_t u = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; u < tasks * slices; u += warps) {
+        const int32_t slice = (int32_t)(u / tasks);
+        const int64_t t = u - slice * tasks;
+        const int32_t g = (int32_t)(t / chunks), c0 = (int32_t)(t % chunks) * kLoopCols;
+        const JobDesc jd = p.jobs[p.row_job[g]];
+        if (c0 >= jd.n_cols) continue;
+        const RowDesc rd = p.rows[g];
+        const uint4* bm = jd.base_slot >= 0 ? reinterpret_cast<const uint4*>(p.masks + (int64_t)jd.base_slot * p.W) : nullptr;
+        const uint4* bi = jd.base_item >= 0 ? reinterpret_cast<const uint4*>(row_of(p, jd.base_item)) : nullptr;
+        const uint4* rm = rd.slot >= 0 ? reinterpret_cast<const uint4*>(p.masks + (int64_t)rd.slot * p.W) : nullptr;
+        const uint4* ri = rd.item >= 0 ? reinterpret_cast<const uint4*>(row_of(p, rd.item)) : nullptr;
+        const uint4* col[kLoopCols];   // null: all ones
+        int32_t acc[kLoopCols];
+#pragma unroll
+        for (int k = 0; k < kLoopCols; k++) {
+            const int32_t c = min(c0 + k, jd.n_cols - 1);
+            const int32_t id = c == jd.self_col ? -1 : p.items[jd.col_off + c];
+            col[k] = id >= 0 ? reinterpret_cast<const uint4*>(row_of(p, id)) : nullptr;
+            acc[k] = 0;
+        }
+        const int32_t W4 = jd.words >> 2, per = (W4 + slices - 1) / slices;
+        for (int32_t w = slice * per + lane; w < min(W4, (slice + 1) * per); w += 32) {
+            uint4 v = make_uint4(~0u, ~0u, ~0u, ~0u);
+            auto andv = [&](uint4 x) { v.x &= x.x; v.y &= x.y; v.z &= x.z; v.w &= x.w; };
+            if (bm) andv(bm[w]);
+            if (bi) andv(__ldg(bi + w));
+            if (rm) andv(rm[w]);
+            if (ri) andv(__ldg(ri + w));
+#pragma unroll
+            for (int k = 0; k < kLoopCols; k++) {
+                const uint4 x = col[k] ? __ldg(col[k] + w) : make_uint4(~0u, ~0u, ~0u, ~0u);
+                acc[k] += __popc(v.x & x.x) + __popc(v.y & x.y) + __popc(v.z & x.z) + __popc(v.w & x.w);
+            }
+        }
+        int32_t mine = 0;
+#pragma unroll
+        for (int k = 0; k < kLoopCols; k++) {
+            const int32_t n = __reduce_add_sync(0xffffffffu, acc[k]);
+            if (lane == k) mine = n;
+        }
+        if (lane < kLoopCols && c0 + lane < jd.n_cols) {
+            int32_t* out = p.counts + jd.out_off + (int64_t)p.row_local[g] * jd.n_cols + c0 + lane;
+            if (slices == 1) *out = mine;
+            else if (mine) atomicAdd(out, mine);
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kLoopThreads, 1) k_res_loop(ResPtrs p, uint32_t* bar) {
+    ResStatus* st = p.st;
+    uint32_t arrived = 0;
+    bool first = true;
+    while (true) {
+        if (blockIdx.x == 0) {
+            // a launch gives the device back after max_launch_ns; the next one continues
+            const bool late = !first && globaltimer() - st->launch_t0 > p.max_launch_ns;
+            if (__syncthreads_or(late)) {
+                if (threadIdx.x == 0) st->loop_go = 2;
+            } else {
+                res_pack<kLoopThreads, true>(p);
+                __syncthreads();
+                if (threadIdx.x == 0) st->loop_go = st->jobs > 0 && st->small && !st->error ? 1 : 0;
+            }
+        }
+        first = false;
+        bool ok = grid_barrier(bar, arrived += gridDim.x);
+        if (!ok || st->loop_go != 1) {
+            if (!ok && threadIdx.x == 0) atomicExch(&st->error, 3);
+            return;
+        }
+        phase_begin(&st->ph_s[kPhLop3]);
+        const int32_t slices = loop_slices(p);
+        if (slices > 1) {
+            const int64_t n = st->out_total;
+            for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+                p.counts[i] = 0;
+            if (!grid_barrier(bar, arrived += gridDim.x)) {
+                if (threadIdx.x == 0) atomicExch(&st->error, 3);
+                return;
+            }
+        }
+        loop_count(p, slices);
+        phase_end(&st->ph_e[kPhLop3]);
+        ok = grid_barrier(bar, arrived += gridDim.x);
+        if (ok) {
+            phase_begin(&st->ph_s[kPhExpand]);
+            const int32_t rows = st->rows;
+            const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+            for (int64_t g = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; g < rows; g += warps)
+                expand_row(p, g, threadIdx.x & 31);
+            phase_end(&st->ph_e[kPhExpand]);
+            ok = grid_barrier(bar, arrived += gridDim.x);
+        }
+        if (ok) {
+            phase_begin(&st->ph_s[kPhMasks]);
+            build_masks(p);
+            phase_end(&st->ph_e[kPhMasks]);
+            if (blockIdx.x == 0 && threadIdx.x == 0) st->waves += 1;
+            ok = grid_barrier(bar, arrived += gridDim.x);
+        }
+        if (!ok) {
+            if (threadIdx.x == 0) atomicExch(&st->error, 3);
+            return;
+        }
+    }
+}
+
 // ---------------------------------------------------------------------------------- graph loop
 // The wave loop as a graph: a conditional WHILE node whose body is
 //   pack -> zero the count block -> persistent counters -> persistent expand -> control.
@@ -1995,7 +2177,7 @@ struct ResidentState {
     Pool fams, items, heads, stack, looks, free_slots, defer, mfi_off, mfi_len, mfi_sup, mfi_items, log_feat, log_label;
     Pool djobs, jobs, rows, row_job, row_local, tiles_l3, tiles_b1, tiles_tc, tiles_gr, counts, status, is_root, dense_freq, top_pos,
         top_diag, proj_list, args, top_sum, mjobs, sup_index;
-    Pool pk_list;
+    Pool pk_list, loop_bar;
     Pool pjobs, pj_off, pj_pool, vrows, vitem;              // projected families
     Pool ord_keys, ord_idx, ord_meta, ord_items, ord_tmp;   // output order of the MFIs
     HostBuf h_status, h_args, h_res, h_setup;
@@ -2013,7 +2195,7 @@ struct ResidentState {
         for (Pool* b : {&fams, &items, &heads, &stack, &looks, &free_slots, &defer, &mfi_off, &mfi_len, &mfi_sup, &mfi_items,
                         &log_feat, &log_label, &djobs, &jobs, &rows, &row_job, &row_local, &tiles_l3, &tiles_b1, &tiles_tc, &tiles_gr, &counts,
                         &status, &is_root, &dense_freq, &top_pos, &top_diag, &proj_list, &args, &top_sum, &mjobs,
-                        &sup_index, &pk_list, &pjobs, &pj_off, &pj_pool, &vrows, &vitem, &ord_keys, &ord_idx, &ord_meta, &ord_items, &ord_tmp}) {
+                        &sup_index, &pk_list, &loop_bar, &pjobs, &pj_off, &pj_pool, &vrows, &vitem, &ord_keys, &ord_idx, &ord_meta, &ord_items, &ord_tmp}) {
             dev_free(b->p, s);
             b->p = nullptr;
             b->bytes = 0;
@@ -2700,9 +2882,22 @@ int mine_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt) {
         used_tc = true;
         if (with_proj) path_launches[TFIM_PATH_PROJ] += hst->waves;
     }
+    const bool loop = !use_graph && W <= (64 * (int64_t)minc >= c->n_bits ? kLoopDenseWords : kLoopMaxWords) && !sup_on && !may_list &&
+                      (o->counter == TFIM_COUNTER_AUTO || o->counter == TFIM_COUNTER_LOP3);
+    if (loop) TFIM_TRY(grow(R.loop_bar, 16, s));
     while (!use_graph) {
-        k_res_pack<<<1, kPackThreads, 0, s>>>(P);
-        TFIM_CUDA(cudaGetLastError());
+        if (loop) {
+            uint32_t* bar = (uint32_t*)R.loop_bar.p;
+            TFIM_CUDA(cudaMemsetAsync(bar, 0, 16, s));
+            P.launch_id = ++R.launch_id;
+            void* args[] = {&P, &bar};
+            TFIM_CUDA(cudaLaunchCooperativeKernel((const void*)k_res_loop, dim3(sm_count), dim3(kLoopThreads), args, 0, s));
+            count_launches++;
+            path_launches[TFIM_PATH_LOP3]++;
+        } else {
+            k_res_pack<<<1, kPackThreads, 0, s>>>(P);
+            TFIM_CUDA(cudaGetLastError());
+        }
         launches++;
         TFIM_CUDA(cudaMemcpyAsync(hst, R.status.p, sizeof(ResStatus), cudaMemcpyDeviceToHost, s));
         const double ts = std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count();
@@ -2713,6 +2908,7 @@ int mine_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt) {
             TFIM_TRY(grow_for(*hst));
             continue;
         }
+        if (loop && hst->loop_go == 2) continue;   // the launch's time limit: go on
         if (hst->jobs == 0) break;
         TFIM_CUDA(cudaMemsetAsync(R.counts.p, 0, (size_t)hst->out_total * 4, s));
         CountArgs a;
@@ -2788,7 +2984,7 @@ int mine_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt) {
         launches++;
         host_waves++;
     }
-    waves += use_graph ? (int64_t)hst->waves : host_waves;
+    waves += host_waves + (int64_t)hst->waves;   // the graph's or the device loop's, and the host's
     // results
     const auto t_read0 = std::chrono::steady_clock::now();
     const ResStatus fin = *hst;
