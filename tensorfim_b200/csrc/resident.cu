@@ -192,6 +192,7 @@ struct ResPtrs {
     PJob* pjobs;
     int32_t* pj_off;              // per family to project: bits before each tile, tiles + 1 entries
     uint32_t* pj_pool;
+    ResStatus* h_st;              // pinned copy of the status record, written by the host-driven packs
 };
 // The dense item id of an F list entry.
 __device__ __forceinline__ int32_t item_of(const ResPtrs& p, int32_t id) { return id < p.n_base ? id : p.vitem[id - p.n_base]; }
@@ -256,6 +257,9 @@ constexpr int kPackItems = 4;
 // 3e7 / 1e8 / 2e8 / 6e8: 2M dense rows 0.395 / 0.314 / 0.314 / 0.313 ms, 196,000 rows of the dense
 // replicated database at 10% 1.03 / 0.91 / 0.90 / 1.02 ms).
 constexpr float kLoopMaxWork = 2e8f;
+// The empty prefix's family up to this many items^2 x words is counted there too (10,000-row dense
+// database 0.394 -> 0.368 ms a mine, 70,000 rows at 90% 0.109 -> 0.088; beyond, the tensor tiles win).
+constexpr double kLoopTopWork = 1e7;
 constexpr int kPackCand = kPackThreads * kPackItems;
 
 // The packed tcgen05 counter takes a family job (its rows are a run of its columns) of at most
@@ -940,7 +944,19 @@ __device__ __forceinline__ void res_pack(const ResPtrs& p) {
     }
 }
 
-__global__ void __launch_bounds__(kPackThreads) k_res_pack(ResPtrs p) { res_pack<kPackThreads, false>(p); }
+// The status record into pinned host memory (one block).
+__device__ __forceinline__ void publish_status(const ResPtrs& p) {
+    __syncthreads();
+    static_assert(sizeof(ResStatus) % 8 == 0, "the record is copied in 8-byte words");
+    const volatile unsigned long long* from = reinterpret_cast<const volatile unsigned long long*>(p.st);
+    unsigned long long* to = reinterpret_cast<unsigned long long*>(p.h_st);
+    for (int i = threadIdx.x; i < (int)(sizeof(ResStatus) / 8); i += blockDim.x) to[i] = from[i];
+}
+
+__global__ void __launch_bounds__(kPackThreads) k_res_pack(ResPtrs p) {
+    res_pack<kPackThreads, false>(p);
+    publish_status(p);
+}
 __global__ void __launch_bounds__(kPackThreads) k_res_pack_g(const ResArgs* __restrict__ args) {
     const ResPtrs p = args->p;
     res_pack<kPackThreads, false>(p);
@@ -1525,52 +1541,53 @@ __global__ void __launch_bounds__(256) k_prune_stack(ResPtrs p) {
     phase_end(&p.st->ph_e[kPhMasks]);
 }
 
-// The expand's first pass for the family of the empty prefix (an n x n count block whose
-// rows are its tail, nT = nF = n): one block per row streams the row with four loads in
-// flight per thread and writes the row's summary.
-__global__ void __launch_bounds__(256) k_top_summary(const int32_t* __restrict__ M, int32_t n, int32_t minc,
-                                                     RowSum* __restrict__ out) {
-    const int32_t i = blockIdx.x;
-    const int32_t* row = M + (int64_t)i * n;
-    const int32_t supc = row[i];
-    const int bs = column_block(n);
-    int n_ext = 0, n_eq = 0, n_tail = 0, prune = 0;
-    unsigned long long blocks = 0;
-    for (int c0 = threadIdx.x; c0 < n; c0 += 4 * 256) {
-        int32_t v4[4];
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const int c = c0 + u * 256;
-            v4[u] = c < n && c != i ? __ldg(row + c) : -1;
-        }
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const int c = c0 + u * 256;
-            const bool e = v4[u] >= minc;
-            const bool eq = e && v4[u] == supc;
-            const bool in_tail = c > i;
-            n_ext += e;
-            n_eq += eq;
-            n_tail += e && !eq && in_tail;
-            prune |= eq && !in_tail;
-            if (e) blocks |= 1ull << (c / bs);
+// The family of the empty prefix (an n x n count block whose rows are its tail, nT = nF = n) is
+// counted in its upper triangle.  This pass reads that once, 32 x 32 entries per block: it
+// forms the expand's first pass over every row (`out`, cleared before) and writes the lower triangle
+// where it matters, the entries of at least minc, and the diagonal.  6,156 items: 104 us as a
+// mirror of the whole triangle and a pass over the rows, 51 us so.
+__global__ void __launch_bounds__(256) k_top_finish(int32_t* __restrict__ M, int32_t n, const int32_t* __restrict__ diag,
+                                                    int32_t minc, RowSum* __restrict__ out) {
+    __shared__ int32_t tile[32][33];
+    const int32_t bi = blockIdx.x, bj = blockIdx.y;   // rows bj, columns bi of the upper triangle
+    if (bj > bi) return;
+    const int lane = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const int bs = column_block(n);   // a multiple of 32: a tile's columns lie in one block
+    int any = 0;
+    for (int k = ty; k < 32; k += 8) {
+        const int32_t r = bj * 32 + k, c = bi * 32 + lane;
+        const int32_t v = r < n && c < n && r < c ? M[(int64_t)r * n + c] : -1;
+        tile[k][lane] = v;
+        const bool e = v >= minc, eq = e && v == diag[r];
+        const unsigned be = __ballot_sync(0xffffffffu, e), bq = __ballot_sync(0xffffffffu, eq);
+        any |= be != 0;
+        if (lane == 0 && be) {   // extensions of row r in its tail
+            atomicAdd(&out[r].n_ext, __popc(be));
+            if (bq) atomicAdd(&out[r].n_eq, __popc(bq));
+            if (be & ~bq) atomicAdd(&out[r].n_tail, __popc(be & ~bq));
+            atomicOr(&out[r].blocks, 1ull << (bi * 32 / bs));
         }
     }
-    typedef cub::BlockReduce<int, 256> RedI;
-    __shared__ typename RedI::TempStorage ti;
-    __shared__ unsigned long long s_blocks;
-    if (threadIdx.x == 0) s_blocks = 0;
-    __syncthreads();
-    if (blocks) atomicOr(&s_blocks, blocks);
-    const int a = RedI(ti).Sum(n_ext);
-    __syncthreads();
-    const int b = RedI(ti).Sum(n_eq);
-    __syncthreads();
-    const int t = RedI(ti).Sum(n_tail);
-    __syncthreads();
-    const int pr = RedI(ti).Reduce(prune, cub::Max());
-    __syncthreads();
-    if (threadIdx.x == 0) out[i] = RowSum{a, b, t, pr, s_blocks, 0};
+    if (bi == bj && threadIdx.x < 32 && bi * 32 + lane < n) {
+        const int32_t r = bi * 32 + lane;
+        M[(int64_t)r * n + r] = diag[r];
+    }
+    if (!__syncthreads_or(any)) return;
+    for (int k = ty; k < 32; k += 8) {
+        const int32_t c = bi * 32 + k, r = bj * 32 + lane;   // row c of the lower triangle, column r
+        const int32_t v = tile[lane][k];
+        const bool e = v >= minc, eq = e && v == diag[c];
+        const unsigned be = __ballot_sync(0xffffffffu, e), bq = __ballot_sync(0xffffffffu, eq);
+        if (e) M[(int64_t)c * n + r] = v;
+        if (lane == 0 && be) {   // extensions of row c outside its tail
+            atomicAdd(&out[c].n_ext, __popc(be));
+            if (bq) {
+                atomicAdd(&out[c].n_eq, __popc(bq));
+                atomicOr(&out[c].prune, 1);
+            }
+            atomicOr(&out[c].blocks, 1ull << (bj * 32 / bs));
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------------- projection
@@ -1804,6 +1821,23 @@ __global__ void __launch_bounds__(128) k_proj_commit(ResPtrs p) {
     }
 }
 
+// The search's initial state, one launch: parts of pinned host memory to their places on the device
+// (in place of a copy each).  Sizes are rounded up to 16 bytes on both sides.
+struct SetupPart {
+    const uint4* src;
+    uint4* dst;
+    int64_t n16;
+};
+struct SetupParts {
+    SetupPart part[16];
+    int32_t n;
+};
+__global__ void __launch_bounds__(256) k_res_setup(SetupParts s) {   // blockIdx.y: the part
+    const SetupPart q = s.part[blockIdx.y];
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < q.n16; i += (int64_t)gridDim.x * blockDim.x)
+        q.dst[i] = q.src[i];
+}
+
 // ---------------------------------------------------------------------------------- device loop
 // Searches over short rows are chains of small waves: a 10,000-row dense database takes eight
 // waves of about 10 us of counting, and each cost a launch of every phase, a clear, a status copy
@@ -1918,6 +1952,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_res_loop(ResPtrs p, uint32_
         bool ok = grid_barrier(bar, arrived += gridDim.x);
         if (!ok || st->loop_go != 1) {
             if (!ok && threadIdx.x == 0) atomicExch(&st->error, 3);
+            if (blockIdx.x == 0) publish_status(p);
             return;
         }
         phase_begin(&st->ph_s[kPhLop3]);
@@ -1928,6 +1963,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_res_loop(ResPtrs p, uint32_
                 p.counts[i] = 0;
             if (!grid_barrier(bar, arrived += gridDim.x)) {
                 if (threadIdx.x == 0) atomicExch(&st->error, 3);
+                if (blockIdx.x == 0) publish_status(p);
                 return;
             }
         }
@@ -1952,6 +1988,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_res_loop(ResPtrs p, uint32_
         }
         if (!ok) {
             if (threadIdx.x == 0) atomicExch(&st->error, 3);
+            if (blockIdx.x == 0) publish_status(p);
             return;
         }
     }
@@ -2026,34 +2063,99 @@ __global__ void k_res_control(const ResArgs* __restrict__ args, cudaGraphConditi
 // ------------------------------------------------------------------------ output order
 // The MFIs leave the device in their output order: descending support, then item lists
 // (each in descending order) compared lexicographically, larger first.  The sort key packs
-// the support and the two largest items, complemented so that an ascending radix sort gives
-// that order.  Narrow keys (support below 2^24, item ids below 2^20 - 1) hold both items;
-// wide ones only the first.  Lists whose keys are equal are finished on the host.
+// the support and the two largest items in as few bits as the database needs, complemented so
+// that an ascending radix sort gives that order; where 64 bits do not hold them (i_bits = 0), 32
+// bits of support and the largest item.  Lists whose keys are equal are finished on the host.
+struct MfiKey {
+    int32_t s_bits, i_bits;
+    __host__ __device__ int bits() const { return i_bits ? s_bits + 2 * i_bits : 64; }
+};
+__device__ __forceinline__ uint64_t mfi_key(MfiKey f, const int32_t* items, int32_t l, uint32_t sup) {
+    int32_t a = -1, b = -1;   // the two largest items
+    for (int32_t q = 0; q < l; q++) {
+        const int32_t x = items[q];
+        if (x > a) {
+            b = a;
+            a = x;
+        } else if (x > b) {
+            b = x;
+        }
+    }
+    if (!f.i_bits) return ((uint64_t)(0xFFFFFFFFu - sup) << 32) | (uint64_t)(0xFFFFFFFFu - (uint32_t)(a + 1));
+    const uint64_t im = (1ull << f.i_bits) - 1, smax = (1ull << f.s_bits) - 1;
+    return ((smax - sup) << (2 * f.i_bits)) | ((im - (uint64_t)(a + 1)) << f.i_bits) | (im - (uint64_t)(b + 1));
+}
+
 __global__ void __launch_bounds__(256) k_mfi_keys(const int32_t* __restrict__ off, const int32_t* __restrict__ len,
                                                   const int32_t* __restrict__ sup, const int32_t* __restrict__ items,
-                                                  int32_t n, int wide, uint64_t* __restrict__ keys,
+                                                  int32_t n, MfiKey f, uint64_t* __restrict__ keys,
                                                   int32_t* __restrict__ idx) {
     for (int32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        const int32_t o = off[k], l = len[k];
-        int32_t a = -1, b = -1;   // the two largest items
-        for (int32_t q = 0; q < l; q++) {
-            const int32_t x = items[o + q];
-            if (x > a) {
-                b = a;
-                a = x;
-            } else if (x > b) {
-                b = x;
-            }
-        }
-        const uint32_t s = (uint32_t)sup[k];
-        uint64_t key;
-        if (wide) key = ((uint64_t)(0xFFFFFFFFu - s) << 32) | (uint64_t)(0xFFFFFFFFu - (uint32_t)(a + 1));
-        else
-            key = ((uint64_t)(0xFFFFFFu - s) << 40) | ((uint64_t)(0xFFFFFu - (uint32_t)(a + 1)) << 20) |
-                  (uint64_t)(0xFFFFFu - (uint32_t)(b + 1));
-        keys[k] = key;
+        keys[k] = mfi_key(f, items + off[k], len[k], (uint32_t)sup[k]);
         idx[k] = k;
     }
+}
+
+// Few MFIs (at most kFinishMax): one block forms the keys, sorts, places lengths, supports and items
+// in output order and hands them to pinned host memory, in place of six launches and three
+// copies (1,612 MFIs: 57 us of read-back in all against 75).
+constexpr int kFinishThreads = 1024, kFinishItems = 4;
+constexpr int kFinishMax = kFinishThreads * kFinishItems;
+constexpr int64_t kFinishMaxItems = 1 << 16;
+__global__ void __launch_bounds__(kFinishThreads) k_mfi_finish(const int32_t* off, const int32_t* len, const int32_t* sup,
+                                                               const int32_t* items, int32_t n, int64_t ni, MfiKey f,
+                                                               uint4* dev, uint4* host) {
+    typedef cub::BlockRadixSort<uint64_t, kFinishThreads, kFinishItems, int32_t> Sort;
+    __shared__ union {
+        typename Sort::TempStorage sort;
+        int32_t scan[33];
+        struct { int32_t from[kFinishMax], to[kFinishMax]; } g;   // each MFI's place before and after
+    } sm;
+    // keys, lengths, supports, items: one after the other, as the host reads them
+    uint64_t* d_key = reinterpret_cast<uint64_t*>(dev);
+    int32_t* d_len = reinterpret_cast<int32_t*>(d_key + n);
+    int32_t* d_sup = d_len + n;
+    int32_t* d_items = d_sup + n;
+    const int tid = threadIdx.x;
+    uint64_t key[kFinishItems];
+    int32_t idx[kFinishItems];
+#pragma unroll
+    for (int q = 0; q < kFinishItems; q++) {
+        const int32_t k = tid * kFinishItems + q;
+        idx[q] = k;
+        key[q] = k < n ? mfi_key(f, items + off[k], len[k], (uint32_t)sup[k]) : ~0ull;
+    }
+    Sort(sm.sort).Sort(key, idx, 0, f.bits());   // stable: the padding (all ones) stays last
+    __syncthreads();
+    int32_t l[kFinishItems], v[1] = {0}, ex[1], tot[1];
+#pragma unroll
+    for (int q = 0; q < kFinishItems; q++) {
+        l[q] = tid * kFinishItems + q < n ? len[idx[q]] : 0;
+        v[0] += l[q];
+    }
+    block_scan<1>(v, ex, tot, sm.scan, true);
+    int32_t o = ex[0];
+#pragma unroll
+    for (int q = 0; q < kFinishItems; q++) {
+        const int32_t k = tid * kFinishItems + q;
+        if (k < n) {
+            d_key[k] = key[q];
+            d_len[k] = l[q];
+            d_sup[k] = sup[idx[q]];
+            sm.g.from[k] = idx[q];
+            sm.g.to[k] = o;
+            o += l[q];
+        }
+    }
+    __syncthreads();
+    // items: eight lanes per MFI
+    for (int32_t k = tid >> 3; k < n; k += kFinishThreads >> 3) {
+        const int32_t m = sm.g.from[k], src = off[m], ll = len[m], dst = sm.g.to[k];
+        for (int32_t x = tid & 7; x < ll; x += 8) d_items[dst + x] = items[src + x];
+    }
+    __syncthreads();
+    const int64_t n16 = ((int64_t)n * 16 + ni * 4 + 15) >> 4;
+    for (int64_t i = tid; i < n16; i += kFinishThreads) host[i] = dev[i];
 }
 
 // Lengths and supports in sorted order.
@@ -2180,7 +2282,7 @@ struct ResidentState {
     Pool pk_list, loop_bar;
     Pool pjobs, pj_off, pj_pool, vrows, vitem;              // projected families
     Pool ord_keys, ord_idx, ord_meta, ord_items, ord_tmp;   // output order of the MFIs
-    HostBuf h_status, h_args, h_res, h_setup;
+    HostBuf h_status, h_args, h_res, h_setup, h_first, h_tiles;
     // the database's part of the search's initial state (root flags, the top family in
     // increasing support order), computed at a context's first resident mine and its pinned
     // staging reused by later mines; setup_uid names the context it belongs to
@@ -2204,6 +2306,8 @@ struct ResidentState {
         h_args.release();
         h_res.release();
         h_setup.release();
+        h_first.release();
+        h_tiles.release();
     }
 };
 
@@ -2286,10 +2390,19 @@ int order_mfis(ResidentState& R, const tfim_ctx* c, const ResPtrs& P, int32_t n,
                cudaStream_t s, uint64_t* hkey, int32_t* hmeta, int32_t* hitems) {
     int32_t max_sup = 0;
     for (int32_t f : c->dense_freq) max_sup = std::max(max_sup, f);
-    const int wide = c->n_bits > 0xFFFFFF || max_sup > 0xFFFFFF || c->info.n_dense > 0xFFFFF ? 1 : 0;
+    auto width = [](uint32_t x) { int b = 1; while (b < 32 && (x >> b)) b++; return b; };
+    MfiKey f{width((uint32_t)std::max<int64_t>(max_sup, c->n_bits)), width((uint32_t)c->info.n_dense)};
+    if (f.s_bits + 2 * f.i_bits > 64) f.i_bits = 0;
+    if (n <= kFinishMax && ni <= kFinishMaxItems) {
+        TFIM_TRY(grow(R.ord_items, (size_t)n * 16 + (size_t)ni * 4 + 16, s));
+        k_mfi_finish<<<1, kFinishThreads, 0, s>>>(P.mfi_off, P.mfi_len, P.mfi_sup, P.mfi_items, n, ni, f,
+                                                  (uint4*)R.ord_items.p, (uint4*)hkey);
+        TFIM_CUDA(cudaGetLastError());
+        return TFIM_OK;
+    }
     size_t t_sort = 0, t_scan = 0;
     TFIM_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, t_sort, (const uint64_t*)nullptr, (uint64_t*)nullptr,
-                                              (const int32_t*)nullptr, (int32_t*)nullptr, n, 0, 64, s));
+                                              (const int32_t*)nullptr, (int32_t*)nullptr, n, 0, f.bits(), s));
     TFIM_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, t_scan, (const int32_t*)nullptr, (int32_t*)nullptr, n, s));
     TFIM_TRY(grow(R.ord_keys, (size_t)n * 16, s));
     TFIM_TRY(grow(R.ord_idx, (size_t)n * 8, s));
@@ -2305,10 +2418,10 @@ int order_mfis(ResidentState& R, const tfim_ctx* c, const ResPtrs& P, int32_t n,
     int32_t* off_o = sup_o + n;
     int32_t* items_o = (int32_t*)R.ord_items.p;
     const unsigned grid = (unsigned)std::min<int64_t>(((int64_t)n + 255) / 256, (int64_t)sm_count * 8);
-    k_mfi_keys<<<grid, 256, 0, s>>>(P.mfi_off, P.mfi_len, P.mfi_sup, P.mfi_items, n, wide, k_in, i_in);
+    k_mfi_keys<<<grid, 256, 0, s>>>(P.mfi_off, P.mfi_len, P.mfi_sup, P.mfi_items, n, f, k_in, i_in);
     TFIM_CUDA(cudaGetLastError());
     size_t t = R.ord_tmp.bytes;
-    TFIM_CUDA(cub::DeviceRadixSort::SortPairs(R.ord_tmp.p, t, k_in, k_out, i_in, i_out, n, 0, 64, s));
+    TFIM_CUDA(cub::DeviceRadixSort::SortPairs(R.ord_tmp.p, t, k_in, k_out, i_in, i_out, n, 0, f.bits(), s));
     k_mfi_permute<<<grid, 256, 0, s>>>(i_out, P.mfi_len, P.mfi_sup, n, len_o, sup_o);
     TFIM_CUDA(cudaGetLastError());
     t = R.ord_tmp.bytes;
@@ -2412,7 +2525,7 @@ int mine_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt) {
     int64_t cap_item = small ? n0 : std::max<int64_t>(4 * top_out + 2 * n0, 1 << 20);   // holds the top family's list
     int64_t cap_head = 1 << 20, cap_mfi = 1 << 16, cap_mfi_items = 1 << 20, cap_slots = 1 << 12, cap_log = 1 << 16;
     if (small) cap_head = cap_mfi = cap_mfi_items = cap_slots = cap_log = 1;
-    TFIM_TRY(grow(R.status, sizeof(ResStatus), s));
+    TFIM_TRY(grow(R.status, sizeof(ResStatus) + 16, s));
     TFIM_TRY(grow(R.fams, cap_fam * sizeof(DFam), s));
     TFIM_TRY(grow(R.items, cap_item * 4, s));
     TFIM_TRY(grow(R.heads, cap_head * 4, s));
@@ -2457,81 +2570,6 @@ int mine_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt) {
     // mask slots (grown on demand)
     int64_t slot_cap = c->d_masks.bytes / ((size_t)W * 4);
 
-    // the search's initial state, staged in pinned memory and copied asynchronously:
-    // root flags, F1 counts, the top family record, its F list and its single job, rows,
-    // F positions and row supports, the status record
-    DFam top;
-    top.slot = -1; top.item = -1; top.head_off = 0; top.head_len = 0; top.F_off = 0; top.nF = n0; top.nT = n0;
-    top.sup = 0; top.next_row = n0; top.rows_done = 0; top.state = 0; top.top = 1;
-    top.W = (int32_t)W; top.n = (int32_t)c->n_bits;
-    ResStatus hs;
-    memset(&hs, 0, sizeof hs);
-    for (int k = 0; k < kPhases; k++) hs.ph_s[k] = ~0ull;
-    hs.fam_n = 1;
-    hs.item_n = n0;
-    hs.jobs = 1;
-    hs.rows = n0;
-    hs.out_total = top_out;
-    hs.max_cols = n0;
-    hs.nodes = n0;
-    hs.supports = (unsigned long long)top_out;
-    {
-        // the staging blob is the same for every mine of this database: built once, and the
-        // parts (whose device pools may have moved) copied again on every mine
-        const size_t nd = (size_t)std::max<int32_t>(c->info.n_dense, 1);
-        struct Part { void* dst; size_t off, bytes; };
-        std::vector<Part> parts;
-        size_t total = 0;
-        auto part = [&](void* dst, size_t bytes) {
-            parts.push_back(Part{dst, total, bytes});
-            total += (bytes + 15) & ~size_t(15);
-            return parts.size() - 1;
-        };
-        const size_t p_root = part(R.is_root.p, is_root.size()), p_freq = part(R.dense_freq.p, c->dense_freq.size() * 4),
-                     p_fam = part(R.fams.p, sizeof(DFam)), p_F = part(R.items.p, (size_t)n0 * 4),
-                     p_dj = part(R.djobs.p, sizeof(DJob)), p_jd = part(R.jobs.p, sizeof(JobDesc)),
-                     p_rows = part(R.rows.p, (size_t)n0 * sizeof(RowDesc)), p_rj = part(R.row_job.p, (size_t)n0 * 4),
-                     p_rl = part(R.row_local.p, (size_t)n0 * 4), p_pos = part(R.top_pos.p, nd * 4),
-                     p_diag = part(R.top_diag.p, (size_t)n0 * 4), p_st = part(R.status.p, sizeof(ResStatus));
-        unsigned char* h = nullptr;
-        if (fresh_setup || !R.h_setup.p || R.setup_total != total) {
-            TFIM_TRY(R.h_setup.reserve(total));
-            h = R.h_setup.as<unsigned char>();
-            auto at = [&](size_t k) { return (void*)(h + parts[k].off); };
-            memcpy(at(p_root), is_root.data(), is_root.size());
-            memcpy(at(p_freq), c->dense_freq.data(), c->dense_freq.size() * 4);
-            memcpy(at(p_fam), &top, sizeof top);
-            memcpy(at(p_F), F0.data(), (size_t)n0 * 4);
-            {
-                DJob dj{};
-                dj.kind = kJobFam; dj.nr = n0; dj.slot = -1; dj.log = -1; dj.sl3 = 1;
-                *(DJob*)at(p_dj) = dj;
-            }
-            *(JobDesc*)at(p_jd) = JobDesc{-1, -1, n0, n0, 0, 0, 0, -1, (int32_t)W};
-            RowDesc* rows = (RowDesc*)at(p_rows);
-            int32_t* rj = (int32_t*)at(p_rj);
-            int32_t* rl = (int32_t*)at(p_rl);
-            int32_t* pos = (int32_t*)at(p_pos);
-            int32_t* diag = (int32_t*)at(p_diag);
-            std::fill(pos, pos + nd, -1);
-            for (int32_t k = 0; k < n0; k++) {
-                rows[k] = RowDesc{-1, F0[k]};
-                rj[k] = 0;
-                rl[k] = k;
-                pos[F0[k]] = k;
-                diag[k] = c->bit_support[F0[k]];
-            }
-            memcpy(at(p_st), &hs, sizeof hs);
-            R.setup_uid = c->uid;
-            R.setup_total = total;
-        }
-        h = R.h_setup.as<unsigned char>();
-        for (const Part& q : parts)
-            if (q.bytes) TFIM_CUDA(cudaMemcpyAsync(q.dst, h + q.off, q.bytes, cudaMemcpyHostToDevice, s));
-    }
-    TFIM_TRY(R.h_status.reserve(sizeof(ResStatus)));
-    ResStatus* hst = R.h_status.as<ResStatus>();
-
     // top family counting: pair co-occurrence or the symmetric bitmap Gram (cost model)
     int top_mode;
     {
@@ -2552,6 +2590,113 @@ int mine_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt) {
     // the tcgen05 wave counter (38 items x 2M transactions: 17 us against 143 on the CUDA-core tiles)
     const bool top_i8 = o->counter != TFIM_COUNTER_LOP3 && o->counter != TFIM_COUNTER_TENSOR && n0 >= tn.i8_min_rows &&
                         n0 >= tn.i8_min_cols;
+
+    // the projected counter, which reads the transaction list, may be picked
+    const bool may_list = c->csr_exact && (o->counter == TFIM_COUNTER_PROJ ||
+                                           (o->counter == TFIM_COUNTER_AUTO && (o->proj_auto >= 0 ? o->proj_auto : tn.proj_auto)));
+    const bool use_graph = o->use_graphs != 0;
+    // small waves run in the device loop; a small enough family of the empty prefix is its first wave
+    const bool loop = !use_graph && W <= (64 * (int64_t)minc >= c->n_bits ? kLoopDenseWords : kLoopMaxWords) && !sup_on && !may_list &&
+                      (o->counter == TFIM_COUNTER_AUTO || o->counter == TFIM_COUNTER_LOP3);
+    // Children of the empty prefix move to universes of their own when the database is long enough
+    // for a wave's counting to outweigh the extra status read (small_pools: any length, so that
+    // short ones exercise it), some frequent item lies in at most half of it, and no counter that
+    // reads the transaction list may be picked.
+    const bool project = (W >= (1 << 12) || small) && 2 * (int64_t)c->bit_support[F0.front()] <= c->n_bits &&
+                         64 * (int64_t)minc >= c->n_bits && !may_list;
+    const bool top_loop = loop && !project && o->top_counter == 0 && top_mode == 1 && n0 <= wave_rows &&
+                          (double)n0 * n0 * (double)W <= kLoopTopWork;
+
+    // the search's initial state, staged in pinned memory and copied asynchronously:
+    // root flags, F1 counts, the top family record, its F list and its single job, rows,
+    // F positions and row supports, the status record
+    DFam top;
+    top.slot = -1; top.item = -1; top.head_off = 0; top.head_len = 0; top.F_off = 0; top.nF = n0; top.nT = n0;
+    top.sup = 0; top.next_row = top_loop ? 0 : n0; top.rows_done = 0; top.state = 0; top.top = 1;
+    top.W = (int32_t)W; top.n = (int32_t)c->n_bits;
+    ResStatus hs;
+    memset(&hs, 0, sizeof hs);
+    for (int k = 0; k < kPhases; k++) hs.ph_s[k] = ~0ull;
+    hs.fam_n = 1;
+    hs.item_n = n0;
+    hs.jobs = 1;
+    hs.rows = n0;
+    hs.out_total = top_out;
+    hs.max_cols = n0;
+    if (top_loop) {
+        hs.stack_n = 1;   // entry 0: the top family
+    } else {
+        hs.nodes = n0;
+        hs.supports = (unsigned long long)top_out;
+    }
+    {
+        SetupParts setup{};
+        // the staging blob is the same for every mine of this database: built once, and the
+        // parts (whose device pools may have moved) copied again on every mine
+        const size_t nd = (size_t)std::max<int32_t>(c->info.n_dense, 1);
+        struct Part { void* dst; size_t off, bytes; };
+        std::vector<Part> parts;
+        size_t total = 0;
+        auto part = [&](void* dst, size_t bytes) {
+            parts.push_back(Part{dst, total, bytes});
+            total += (bytes + 15) & ~size_t(15);
+            return parts.size() - 1;
+        };
+        const size_t p_root = part(R.is_root.p, is_root.size()), p_freq = part(R.dense_freq.p, c->dense_freq.size() * 4),
+                     p_F = part(R.items.p, (size_t)n0 * 4),
+                     p_dj = part(R.djobs.p, sizeof(DJob)), p_jd = part(R.jobs.p, sizeof(JobDesc)),
+                     p_rows = part(R.rows.p, (size_t)n0 * sizeof(RowDesc)), p_rj = part(R.row_job.p, (size_t)n0 * 4),
+                     p_rl = part(R.row_local.p, (size_t)n0 * 4), p_pos = part(R.top_pos.p, nd * 4),
+                     p_diag = part(R.top_diag.p, (size_t)n0 * 4);
+        unsigned char* h = nullptr;
+        if (fresh_setup || !R.h_setup.p || R.setup_total != total) {
+            TFIM_TRY(R.h_setup.reserve(total));
+            h = R.h_setup.as<unsigned char>();
+            auto at = [&](size_t k) { return (void*)(h + parts[k].off); };
+            memcpy(at(p_root), is_root.data(), is_root.size());
+            memcpy(at(p_freq), c->dense_freq.data(), c->dense_freq.size() * 4);
+            memcpy(at(p_F), F0.data(), (size_t)n0 * 4);
+            {
+                DJob dj{};
+                dj.kind = kJobFam; dj.nr = n0; dj.slot = -1; dj.log = -1; dj.sl3 = 1;
+                *(DJob*)at(p_dj) = dj;
+            }
+            *(JobDesc*)at(p_jd) = JobDesc{-1, -1, n0, n0, 0, 0, 0, -1, (int32_t)W};
+            RowDesc* rows = (RowDesc*)at(p_rows);
+            int32_t* rj = (int32_t*)at(p_rj);
+            int32_t* rl = (int32_t*)at(p_rl);
+            int32_t* pos = (int32_t*)at(p_pos);
+            int32_t* diag = (int32_t*)at(p_diag);
+            std::fill(pos, pos + nd, -1);
+            for (int32_t k = 0; k < n0; k++) {
+                rows[k] = RowDesc{-1, F0[k]};
+                rj[k] = 0;
+                rl[k] = k;
+                pos[F0[k]] = k;
+                diag[k] = c->bit_support[F0[k]];
+            }
+            R.setup_uid = c->uid;
+            R.setup_total = total;
+        }
+        h = R.h_setup.as<unsigned char>();
+        for (const Part& q : parts)
+            if (q.bytes) setup.part[setup.n++] = SetupPart{(const uint4*)(h + q.off), (uint4*)q.dst, (int64_t)(q.bytes + 15) / 16};
+        // this mine's records: status, the top family, the stack's first entry
+        const size_t o_top = (sizeof hs + 15) & ~size_t(15), o_stack = o_top + sizeof top;
+        TFIM_TRY(R.h_first.reserve(o_stack + 16));
+        unsigned char* hf = R.h_first.as<unsigned char>();
+        memcpy(hf, &hs, sizeof hs);
+        memcpy(hf + o_top, &top, sizeof top);
+        memset(hf + o_stack, 0, 16);
+        setup.part[setup.n++] = SetupPart{(const uint4*)hf, (uint4*)R.status.p, (int64_t)o_top / 16};
+        setup.part[setup.n++] = SetupPart{(const uint4*)(hf + o_top), (uint4*)R.fams.p, (int64_t)sizeof top / 16};
+        setup.part[setup.n++] = SetupPart{(const uint4*)(hf + o_stack), (uint4*)R.stack.p, 1};
+        static_assert(sizeof(DFam) % 16 == 0, "a family record is whole 16-byte pieces");
+        k_res_setup<<<dim3((unsigned)std::min<size_t>(16, (size_t)n0 / 512 + 1), (unsigned)setup.n), 256, 0, s>>>(setup);
+        TFIM_CUDA(cudaGetLastError());
+    }
+    TFIM_TRY(R.h_status.reserve(sizeof(ResStatus)));
+    ResStatus* hst = R.h_status.as<ResStatus>();
 
     double sync_ms = 0, kernel_ms = 0;
     int64_t launches = 0, count_launches = 0, bytes_alg = 0, waves = 0;
@@ -2624,6 +2769,7 @@ int mine_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt) {
         P.pjobs = (PJob*)R.pjobs.p;
         P.pj_off = (int32_t*)R.pj_off.p;
         P.pj_pool = (uint32_t*)R.pj_pool.p;
+        P.h_st = hst;
     };
     // capacity for the worst case of one expand over `rows` rows of at most `max_cols`
     // columns each and `out_total` counts
@@ -2691,14 +2837,6 @@ int mine_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt) {
         return TFIM_OK;
     };
 
-    // Children of the empty prefix move to universes of their own when the database is long enough
-    // for a wave's counting to outweigh the extra status read (small_pools: any length, so that
-    // short ones exercise it), some frequent item lies in at most half of it, and no counter that
-    // reads the transaction list may be picked.
-    const bool may_list = c->csr_exact && (o->counter == TFIM_COUNTER_PROJ ||
-                                           (o->counter == TFIM_COUNTER_AUTO && (o->proj_auto >= 0 ? o->proj_auto : tn.proj_auto)));
-    const bool project = (W >= (1 << 12) || small) && 2 * (int64_t)c->bit_support[F0.front()] <= c->n_bits &&
-                         64 * (int64_t)minc >= c->n_bits && !may_list;
     auto project_families = [&]() -> int {
         const int64_t nt = proj_tiles(W);
         TFIM_TRY(grow(R.pjobs, (size_t)(n0 + 1) * sizeof(PJob), s));
@@ -2748,7 +2886,9 @@ int mine_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt) {
     // wave 1: the top family, counted whole
     *hst = hs;
     TFIM_TRY(ensure(hs, hs.rows, hs.jobs, hs.out_total, 0, hs.max_cols));
-    {
+    if (top_loop) {
+        stt->setup_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_entry).count();
+    } else {
         std::vector<TileDesc> tl;
         if (top_mode == 1) {
             if (top_i8) {
@@ -2775,9 +2915,12 @@ int mine_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt) {
     TFIM_TRY(grow(R.tiles_gr, cap_tiles * sizeof(TileDesc), s));
             refresh_ptrs();
         }
-        if (!tl.empty())
-            TFIM_CUDA(cudaMemcpyAsync(top_b1 ? R.tiles_b1.p : R.tiles_l3.p, tl.data(), tl.size() * sizeof(TileDesc),
+        if (!tl.empty()) {
+            TFIM_TRY(R.h_tiles.reserve(tl.size() * sizeof(TileDesc)));
+            memcpy(R.h_tiles.p, tl.data(), tl.size() * sizeof(TileDesc));
+            TFIM_CUDA(cudaMemcpyAsync(top_b1 ? R.tiles_b1.p : R.tiles_l3.p, R.h_tiles.p, tl.size() * sizeof(TileDesc),
                                       cudaMemcpyHostToDevice, s));
+        }
         TFIM_CUDA(cudaMemsetAsync(R.counts.p, 0, (size_t)top_out * 4, s));
         CountArgs a;
         a.bitmap = c->d_bitmap; a.W = W; a.masks = c->d_masks.as<uint32_t>(); a.jobs = P.jobs; a.rows = P.rows;
@@ -2794,9 +2937,11 @@ int mine_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt) {
             bytes_alg += row_bytes * 2 * n0 + 4 * top_out;
         }
         TFIM_CUDA(cudaEventRecord(c->ev1, s));
-        TFIM_TRY(launch_mirror(P.counts, n0, top_mode == 2 ? (const int32_t*)R.top_diag.p : nullptr, s));
         TFIM_TRY(grow(R.top_sum, (size_t)n0 * sizeof(RowSum), s));
-        k_top_summary<<<n0, 256, 0, s>>>(P.counts, n0, minc, (RowSum*)R.top_sum.p);
+        TFIM_CUDA(cudaMemsetAsync(R.top_sum.p, 0, (size_t)n0 * sizeof(RowSum), s));
+        const unsigned nb = (unsigned)((n0 + 31) / 32);
+        TFIM_CHECK(nb <= 65535, TFIM_E_INVALID, "family of %d items exceeds the grid", n0);
+        k_top_finish<<<dim3(nb, nb), 256, 0, s>>>(P.counts, n0, (const int32_t*)R.top_diag.p, minc, (RowSum*)R.top_sum.p);
         TFIM_CUDA(cudaGetLastError());
         launches += 3;
         count_launches++;
@@ -2820,9 +2965,8 @@ int mine_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt) {
     }
     // the counting path of the empty-prefix family, its work and (read at the end) its time
     const int top_path = top_mode == 2 ? TFIM_PATH_PAIRS : top_i8 ? TFIM_PATH_TC : top_b1 ? TFIM_PATH_B1 : TFIM_PATH_LOP3;
-    path_launches[top_path]++;
+    if (!top_loop) path_launches[top_path]++;
     // following waves
-    const bool use_graph = o->use_graphs != 0;
     int64_t host_waves = 0;
     if (use_graph) {
         TFIM_TRY(grow(R.args, sizeof(ResArgs), s));
@@ -2882,8 +3026,6 @@ int mine_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt) {
         used_tc = true;
         if (with_proj) path_launches[TFIM_PATH_PROJ] += hst->waves;
     }
-    const bool loop = !use_graph && W <= (64 * (int64_t)minc >= c->n_bits ? kLoopDenseWords : kLoopMaxWords) && !sup_on && !may_list &&
-                      (o->counter == TFIM_COUNTER_AUTO || o->counter == TFIM_COUNTER_LOP3);
     if (loop) TFIM_TRY(grow(R.loop_bar, 16, s));
     while (!use_graph) {
         if (loop) {
@@ -2899,7 +3041,6 @@ int mine_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt) {
             TFIM_CUDA(cudaGetLastError());
         }
         launches++;
-        TFIM_CUDA(cudaMemcpyAsync(hst, R.status.p, sizeof(ResStatus), cudaMemcpyDeviceToHost, s));
         const double ts = std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count();
         TFIM_CUDA(cudaStreamSynchronize(s));
         sync_ms += (std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count() - ts) * 1e3;
@@ -2992,7 +3133,7 @@ int mine_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt) {
     // sort keys, lengths, supports, items
     const int32_t nm = fin.mfi_n;
     const int64_t ni = fin.mfi_item_n;
-    TFIM_TRY(R.h_res.reserve(((size_t)nm * 4 + (size_t)ni + 2) * 4));
+    TFIM_TRY(R.h_res.reserve(((size_t)nm * 4 + (size_t)ni + 8) * 4));   // (whole 16-byte pieces)
     uint64_t* hkey = R.h_res.as<uint64_t>();
     int32_t* hlen = (int32_t*)(hkey + nm);
     int32_t* hsup = hlen + nm;
@@ -3007,7 +3148,7 @@ int mine_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt) {
         TFIM_CUDA(cudaMemcpyAsync(c->la_feats.data(), R.log_feat.p, (size_t)fin.log_n * 32 * 4, cudaMemcpyDeviceToHost, s));
         TFIM_CUDA(cudaMemcpyAsync(c->la_labels.data(), R.log_label.p, (size_t)fin.log_n * 4, cudaMemcpyDeviceToHost, s));
     }
-    const bool used_f4 = top_i8 && top_mode == 1;
+    const bool used_f4 = top_i8 && top_mode == 1 && !top_loop;
     TFIM_TRY(c->h_flags.reserve(64));
     int32_t* flags = c->h_flags.as<int32_t>();
     flags[0] = flags[1] = 0;
@@ -3045,14 +3186,16 @@ int mine_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt) {
     // device times: the empty-prefix family's counting (events) and every later wave's phases
     // (stamps folded by the pack)
     {
-        float top_ms = 0;
-        cudaEventElapsedTime(&top_ms, c->ev0, c->ev1);
-        stt->top_ms += top_ms;
-        kernel_ms += top_ms;
-        stt->path_ms[top_path] += top_ms;
-        stt->path_bytes[top_path] += bytes_alg;
-        stt->path_bitops[top_path] += top_mode == 2 ? 0 : (int64_t)n0 * (n0 + 1) / 2 * c->n_bits;
-        stt->path_supports[top_path] += top_out;
+        if (!top_loop) {
+            float top_ms = 0;
+            cudaEventElapsedTime(&top_ms, c->ev0, c->ev1);
+            stt->top_ms += top_ms;
+            kernel_ms += top_ms;
+            stt->path_ms[top_path] += top_ms;
+            stt->path_bytes[top_path] += bytes_alg;
+            stt->path_bitops[top_path] += top_mode == 2 ? 0 : (int64_t)n0 * (n0 + 1) / 2 * c->n_bits;
+            stt->path_supports[top_path] += top_out;
+        }
         const double ns = 1e-6;
         const int ph_of_path[6] = {kPhLop3, kPhB1, kPhTc, -1, kPhProj, kPhGram};
         const int cls_of_path[6] = {kClsLop3, kClsB1, kClsTc, -1, kClsProj, kClsGram};
