@@ -114,10 +114,11 @@ int count_wave_impl(tfim_ctx* c, int32_t b, int32_t min_count, const WaveLists& 
     std::vector<int32_t> cols(d);
     std::iota(cols.begin(), cols.end(), 0);
     std::vector<TileDesc> tiles;
+    bool wide = false;
     const int64_t W = c->W;
     if (d == 0) {
     } else if (i8) {
-        tiles_f4(0, b, d, W, 148, tiles);
+        wide = tiles_f4(0, b, d, W, 148, tiles);
     } else if (b1) {
         const int64_t base = (int64_t)((b + kB1Rows - 1) / kB1Rows) * ((d + kB1Cols - 1) / kB1Cols);
         const int64_t want = (int64_t)(tn.b1_tiles_per_sm * 148);
@@ -173,7 +174,7 @@ int count_wave_impl(tfim_ctx* c, int32_t b, int32_t min_count, const WaveLists& 
     *flag_to = 0;
     if (d > 0) {
         if (i8) TFIM_TRY(count_f4_flag(&flag));
-        TFIM_TRY(i8 ? launch_count_f4(a, s) : b1 ? launch_count_b1(a, s) : launch_count_lop3(a, s));
+        TFIM_TRY(i8 ? launch_count_f4(a, wide, s) : b1 ? launch_count_b1(a, s) : launch_count_lop3(a, s));
         TFIM_TRY(group_reduce(c, d_counts, (int64_t)b * d, TFIM_DT_I32, TFIM_RED_SUM, s));
     }
     TFIM_TRY(launch_nfreq(d_counts, b, d, min_count, d_nfreq, s, out, flag, flag ? (int32_t*)flag_to : nullptr));

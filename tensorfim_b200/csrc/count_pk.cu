@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(kPThreads, 1) k_count_pk(CountArgs a_val, cons
 #pragma unroll
                             for (int k = 0; k < 4; k++)
                                 mma_mxf4(acc, smem_desc(blk + k * 32), smem_desc(blk + (uint32_t)u0 * 1024u + k * 32), idesc,
-                                         tmem + kPScale + 32u * (uint32_t)min(k, 2), (st > 0 || kb > 0 || k > 0) ? 1u : 0u);
+                                         tmem + kPScale + kScaleCols * (uint32_t)min(k, 2), (st > 0 || kb > 0 || k > 0) ? 1u : 0u);
                         }
                         tc_commit(smem_u32(&sh.empty[s]));
                     }

@@ -2890,9 +2890,10 @@ int mine_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt) {
         stt->setup_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_entry).count();
     } else {
         std::vector<TileDesc> tl;
+        bool top_wide = false;
         if (top_mode == 1) {
             if (top_i8) {
-                tiles_f4(0, n0, n0, W, sm_count, tl, true);
+                top_wide = tiles_f4(0, n0, n0, W, sm_count, tl, true);
             } else if (top_b1) {
                 const int64_t base = (int64_t)((n0 + kB1Rows - 1) / kB1Rows) * ((n0 + kB1Cols - 1) / kB1Cols);
                 const int64_t want = (int64_t)(tn.b1_tiles_per_sm * sm_count);
@@ -2933,7 +2934,7 @@ int mine_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt) {
         } else {
             a.tiles = top_b1 ? P.tiles_b1 : P.tiles_l3;
             a.n_tiles = (int32_t)tl.size();
-            TFIM_TRY(top_i8 ? launch_count_f4(a, s) : top_b1 ? launch_count_b1(a, s) : launch_count_lop3(a, s));
+            TFIM_TRY(top_i8 ? launch_count_f4(a, top_wide, s) : top_b1 ? launch_count_b1(a, s) : launch_count_lop3(a, s));
             bytes_alg += row_bytes * 2 * n0 + 4 * top_out;
         }
         TFIM_CUDA(cudaEventRecord(c->ev1, s));

@@ -45,6 +45,18 @@ __device__ __forceinline__ void mma_mxf4(uint32_t tmem_d, uint64_t da, uint64_t 
         "l"(da), "l"(db), "r"(idesc), "r"(sf), "r"(accumulate));
 }
 
+// The same with the A operand in tensor memory: lane = row, a 32-bit cell holds eight values.
+__device__ __forceinline__ void mma_mxf4_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t sf,
+                                            uint32_t accumulate) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        "setp.ne.b32 p, %5, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::mxf4.block_scale.scale_vec::2X [%0], [%1], %2, %3, [%4], [%4], p;\n\t"
+        "}\n" ::"r"(tmem_d),
+        "r"(tmem_a), "l"(db), "r"(idesc), "r"(sf), "r"(accumulate));
+}
+
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
@@ -74,13 +86,21 @@ __device__ __forceinline__ void tc_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
-// One value into 32 columns of this warp's 32 lanes.
-__device__ __forceinline__ void tmem_fill32(uint32_t taddr, uint32_t v) {
+// One value into 16 columns of this warp's 32 lanes.
+__device__ __forceinline__ void tmem_fill16(uint32_t taddr, uint32_t v) {
     asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {"
-        "%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, "
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {"
         "%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1};" ::"r"(taddr),
         "r"(v)
+        : "memory");
+}
+// 16 columns of this warp's 32 lanes.
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {"
+        "%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
+        "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
+        "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
         : "memory");
 }
 
@@ -99,12 +119,13 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
 }
 
 
-// The three scale regions, 32 columns each, of this warp's 32 lanes: every byte 2, 1 and 1/2
+// The three scale regions, kScaleCols columns each, of this warp's 32 lanes: every byte 2, 1 and 1/2
 // (UE8M0), so that the regions do not depend on the scale factors' layout.
+constexpr uint32_t kScaleCols = 16;
 __device__ __forceinline__ void tmem_fill_scales(uint32_t lanes) {
-    tmem_fill32(lanes, 0x80808080u);
-    tmem_fill32(lanes + 32, 0x7F7F7F7Fu);
-    tmem_fill32(lanes + 64, 0x7E7E7E7Eu);
+    tmem_fill16(lanes, 0x80808080u);
+    tmem_fill16(lanes + kScaleCols, 0x7F7F7F7Fu);
+    tmem_fill16(lanes + 2 * kScaleCols, 0x7E7E7E7Eu);
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 

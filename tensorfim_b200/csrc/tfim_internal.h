@@ -194,11 +194,11 @@ int configure_count_kernels();
 // an mbarrier wait expired is copied to pinned memory in stream order and checked (and
 // cleared) once the stream has been waited for anyway.
 constexpr int kF4Cols = 128, kF4Rows = 256;
-int launch_count_f4(const CountArgs& a, cudaStream_t s);
+int launch_count_f4(const CountArgs& a, bool wide, cudaStream_t s);   // wide: what tiles_f4 returned
 int count_f4_status_fetch(int32_t* pinned, cudaStream_t s);
 int count_f4_flag(const int32_t** flag);   // the flag's address on the current device
 int count_f4_status_check(int32_t v);
-void tiles_f4(int32_t job, int32_t nr, int32_t nc, int64_t W, int sms, std::vector<TileDesc>& out, bool upper = false);
+bool tiles_f4(int32_t job, int32_t nr, int32_t nc, int64_t W, int sms, std::vector<TileDesc>& out, bool upper = false);
 // Packed tcgen05 kind::mxf4 family counter (count_pk.cu): a tile holds the X rows of `nr` jobs of at
 // most kPkMaxCols columns, CountArgs::pk_list[job .. job + nr), of a class of c0 jobs per tile, over
 // a word slice of at most 2^18 words (its jobs may have fewer).  The persistent form reads its
