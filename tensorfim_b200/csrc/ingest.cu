@@ -116,6 +116,80 @@ __global__ void k_hist_sum(const int32_t* __restrict__ partial, int32_t parts, i
     freq[i] = v;
 }
 
+// Dense ids from the F1 histogram, one block: survivors (count >= min_count) of the ids 1..bins-1 in
+// ascending order, then id 0 if it survives; map[id] = dense id or -1.  On the host the same loops
+// over 40,000 ids and the two stable sorts below took 0.45 ms of a 300,000-row open.
+struct DenseCounts {
+    int32_t n_surv, n_dense, dimension, roots;
+};
+__global__ void __launch_bounds__(1024) k_dense_ids(const int32_t* __restrict__ freq, int32_t bins, int32_t min_count,
+                                                    int32_t root_min, int32_t* __restrict__ map,
+                                                    int32_t* __restrict__ dense_to_orig, int32_t* __restrict__ dense_freq,
+                                                    DenseCounts* out) {
+    typedef cub::BlockScan<int32_t, 1024> Scan;
+    __shared__ typename Scan::TempStorage ts;
+    __shared__ int32_t s_dim, s_roots;
+    if (threadIdx.x == 0) s_dim = s_roots = 0;
+    __syncthreads();
+    int32_t base = 0;
+    for (int64_t i0 = 0; i0 < bins; i0 += 4096) {
+        int32_t f[4], on[4], at[4], total = 0, dim = 0, roots = 0;
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int64_t i = i0 + threadIdx.x * 4 + q;
+            f[q] = i < bins ? freq[i] : 0;
+            on[q] = i > 0 && i < bins && f[q] >= min_count;
+            dim += f[q] != 0;
+            roots += i < bins && f[q] >= root_min;
+        }
+        Scan(ts).ExclusiveSum(on, at, total);
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int64_t i = i0 + threadIdx.x * 4 + q;
+            if (i >= bins) break;
+            map[i] = on[q] ? base + at[q] : -1;
+            if (on[q]) {
+                dense_to_orig[base + at[q]] = (int32_t)i;
+                dense_freq[base + at[q]] = f[q];
+            }
+        }
+        if (dim) atomicAdd(&s_dim, dim);
+        if (roots) atomicAdd(&s_roots, roots);
+        base += total;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        int32_t n = base;
+        if (freq[0] >= min_count) {   // the parked id 0
+            map[0] = n;
+            dense_to_orig[n] = 0;
+            dense_freq[n] = freq[0];
+            n++;
+        }
+        *out = DenseCounts{base, n, s_dim, s_roots};
+    }
+}
+
+// A stable order by rank: order[rank of i] = i, larger values first (or smaller first).  A block
+// ranks 256 items against all of them; n^2 comparisons, 38M for 6,156 items.
+__global__ void __launch_bounds__(256) k_rank_order(const int32_t* __restrict__ value, int32_t n, int descending,
+                                                    int32_t* __restrict__ order) {
+    __shared__ int32_t tile[1024];
+    const int32_t i = blockIdx.x * 256 + threadIdx.x;
+    const int32_t flip = descending ? -1 : 0;   // ~v reverses the order
+    const int32_t v = i < n ? value[i] ^ flip : 0;
+    int32_t rank = 0;
+    for (int32_t j0 = 0; j0 < n; j0 += 1024) {
+        __syncthreads();
+        for (int k = threadIdx.x; k < 1024; k += 256) tile[k] = j0 + k < n ? value[j0 + k] ^ flip : INT_MAX;
+        __syncthreads();
+        const int m = min(1024, n - j0);
+        for (int k = 0; k < m; k++) rank += tile[k] < v || (tile[k] == v && j0 + k < i);
+    }
+    if (i < n) order[rank] = i;
+}
+constexpr int32_t kRankMax = 1 << 15;   // beyond, the quadratic pass loses to the host's sort
+
 // Row passes over the transaction list give a row to eight lanes: its ids come in 32-byte
 // pieces, four rows per warp load, whether rows hold ten ids or a hundred (a thread per row read
 // 784,000 rows of 74 ids at 1.9 TB/s in the first pass and 0.7 TB/s in the second).
@@ -276,10 +350,19 @@ int compute_bit_supports(tfim_ctx* c) {
     const int32_t rows = c->from_db ? c->info.n_dense : c->n_counted;
     std::vector<int32_t> all(std::max<int32_t>(rows, 0), 0);
     if (rows > 0) {
-        TFIM_TRY(c->d_scratch[7].reserve((size_t)rows * 4));
+        TFIM_TRY(c->d_scratch[7].reserve((size_t)rows * 8));
         k_row_popc<<<rows, 256, 0, c->stream>>>(c->d_bitmap, c->W, rows, c->d_scratch[7].as<int32_t>());
         TFIM_CUDA(cudaGetLastError());
         TFIM_CUDA(cudaMemcpyAsync(all.data(), c->d_scratch[7].p, (size_t)rows * 4, cudaMemcpyDeviceToHost, c->stream));
+        // the counted rows in increasing support (the search's first family)
+        c->support_order.clear();
+        if (!c->sharded && c->n_counted > 0 && c->n_counted <= kRankMax) {
+            c->support_order.resize(c->n_counted);
+            int32_t* order = c->d_scratch[7].as<int32_t>() + rows;
+            k_rank_order<<<(c->n_counted + 255) / 256, 256, 0, c->stream>>>(c->d_scratch[7].as<int32_t>(), c->n_counted, 0, order);
+            TFIM_CUDA(cudaGetLastError());
+            TFIM_CUDA(cudaMemcpyAsync(c->support_order.data(), order, (size_t)c->n_counted * 4, cudaMemcpyDeviceToHost, c->stream));
+        }
         TFIM_CUDA(cudaStreamSynchronize(c->stream));
     }
     int64_t total = 0;
@@ -330,7 +413,6 @@ int ingest_device_csr(tfim_ctx* c, const int64_t* d_off_p, const int32_t* d_item
     for (DevBuf* b : {&d_stats, &d_freq, &d_map, &d_flag, &d_idx, &d_tmp}) b->stream = s;
     int rc = TFIM_OK;
     ScanStats hs{};
-    std::vector<int32_t> freq;
     int64_t id_max = 0, id_min = INT_MAX;
     // all device scratch below is released at the end of this function
     auto done = [&](int r) {
@@ -345,7 +427,7 @@ int ingest_device_csr(tfim_ctx* c, const int64_t* d_off_p, const int32_t* d_item
     if (n_rows > 0) k_row_lengths<<<grid_for(n_rows), 256, 0, s>>>(d_off_p, n_rows, d_stats.as<ScanStats>());
     cudaMemcpyAsync(&hs, d_stats.p, sizeof hs, cudaMemcpyDeviceToHost, s);
     if (cudaStreamSynchronize(s) != cudaSuccess) { set_error("ingest statistics pass failed: %s", cudaGetErrorString(cudaGetLastError())); return done(TFIM_E_CUDA); }
-    int64_t n_rows_all = n_rows;
+    int64_t n_rows_all = n_rows, nnz_all = nnz;
     if (c->sharded) {
         // the whole database's statistics: errors, id range and row lengths (MIN as -MAX(-x))
         int64_t mx[6] = {hs.neg, hs.bad_off, nnz > 0 ? (int64_t)hs.id_max : -1, n_rows > 0 ? (int64_t)hs.len_max : 0,
@@ -355,6 +437,7 @@ int ingest_device_csr(tfim_ctx* c, const int64_t* d_off_p, const int32_t* d_item
         hs.neg = (int32_t)mx[0];
         hs.bad_off = (int32_t)mx[1];
         n_rows_all = sm[0];
+        nnz_all = sm[2];
         hs.len_sum = (unsigned long long)sm[1];
         if (sm[2] > 0) { id_max = mx[2]; id_min = -mx[4]; }
         hs.len_max = mx[3];
@@ -388,8 +471,31 @@ int ingest_device_csr(tfim_ctx* c, const int64_t* d_off_p, const int32_t* d_item
         }
     }
     if ((rc = group_reduce(c, d_freq.p, id_max + 1, TFIM_DT_I32, TFIM_RED_SUM, s))) return done(rc);
-    freq.assign((size_t)id_max + 1, 0);
-    cudaMemcpyAsync(freq.data(), d_freq.p, (size_t)(id_max + 1) * 4, cudaMemcpyDeviceToHost, s);
+    const int32_t bins = (int32_t)(id_max + 1);
+    const double fthr = (double)n_rows_all * thr;             // kernel_bitmap.cu:806
+    const int32_t min_count = (int32_t)std::max(0.0, std::ceil(fthr));   // v >= fthr  <=>  v >= ceil(fthr) for integer v
+    // the smallest count v with v / rows > thr (kernel_bitmap.cu:815-816), the quotient rounded as there
+    int32_t root_min = INT_MAX;
+    if (n_rows_all > 0) {
+        int64_t lo = 0, hi = INT_MAX;
+        while (lo < hi) {
+            const int64_t mid = (lo + hi) / 2;
+            if ((double)mid / (double)n_rows_all > thr) hi = mid; else lo = mid + 1;
+        }
+        root_min = (int32_t)lo;
+    }
+    // map, then dense_to_orig, dense_freq and the frequency order, then the counts
+    // (an id survives with at least min_count of the nnz_all occurrences)
+    const size_t tab = ((size_t)bins + 3) & ~size_t(3);
+    const size_t cap = (std::min<size_t>(bins, (size_t)(nnz_all / std::max(min_count, 1)) + 1) + 4) & ~size_t(3);
+    if ((rc = d_map.reserve((tab + 3 * cap) * 4 + sizeof(DenseCounts)))) return done(rc);
+    int32_t* t_orig = d_map.as<int32_t>() + tab;
+    int32_t* t_freq = t_orig + cap;
+    int32_t* t_order = t_freq + cap;
+    DenseCounts* t_counts = (DenseCounts*)(t_order + cap);
+    k_dense_ids<<<1, 1024, 0, s>>>(d_freq.as<int32_t>(), bins, min_count, root_min, d_map.as<int32_t>(), t_orig, t_freq, t_counts);
+    DenseCounts dc{};
+    cudaMemcpyAsync(&dc, t_counts, sizeof dc, cudaMemcpyDeviceToHost, s);
     if (cudaStreamSynchronize(s) != cudaSuccess) { set_error("F1 histogram failed: %s", cudaGetErrorString(cudaGetLastError())); return done(TFIM_E_CUDA); }
 
     tfim_db_info& I = c->info;
@@ -400,51 +506,36 @@ int ingest_device_csr(tfim_ctx* c, const int64_t* d_off_p, const int32_t* d_item
     I.trans_len_min = n_rows_all > 0 ? hs.len_min : INT_MAX;
     I.trans_len_max = n_rows_all > 0 ? hs.len_max : 0;
     I.trans_len_mean = n_rows_all > 0 ? (double)hs.len_sum / (double)n_rows_all : 0.0;
-    int64_t dim = 0;
-    for (int64_t i = 0; i <= id_max; i++) dim += freq[i] != 0;
-    I.dimension = dim;
+    I.dimension = dc.dimension;
     I.support_threshold = thr;
-    const double fthr = (double)n_rows_all * thr;             // kernel_bitmap.cu:806
     I.frequency_threshold = fthr;
-    I.min_count = (int32_t)std::max(0.0, std::ceil(fthr));     // v >= fthr  <=>  v >= ceil(fthr) for integer v
-    int64_t dimred = 0;
-    for (int64_t i = 0; i <= id_max; i++)                       // kernel_bitmap.cu:815-816
-        if ((double)freq[i] / (double)n_rows_all > thr) dimred++;
-    I.dimension_reduced = dimred;
+    I.min_count = min_count;
+    I.dimension_reduced = dc.roots;
 
-    // dense ids (kernel_bitmap.cu:348-373)
-    std::vector<int32_t> map((size_t)id_max + 1, -1);
-    c->dense_to_orig.clear();
-    c->dense_freq.clear();
-    for (int64_t i = 1; i <= id_max; i++)
-        if ((double)freq[i] >= fthr) {
-            map[i] = (int32_t)c->dense_to_orig.size();
-            c->dense_to_orig.push_back((int32_t)i);
-            c->dense_freq.push_back(freq[i]);
-        }
-    const int32_t n_surv = (int32_t)c->dense_to_orig.size();
-    if ((double)freq[0] >= fthr) {   // kernel_bitmap.cu:356 (true for an empty set: 0 >= 0.0)
-        map[0] = n_surv;
-        c->dense_to_orig.push_back(0);
-        c->dense_freq.push_back(freq[0]);
-    }
-    const int32_t n_dense = (int32_t)c->dense_to_orig.size();
+    // dense ids (kernel_bitmap.cu:348-373); a frequent id 0 is parked last (:356, true for an empty
+    // set: 0 >= 0.0)
+    const int32_t n_surv = dc.n_surv, n_dense = dc.n_dense;
     I.n_survivors = n_surv;
     I.n_dense = n_dense;
     I.item_id_max_dense = n_dense - 1;
     c->n_counted = n_surv;
-    c->items_in_freq_sort.resize(n_dense);
-    std::iota(c->items_in_freq_sort.begin(), c->items_in_freq_sort.end(), 0);
-    std::stable_sort(c->items_in_freq_sort.begin(), c->items_in_freq_sort.end(),
-                     [&](int a, int b) { return c->dense_freq[a] > c->dense_freq[b]; });
-    const int64_t n_roots = std::min<int64_t>(dimred, n_dense);
-    c->roots.assign(c->items_in_freq_sort.begin(), c->items_in_freq_sort.begin() + n_roots);
+    c->dense_to_orig.assign(n_dense, 0);
+    c->dense_freq.assign(n_dense, 0);
+    c->items_in_freq_sort.assign(n_dense, 0);
+    if (n_dense > 0) {
+        // (waited for with the row reduction below)
+        cudaMemcpyAsync(c->dense_to_orig.data(), t_orig, (size_t)n_dense * 4, cudaMemcpyDeviceToHost, s);
+        cudaMemcpyAsync(c->dense_freq.data(), t_freq, (size_t)n_dense * 4, cudaMemcpyDeviceToHost, s);
+        if (n_dense <= kRankMax) {
+            k_rank_order<<<(n_dense + 255) / 256, 256, 0, s>>>(t_freq, n_dense, 1, t_order);
+            cudaMemcpyAsync(c->items_in_freq_sort.data(), t_order, (size_t)n_dense * 4, cudaMemcpyDeviceToHost, s);
+        }
+    }
 
     // reduced rows, their numbering, and the reduced transaction list in dense ids
-    if ((rc = d_map.reserve((size_t)(id_max + 1) * 4)) || (rc = d_flag.reserve((size_t)std::max<int64_t>(n_rows, 1) * 4)) ||
+    if ((rc = d_flag.reserve((size_t)std::max<int64_t>(n_rows, 1) * 4)) ||
         (rc = d_idx.reserve((size_t)std::max<int64_t>(n_rows, 1) * 16)))
         return done(rc);
-    cudaMemcpyAsync(d_map.p, map.data(), (size_t)(id_max + 1) * 4, cudaMemcpyHostToDevice, s);
     int64_t n_red = 0, n_red_items = 0;
     int64_t* red_idx = d_idx.as<int64_t>();
     int64_t* item_off = red_idx + std::max<int64_t>(n_rows, 1);
@@ -468,7 +559,17 @@ int ingest_device_csr(tfim_ctx* c, const int64_t* d_off_p, const int32_t* d_item
         if (cudaStreamSynchronize(s) != cudaSuccess) { set_error("row reduction failed: %s", cudaGetErrorString(cudaGetLastError())); return done(TFIM_E_CUDA); }
         n_red = last[0] + (last_len > 0);
         n_red_items = last[1] + last_len;
+    } else if (cudaStreamSynchronize(s) != cudaSuccess) {
+        set_error("dense ids failed: %s", cudaGetErrorString(cudaGetLastError()));
+        return done(TFIM_E_CUDA);
     }
+    if (n_dense > kRankMax) {
+        std::iota(c->items_in_freq_sort.begin(), c->items_in_freq_sort.end(), 0);
+        std::stable_sort(c->items_in_freq_sort.begin(), c->items_in_freq_sort.end(),
+                         [&](int a, int b) { return c->dense_freq[a] > c->dense_freq[b]; });
+    }
+    const int64_t n_roots = std::min<int64_t>(dc.roots, n_dense);
+    c->roots.assign(c->items_in_freq_sort.begin(), c->items_in_freq_sort.begin() + n_roots);
     int64_t n_red_all = n_red;
     if (c->sharded) {
         int64_t mx[2] = {n_red > 0 ? (int64_t)hs.red_max : 0, n_red > 0 ? -(int64_t)hs.red_min : -(int64_t)LLONG_MAX};

@@ -2492,10 +2492,14 @@ int mine_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt) {
         for (int32_t r : c->roots) R.is_root_h[r] = 1;
         // top family: the counted items frequent by bitmap support, increasing support
         R.F0.clear();
-        for (int32_t e = 0; e < d; e++)
+        const bool ordered = (int32_t)c->support_order.size() == d;
+        for (int32_t k = 0; k < d; k++) {
+            const int32_t e = ordered ? c->support_order[k] : k;
             if (c->bit_support[e] >= minc) R.F0.push_back(e);
-        std::stable_sort(R.F0.begin(), R.F0.end(),
-                         [&](int32_t a, int32_t b) { return c->bit_support[a] < c->bit_support[b]; });
+        }
+        if (!ordered)
+            std::stable_sort(R.F0.begin(), R.F0.end(),
+                             [&](int32_t a, int32_t b) { return c->bit_support[a] < c->bit_support[b]; });
     }
     const std::vector<char>& is_root = R.is_root_h;
     const std::vector<int32_t>& F0 = R.F0;
