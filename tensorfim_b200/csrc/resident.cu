@@ -82,6 +82,7 @@ struct ResStatus {
     int32_t jobs, rows, tiles_l3, tiles_b1, n_proj, n_mjobs;   // n_mjobs: masks the last expand asked for
     int32_t pj_n, pj_rows;                   // families to project, their rows in all,
     int64_t pj_words;                        // and the words these take
+    int64_t pj_groups;                       // at most so many groups of 32 items hold their columns
     int64_t out_total;
     int32_t max_cols, max_head, starved, error;
     // grow: the wave the pack built does not fit the pools; nothing was consumed and the
@@ -192,6 +193,14 @@ struct ResPtrs {
     PJob* pjobs;
     int32_t* pj_off;              // per family to project: bits before each tile, tiles + 1 entries
     uint32_t* pj_pool;
+    // transactions as rows, for the projection: pj_chunks x N32 transactions x pj_gc words of 32 items
+    // (positions in the top family's order), and per family its column at each position (or -1) and
+    // the groups of each chunk with columns; null when the rows are compressed word by word
+    uint32_t* pj_tm;
+    int16_t* pj_inv;
+    uint32_t* pj_gbits;
+    int32_t* pj_pos;
+    int32_t pj_chunks, pj_gc;
     ResStatus* h_st;              // pinned copy of the status record, written by the host-driven packs
 };
 // The dense item id of an F list entry.
@@ -1595,23 +1604,33 @@ __global__ void __launch_bounds__(256) k_top_finish(int32_t* __restrict__ M, int
 // these are at most half of the database, the family is moved to a universe of its own: the
 // rows of its F list are compressed to the set bits of t's row (bit k of a compressed row = the
 // k-th transaction of t), and the family and all its descendants count there with an all-ones
-// base, over sup(t) instead of N transactions.  Supports do not change.  AND + popc costs about
-// 8 issue slots per word and pair (popc runs at 16 lanes per SM and clock), the compression
-// about 25 per word and row once, so it pays from a few tail rows on.
+// base, over sup(t) instead of N transactions.  Supports do not change.  It pays from a few tail
+// rows on: a family reads its rows again for every one of them.
 // Measured on the 6.3M-row dense database (267 items, minsup 6%): counting of the later waves
-// 62 -> 25 ms, masks 1.8 -> 0.6 ms, compression 5.7 ms; the mine 64.8 -> 33.0 ms.
+// 62 -> 25 ms, masks 1.8 -> 0.6 ms, compression 2.4 ms; the mine 64.8 -> 29.7 ms.  Lines at
+// 3/4 and 19/20 of N instead of 1/2 moved the mine by less than its noise, as did 2 tail rows.
 constexpr int kProjMinTail = 4;        // tail rows from which a family is projected
-constexpr int kProjTile = 1024;        // words of a row per block
-constexpr int kProjThreads = kProjTile / 8;
-constexpr int kProjCols = 4;           // rows compressed between two barriers
+constexpr int kProjTile = 64;          // words of a row per tile; rows are padded to this
+constexpr int kProjGroups = 13;        // most groups of 32 items in a transposed chunk (odd)
+constexpr int kProjWarps = 20;
+constexpr int kProjWords = 1024;       // word by word: words of a row per block,
+constexpr int kProjWordTiles = kProjWords / kProjTile;
+constexpr int kProjThreads = kProjWords / 8;
+constexpr int kProjCols = 4;           // and rows compressed between two barriers
+// Columns per group of 32 items from which rows are compressed by transposing.  Its cost is per
+// group with columns, the word-by-word way's per column: 2.2 and 5.6 ms at 21 columns a group (the
+// 6.3M-row dense database), so they meet near 8.  The number of groups is only bounded here,
+// by all groups or one per column (7 columns a group by that bound there), hence the lower line.
+constexpr int kProjMinCols = 6;
 
 // One block: the children of the empty prefix worth projecting, their places in the row table
 // and the pool.
 __global__ void __launch_bounds__(kPackThreads) k_proj_plan(ResPtrs p) {
-    __shared__ int64_t sm64[3 * 33];
+    __shared__ int64_t sm64[4 * 33];
     const int tid = threadIdx.x;
     const int32_t n_fam = p.st->fam_n;
-    int64_t cnt = 0, rows = 0, words = 0;
+    int64_t cnt = 0, rows = 0, words = 0, groups = 0;
+    const int32_t n_groups = (p.fams[0].nF + 31) / 32;
     for (int32_t base = 1; base < n_fam; base += kPackThreads) {
         const int32_t fid = base + tid;
         DFam f{};
@@ -1622,49 +1641,50 @@ __global__ void __launch_bounds__(kPackThreads) k_proj_plan(ResPtrs p) {
                  64 * (int64_t)f.sup >= f.n;
         }
         const int64_t Wp = ((int64_t)f.sup + 2047) / 2048 * 64;
-        int64_t v[3] = {on ? 1 : 0, on ? f.nF : 0, on ? f.nF * Wp : 0}, ex[3], tot[3];
-        block_scan<3>(v, ex, tot, sm64, true);
+        int64_t v[4] = {on ? 1 : 0, on ? f.nF : 0, on ? f.nF * Wp : 0, on ? min(f.nF, n_groups) : 0}, ex[4], tot[4];
+        block_scan<4>(v, ex, tot, sm64, true);
         if (on)
             p.pjobs[cnt + ex[0]] =
                 PJob{fid, f.item, f.F_off, f.nF, (int32_t)Wp, (int32_t)(rows + ex[1]), f.sup, 0, words + ex[2]};
         cnt += tot[0];
         rows += tot[1];
         words += tot[2];
+        groups += tot[3];
     }
     if (tid == 0) {
+        p.st->pj_groups = groups;
         p.st->pj_n = (int32_t)cnt;
         p.st->pj_rows = (int32_t)rows;
         p.st->pj_words = words;
     }
 }
 
-__host__ __device__ __forceinline__ int64_t proj_tiles(int64_t W) { return (W + kProjTile - 1) / kProjTile; }
-
-// Set bits of every tile of every base row: one warp per (family, tile).
+// Set bits of every tile of every base row: half a warp per (family, tile).  Also the positions
+// of the top family's items.
 __global__ void __launch_bounds__(256) k_proj_count(ResPtrs p, int32_t n_pj) {
-    const int64_t nt = proj_tiles(p.W), W4 = p.W >> 2;
+    const int64_t nt = p.W / kProjTile;
     const int lane = threadIdx.x & 31;
-    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t u = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; u < n_pj * nt; u += warps) {
-        const int64_t k = u / nt, tile = u % nt;
+    if (p.pj_pos)
+        for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < p.fams[0].nF; i += gridDim.x * blockDim.x)
+            p.pj_pos[p.items[p.fams[0].F_off + i]] = i;
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5), half = (nt + 1) / 2;
+    for (int64_t u = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; u < n_pj * half; u += warps) {
+        const int64_t k = u / half, tile = 2 * (u % half) + (lane >> 4);
         const uint4* row = reinterpret_cast<const uint4*>(row_of(p, p.pjobs[k].item));
         int32_t n = 0;
-#pragma unroll
-        for (int q = 0; q < kProjTile / 128; q++) {
-            const int64_t w = tile * (kProjTile / 4) + q * 32 + lane;
-            if (w < W4) {
-                const uint4 x = __ldg(row + w);
-                n += __popc(x.x) + __popc(x.y) + __popc(x.z) + __popc(x.w);
-            }
+        if (tile < nt) {
+            const uint4 x = __ldg(row + tile * (kProjTile / 4) + (lane & 15));
+            n = __popc(x.x) + __popc(x.y) + __popc(x.z) + __popc(x.w);
         }
-        n = __reduce_add_sync(0xffffffffu, n);
-        if (lane == 0) p.pj_off[k * (nt + 1) + tile + 1] = n;
+#pragma unroll
+        for (int o = 8; o; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
+        if ((lane & 15) == 0 && tile < nt) p.pj_off[k * (nt + 1) + tile + 1] = n;
     }
 }
 
 // Bits before each tile: one warp per family.
 __global__ void __launch_bounds__(256) k_proj_scan(ResPtrs p, int32_t n_pj) {
-    const int64_t nt = proj_tiles(p.W);
+    const int64_t nt = p.W / kProjTile;
     const int lane = threadIdx.x & 31;
     const int64_t k = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     if (k >= n_pj) return;
@@ -1685,11 +1705,11 @@ __global__ void __launch_bounds__(256) k_proj_scan(ResPtrs p, int32_t n_pj) {
     if (lane == 0 && sum != p.pjobs[k].sup) atomicExch(&p.st->error, 2);
 }
 
-// The row table's entries, and zeros in the words that two tiles share and in the padding: one
-// block per family.
+// The row table's entries, zeros in the padding, and what the chosen way of compressing needs: the
+// family's columns by position, or zeros in the words that two tiles share.  One block per family.
 __global__ void __launch_bounds__(256) k_proj_init(ResPtrs p) {
     const PJob q = p.pjobs[blockIdx.x];
-    const int64_t nt = proj_tiles(p.W);
+    const int64_t nt = p.W / kProjTile;
     const int32_t* off = p.pj_off + (int64_t)blockIdx.x * (nt + 1);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int c = warp; c < q.nF; c += blockDim.x >> 5) {
@@ -1698,32 +1718,216 @@ __global__ void __launch_bounds__(256) k_proj_init(ResPtrs p) {
             p.vrows[q.row0 + c] = dst;
             p.vitem[q.row0 + c] = p.items[q.F_off + c];
         }
-        for (int64_t t = lane; t < nt; t += 32) {
-            const int32_t w = off[t] >> 5;
-            if (w < q.Wp) dst[w] = 0;
-        }
+        if (!p.pj_tm)
+            for (int64_t t = lane; t * kProjWordTiles < nt; t += 32) {
+                const int32_t w = off[t * kProjWordTiles] >> 5;
+                if (w < q.Wp) dst[w] = 0;
+            }
         for (int32_t w = (q.sup >> 5) + lane; w < q.Wp; w += 32) dst[w] = 0;
+    }
+    if (!p.pj_tm) return;
+    const int32_t n_g = p.pj_chunks * p.pj_gc;
+    int16_t* inv = p.pj_inv + (int64_t)blockIdx.x * n_g * 32;
+    for (int32_t i = threadIdx.x; i < n_g * 32; i += blockDim.x) inv[i] = -1;
+    __syncthreads();
+    for (int32_t c = threadIdx.x; c < q.nF; c += blockDim.x) inv[p.pj_pos[p.items[q.F_off + c]]] = (int16_t)c;
+    __syncthreads();
+    for (int32_t h = warp; h < p.pj_chunks; h += blockDim.x >> 5) {
+        uint32_t m = 0;
+        for (int32_t g = 0; g < p.pj_gc; g++) m |= (uint32_t)__any_sync(0xffffffffu, inv[(h * p.pj_gc + g) * 32 + lane] >= 0) << g;
+        if (lane == 0) p.pj_gbits[(int64_t)blockIdx.x * p.pj_chunks + h] = m;
     }
 }
 
-// Compresses the rows of one (family, tile) per block.  A thread owns 8 words of the tile and
+// Transposes a 32 x 32 bit matrix in registers: bit i of v[j] becomes bit j of v[i].
+__device__ __forceinline__ void transpose32(uint32_t (&v)[32]) {
+#pragma unroll
+    for (int k = 0; k < 16; k++) {
+        const uint32_t x = v[k], y = v[k + 16];
+        v[k] = __byte_perm(x, y, 0x5410);
+        v[k + 16] = __byte_perm(x, y, 0x7632);
+    }
+#pragma unroll
+    for (int k = 0; k < 32; k++)
+        if (!(k & 8)) {
+            const uint32_t x = v[k], y = v[k + 8];
+            v[k] = __byte_perm(x, y, 0x6240);
+            v[k + 8] = __byte_perm(x, y, 0x7351);
+        }
+#pragma unroll
+    for (int e = 2; e >= 0; e--) {
+        const int sh = 1 << e;
+        const uint32_t m = sh == 4 ? 0x0f0f0f0fu : sh == 2 ? 0x33333333u : 0x55555555u;
+#pragma unroll
+        for (int k = 0; k < 32; k++)
+            if (!(k & sh)) {
+                const uint32_t x = v[k], y = v[k + sh];
+                v[k] = (x & m) | ((y << sh) & ~m);
+                v[k + sh] = ((x >> sh) & m) | (y & ~m);
+            }
+    }
+}
+
+// The database with its transactions as rows: one block per 1,024 transactions and chunk of item
+// groups, a warp per group.
+__global__ void __launch_bounds__(32 * kProjGroups) k_proj_tm(ResPtrs p) {
+    extern __shared__ uint32_t tm_out[];   // [1024][gc], one word of padding per 32 transactions
+    const int gc = p.pj_gc, h = blockIdx.y, lane = threadIdx.x & 31, g = threadIdx.x >> 5;
+    const int64_t w0 = (int64_t)blockIdx.x * 32;
+    const int32_t n0 = p.fams[0].nF, at = (h * gc + g) * 32;
+    const int32_t* F = p.items + p.fams[0].F_off;
+    uint32_t v[32];
+#pragma unroll
+    for (int j = 0; j < 32; j++) v[j] = at + j < n0 ? __ldg(row_of(p, F[at + j]) + w0 + lane) : 0;
+    transpose32(v);
+#pragma unroll
+    for (int j = 0; j < 32; j++) tm_out[(32 * lane + j) * gc + g + lane] = v[j];
+    __syncthreads();
+    uint32_t* dst = p.pj_tm + ((int64_t)h * p.W + w0) * 32 * gc;
+    for (int i = threadIdx.x; i < 1024 * gc; i += blockDim.x) dst[i] = tm_out[i + i / (32 * gc)];
+}
+
+// Compresses families' rows a tile of 2,048 transactions at a time.  The tile's transactions lie in
+// shared memory as rows of item bits; a warp lists a family's transactions of the tile, and a
+// thread picks the 32 of one compressed word, transposes their 32 x 32 bits in registers and stores
+// the words of the group's columns.  Work is per word written, not per word read: about 500
+// instructions for 32 words of up to 32 columns.  A tile writes the words whose first bit is its own; the
+// up to 31 transactions that the last one lacks are fetched from the tiles behind.  Odd row lengths
+// spread the gathered words over the banks.  Bound by latency: 20 warps an SM (what the staged rows
+// leave room for), each with a chain of loads, list and gathers per family.
+// Measured on the 6.3M-row dense database (267 items, minsup 6%): 2.1 ms and 0.14 ms for the
+// transposed copy, against 5.6 ms word by word (k_proj_words).
+__global__ void __launch_bounds__(32 * kProjWarps, 1) k_proj_rows(ResPtrs p, int32_t n_pj, int32_t parts) {
+    extern __shared__ __align__(16) uint32_t pr_smem[];
+    const int gc = p.pj_gc, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t nt = p.W / kProjTile;
+    constexpr int T = kProjTile * 32, kZero = T + 32 * kProjWarps;   // staged rows: the tile, each warp's 32, a zero row
+    uint32_t* rows = pr_smem;
+    uint16_t* list = reinterpret_cast<uint16_t*>(pr_smem + (((kZero + 1) * gc + 3) & ~3)) + warp * (T + 32);
+    for (int i = threadIdx.x; i < gc; i += blockDim.x) rows[kZero * gc + i] = 0;
+    for (int64_t u = blockIdx.x; u < nt * p.pj_chunks * parts; u += gridDim.x) {
+        const int part = (int)(u % parts), h = (int)(u / parts % p.pj_chunks);
+        const int64_t tile = u / parts / p.pj_chunks;
+        const uint32_t* tm = p.pj_tm + (int64_t)h * p.W * 32 * gc;
+        __syncthreads();
+        {
+            const uint4* src = reinterpret_cast<const uint4*>(tm + tile * T * gc);
+            for (int i = threadIdx.x; i < T / 4 * gc; i += blockDim.x) reinterpret_cast<uint4*>(rows)[i] = __ldg(src + i);
+        }
+        __syncthreads();
+        for (int32_t k = part + parts * warp; k < n_pj; k += parts * kProjWarps) {
+            const uint32_t gbits = p.pj_gbits[(int64_t)k * p.pj_chunks + h];
+            if (!gbits) continue;
+            const PJob q = p.pjobs[k];
+            const int32_t off0 = p.pj_off[(int64_t)k * (nt + 1) + tile], off1 = p.pj_off[(int64_t)k * (nt + 1) + tile + 1];
+            const int32_t wa = (off0 + 31) >> 5, n_w = min((off1 + 31) >> 5, q.Wp) - wa;
+            if (n_w <= 0) continue;
+            const uint32_t* base = row_of(p, q.item);
+            // the family's transactions, as offsets into `rows`, from list[off0 % 32] on
+            const int32_t lead = off0 & 31;
+            const uint2 m2 = __ldg(reinterpret_cast<const uint2*>(base + tile * kProjTile) + lane);
+            int32_t n = __popc(m2.x) + __popc(m2.y), pre = n;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int32_t y = __shfl_up_sync(0xffffffffu, pre, o);
+                if (lane >= o) pre += y;
+            }
+            pre += lead - n;
+            for (uint32_t m = m2.x; m; m &= m - 1) list[pre++] = (uint16_t)((64 * lane + __ffs(m) - 1) * gc);
+            for (uint32_t m = m2.y; m; m &= m - 1) list[pre++] = (uint16_t)((64 * lane + 31 + __ffs(m)) * gc);
+            const int32_t end = lead + off1 - off0;                       // list entries used
+            const int32_t need = min(32 * (wa + n_w), q.sup) - off1;      // transactions to fetch from behind
+            for (int32_t i = lane; end + i < 32 * ((end + 31) >> 5); i += 32)
+                list[end + i] = (uint16_t)((i < need ? T + 32 * warp + i : kZero) * gc);
+            uint32_t* far = rows + (T + 32 * warp) * gc;   // the fetched transactions' rows
+            int32_t got = 0;
+            for (int64_t w = (tile + 1) * kProjTile; got < need && w < p.W; w += 32) {   // W is a multiple of 64
+                uint32_t m = __ldg(base + w + lane);
+                const int32_t c = __popc(m);
+                int32_t at = c;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int32_t y = __shfl_up_sync(0xffffffffu, at, o);
+                    if (lane >= o) at += y;
+                }
+                const int32_t all = __shfl_sync(0xffffffffu, at, 31);
+                at += got - c;
+                for (; m && at < need; m &= m - 1, at++) far[at] = (uint32_t)(32 * (w + lane) + __ffs(m) - 1);
+                got += all;
+            }
+            if (need > 0) {
+                __syncwarp();
+                const uint32_t t = lane < min(need, got) ? far[lane] : 0;
+                __syncwarp();
+#pragma unroll 4
+                for (int i = 0; i < need * gc; i += 32) {
+                    const int e = min((i + lane) / gc, 31);
+                    const int64_t te = __shfl_sync(0xffffffffu, t, e);
+                    if (i + lane < need * gc) far[i + lane] = __ldg(tm + te * gc + (i + lane - e * gc));
+                }
+            }
+            __syncwarp();
+            const int32_t total = __popc(gbits) * n_w;
+            const int32_t first = 32 * (wa - (off0 >> 5));                // list entry of word wa's first bit
+            for (int32_t e = lane; e < total; e += 32) {
+                const int32_t gi = e / n_w, w = e - gi * n_w;
+                uint32_t gm = gbits;
+                for (int i = 0; i < gi; i++) gm &= gm - 1;
+                const int g = __ffs(gm) - 1;
+                const uint4* idx = reinterpret_cast<const uint4*>(list + first + 32 * w);
+                const uint32_t* src = rows + g;
+                uint32_t v[32];
+#pragma unroll
+                for (int t = 0; t < 4; t++) {
+                    const uint4 x = idx[t];
+                    v[8 * t] = src[x.x & 0xffffu];
+                    v[8 * t + 1] = src[x.x >> 16];
+                    v[8 * t + 2] = src[x.y & 0xffffu];
+                    v[8 * t + 3] = src[x.y >> 16];
+                    v[8 * t + 4] = src[x.z & 0xffffu];
+                    v[8 * t + 5] = src[x.z >> 16];
+                    v[8 * t + 6] = src[x.w & 0xffffu];
+                    v[8 * t + 7] = src[x.w >> 16];
+                }
+                transpose32(v);
+                const uint4* cols = reinterpret_cast<const uint4*>(p.pj_inv + ((int64_t)k * p.pj_chunks * gc + h * gc + g) * 32);
+                uint32_t* dst = p.pj_pool + q.woff + wa + w;
+#pragma unroll
+                for (int t = 0; t < 4; t++) {
+                    const uint4 x = __ldg(cols + t);
+                    const uint32_t c4[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+                    for (int i = 0; i < 8; i++) {
+                        const int32_t c = (int16_t)(c4[i >> 1] >> (16 * (i & 1)));
+                        if (c >= 0) dst[(int64_t)c * q.Wp] = v[8 * t + i];
+                    }
+                }
+            }
+            __syncwarp();
+        }
+    }
+}
+
+// The same word by word, for families whose few columns are spread over many items: the rows of
+// one (family, kProjWords words) per block.  A thread owns 8 words of the tile and
 // keeps their five move masks (the parallel-suffix compress of H. S. Warren, Hacker's Delight,
 // 7-4) in registers for all rows; per row it loads its 32 bytes, compresses each word and
 // appends it to a bit run that it flushes word by word into the row's shared output, which
 // then goes out whole.  Tiles of all families at one place run together, so that the database's
 // rows are read from L2.
-__global__ void __launch_bounds__(kProjThreads, 4) k_proj_rows(ResPtrs p, int32_t n_pj) {
-    __shared__ uint32_t out[kProjCols][kProjTile + 2];
+__global__ void __launch_bounds__(kProjThreads, 4) k_proj_words(ResPtrs p, int32_t n_pj) {
+    __shared__ uint32_t out[kProjCols][kProjWords + 2];
     __shared__ int32_t s_warp[kProjThreads / 32];
-    const int64_t nt = proj_tiles(p.W);
+    const int64_t nt = p.W / kProjTile, nw = (nt + kProjWordTiles - 1) / kProjWordTiles;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (int i = tid; i < kProjCols * (kProjTile + 2); i += kProjThreads) (&out[0][0])[i] = 0;
-    for (int64_t u = blockIdx.x; u < n_pj * nt; u += gridDim.x) {
+    for (int i = tid; i < kProjCols * (kProjWords + 2); i += kProjThreads) (&out[0][0])[i] = 0;
+    for (int64_t u = blockIdx.x; u < n_pj * nw; u += gridDim.x) {
         const int64_t tile = u / n_pj, k = u % n_pj;
         const PJob q = p.pjobs[k];
-        const int32_t t0 = p.pj_off[k * (nt + 1) + tile], bits = p.pj_off[k * (nt + 1) + tile + 1] - t0;
+        const int32_t* off = p.pj_off + k * (nt + 1);
+        const int32_t t0 = off[tile * kProjWordTiles], bits = off[min((tile + 1) * kProjWordTiles, nt)] - t0;
         if (bits == 0) continue;
-        const int64_t w4 = tile * (kProjTile / 4) + tid * 2;   // this thread's words, 16 bytes each
+        const int64_t w4 = tile * (kProjWords / 4) + tid * 2;   // this thread's words, 16 bytes each
         const bool in = w4 * 4 < p.W;                          // W is a multiple of 64 words
         uint32_t m[8], mv[8][5];
         int32_t n_of[8], n_all = 0;
@@ -2842,7 +3046,8 @@ int mine_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt) {
     };
 
     auto project_families = [&]() -> int {
-        const int64_t nt = proj_tiles(W);
+        const int64_t nt = W / kProjTile;
+        P.pj_tm = nullptr;
         TFIM_TRY(grow(R.pjobs, (size_t)(n0 + 1) * sizeof(PJob), s));
         refresh_ptrs();
         k_proj_plan<<<1, kPackThreads, 0, s>>>(P);
@@ -2862,28 +3067,60 @@ int mine_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt) {
             TFIM_CUDA(cudaMemGetInfo(&mem_free, &mem_total));
             total.store(mem_total);
         }
-        if ((size_t)words * 4 > total.load() / 8) return TFIM_OK;
-        if ((size_t)words * 4 > R.pj_pool.bytes) {   // its old contents are not needed
+        const size_t room = total.load() / 8, row_bytes = (size_t)words * 4;
+        if (row_bytes > room) return TFIM_OK;
+        // groups of 32 items, in chunks that shared memory holds; an odd number per chunk
+        const int32_t groups = (n0 + 31) / 32;
+        P.pj_chunks = (groups + kProjGroups - 1) / kProjGroups;
+        P.pj_gc = ((groups + P.pj_chunks - 1) / P.pj_chunks) | 1;
+        const int64_t n_g = (int64_t)P.pj_chunks * P.pj_gc;
+        const size_t tm_bytes = (size_t)n_g * W * 128, inv_bytes = (size_t)n_pj * n_g * 64,
+                     gb_bytes = (size_t)n_pj * P.pj_chunks * 4, extra = tm_bytes + inv_bytes + gb_bytes + (size_t)P.n_base * 4;
+        const bool by_row = n_rows >= kProjMinCols * hst->pj_groups && n0 <= 32767 && row_bytes + extra <= room;
+        const size_t bytes = row_bytes + (by_row ? extra : 0);
+        if (bytes > R.pj_pool.bytes) {   // its old contents are not needed
             dev_free(R.pj_pool.p, s);
             R.pj_pool = Pool{};
-            if (dev_alloc(&R.pj_pool.p, (size_t)words * 4, s) != TFIM_OK) {
+            if (dev_alloc(&R.pj_pool.p, bytes, s) != TFIM_OK) {
                 R.pj_pool = Pool{};
                 cudaGetLastError();
                 return TFIM_OK;
             }
-            R.pj_pool.bytes = (size_t)words * 4;
+            R.pj_pool.bytes = bytes;
         }
         TFIM_TRY(grow(R.vrows, (size_t)n_rows * 8, s));
         TFIM_TRY(grow(R.vitem, (size_t)n_rows * 4, s));
         TFIM_TRY(grow(R.pj_off, (size_t)n_pj * (size_t)(nt + 1) * 4, s));
         refresh_ptrs();
+        P.pj_pos = nullptr;
+        if (by_row) {
+            char* at = (char*)R.pj_pool.p + row_bytes;
+            P.pj_tm = (uint32_t*)at;
+            P.pj_inv = (int16_t*)(at + tm_bytes);
+            P.pj_gbits = (uint32_t*)(at + tm_bytes + inv_bytes);
+            P.pj_pos = (int32_t*)(at + tm_bytes + inv_bytes + gb_bytes);
+        }
         k_proj_count<<<sm_count * 8, 256, 0, s>>>(P, n_pj);
         k_proj_scan<<<(n_pj + 7) / 8, 256, 0, s>>>(P, n_pj);
         k_proj_init<<<n_pj, 256, 0, s>>>(P);
-        k_proj_rows<<<sm_count * 4, kProjThreads, 0, s>>>(P, n_pj);
+        if (by_row) {
+            const int tm_smem = (1024 * P.pj_gc + 32) * 4;
+            const int smem = ((((kProjTile * 32 + 32 * kProjWarps + 1) * P.pj_gc + 3) & ~3) * 4) +
+                             kProjWarps * (kProjTile * 32 + 32) * 2;
+            TFIM_CUDA(cudaFuncSetAttribute(k_proj_tm, cudaFuncAttributeMaxDynamicSharedMemorySize, tm_smem));
+            TFIM_CUDA(cudaFuncSetAttribute(k_proj_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+            k_proj_tm<<<dim3((unsigned)(W / 32), (unsigned)P.pj_chunks), 32 * P.pj_gc, tm_smem, s>>>(P);
+            // a short database: several blocks per tile, each for a part of the families
+            const int64_t units = nt * P.pj_chunks;
+            const int32_t parts = (int32_t)std::max<int64_t>(
+                1, std::min<int64_t>((4 * sm_count + units - 1) / units, (n_pj + kProjWarps - 1) / kProjWarps));
+            k_proj_rows<<<(unsigned)std::min<int64_t>(units * parts, sm_count), 32 * kProjWarps, smem, s>>>(P, n_pj, parts);
+        } else {
+            k_proj_words<<<sm_count * 4, kProjThreads, 0, s>>>(P, n_pj);
+        }
         k_proj_commit<<<n_pj, 128, 0, s>>>(P);
         TFIM_CUDA(cudaGetLastError());
-        launches += 5;
+        launches += by_row ? 6 : 5;
         return TFIM_OK;
     };
 

@@ -37,3 +37,22 @@ def test_compressed_row_boundaries(oracle_mod, tmp_path, rows):
     with tf.Database.from_csr(db0.offsets, db0.items, 0.07) as db:
         for graphs in (False, True):
             assert db.mine(engine="resident", small_pools=True, graphs=graphs).as_dict() == expected
+
+
+# 420 items: positions in 14 groups of 32, two chunks of groups.  Three wide clusters are compressed
+# through transposed transactions, forty narrow ones word by word; runs of a cluster's transactions leave
+# tiles without any and last words that end many tiles later.
+@pytest.mark.parametrize("clusters,prob,minsup", [(3, 0.5, 0.06), (40, 0.8, 0.014)])
+@pytest.mark.parametrize("runs", [1, 700, 4001, 20_011])
+def test_groups_of_items(oracle_mod, tmp_path, clusters, prob, minsup, runs):
+    rows, per = 20_011, 420 // clusters
+    rng = np.random.Generator(np.random.PCG64(clusters + runs))
+    cluster = np.arange(rows) // runs % clusters if runs < rows else np.arange(rows) * clusters // rows
+    own = np.arange(clusters * per) % clusters == cluster[:, None]
+    hit = own & (rng.random(own.shape) < prob)
+    path = str(tmp_path / "d.txt")
+    with open(path, "w") as f:
+        f.writelines(" ".join(map(str, np.flatnonzero(r) + 1)) + "\n" for r in hit if r.any())
+    expected = oracle_mod.mine_file(path, minsup)
+    with tf.Database.from_file(path, minsup) as db:
+        assert db.mine(engine="resident", small_pools=True).as_dict() == expected
