@@ -311,7 +311,7 @@ typedef struct {
 /* counting paths of tfim_mine_stats.path_* */
 #define TFIM_PATH_LOP3   0   /* AND + popc tiles on CUDA cores */
 #define TFIM_PATH_B1     1   /* b1 AND+POPC mma.sync tiles */
-#define TFIM_PATH_TC     2   /* tcgen05.mma kind::i8 tiles (bits expanded to bytes) */
+#define TFIM_PATH_TC     2   /* tcgen05.mma kind::mxf4 tiles (bits as 4-bit values) */
 #define TFIM_PATH_PAIRS  3   /* pair co-occurrence over the reduced transaction list */
 #define TFIM_PATH_PROJ   4   /* projected counting over the prefix's transactions */
 #define TFIM_PATH_GRAM   5   /* register-tiled AND+popc Gram blocks of dense narrow families */

@@ -179,8 +179,8 @@ class Clocks:
 
 def i8_gemm_peak(device, n: int = 8192, reps: int = 10) -> float | None:
     """Measured dense int8 GEMM rate (multiply-accumulates per second) of torch._int_mm
-    (cuBLASLt) on `device`: the tensor-pipe roof of the kind::i8 counter, whose bit-ops are
-    0/1 multiply-accumulates.  None when the call is unavailable."""
+    (cuBLASLt) on `device`: a library GEMM's tensor rate on 8-bit operands, to set the tcgen05
+    counters' bit-ops (0/1 multiply-accumulates, on 4-bit operands) against.  None when the call is unavailable."""
     import torch
     try:
         a = torch.randint(-8, 8, (n, n), dtype=torch.int8, device=device)
