@@ -37,30 +37,30 @@ def test_packed_tiles_of_every_width(rows, opts):
         assert got.stats["path_supports"][2] > at * at   # more than the top family on the tensor path
 
 
-# 91 items give 4,095 frequent pairs; each lone item adds one set.
-@pytest.mark.parametrize("lone", [0, 1, 2])
-def test_result_sort_boundary(oracle_mod, tmp_path, lone):
+# 91 items give 4,095 frequent pairs, 45 items 990; each lone item adds one set.
+@pytest.mark.parametrize("wide,lone", [(91, 0), (91, 1), (91, 2), (45, 33), (45, 34), (45, 35), (2, 0)])
+def test_result_sort_boundary(oracle_mod, tmp_path, wide, lone):
     rng = np.random.Generator(np.random.PCG64(lone))
-    hit = np.zeros((4000, 91 + lone), dtype=bool)
-    hit[:2000, :91] = rng.random((2000, 91)) < 0.5
+    hit = np.zeros((2000 + 900 * lone, wide + lone), dtype=bool)
+    hit[:2000, :wide] = rng.random((2000, wide)) < 0.5
     for k in range(lone):
-        hit[2000 + 900 * k : 2900 + 900 * k, 91 + k] = True
+        hit[2000 + 900 * k : 2900 + 900 * k, wide + k] = True
     path = str(tmp_path / "d.txt")
     with open(path, "w") as f:
         f.writelines(" ".join(map(str, np.flatnonzero(r) + 1)) + "\n" for r in hit if r.any())
-    minsup = 369.5 / (2000 + 900 * lone)   # between the supports of pairs and triples
+    minsup = 369.5 / sum(r.any() for r in hit)   # between the supports of pairs and triples
     expected = oracle_mod.mine_file(path, minsup)
-    assert len(expected) == 4095 + lone
+    assert len(expected) == wide * (wide - 1) // 2 + lone
     with tf.Database.from_file(path, minsup) as db:
         for engine in ("resident", "batched"):
             assert db.mine(engine=engine).as_dict() == expected
 
 
-@pytest.mark.parametrize("items", [1023, 1025, 32_768, 32_769])
+@pytest.mark.parametrize("items", [31, 33, 1023, 1025, 32_768, 32_769])
 def test_dense_id_tables(items):
     rng = np.random.Generator(np.random.PCG64(items))
     rows = 300
-    held = [np.sort(rng.choice(items, size=40, replace=False)) + 1 for _ in range(rows)]
+    held = [np.sort(rng.choice(items, size=min(40, items), replace=False)) + 1 for _ in range(rows)]
     held[7] = np.arange(1, items + 1)   # every item occurs; most supports tie
     off = np.concatenate([[0], np.cumsum([len(h) for h in held])]).astype(np.int64)
     flat = np.concatenate(held).astype(np.int32)
