@@ -2012,6 +2012,12 @@ __global__ void __launch_bounds__(kProjThreads, 4) k_proj_words(ResPtrs p, int32
     }
 }
 
+// Dynamic shared memory of k_proj_tm and k_proj_rows at `gc` groups per chunk.
+constexpr int proj_tm_smem(int gc) { return (1024 * gc + 32) * 4; }
+constexpr int proj_rows_smem(int gc) {
+    return ((((kProjTile * 32 + 32 * kProjWarps + 1) * gc + 3) & ~3) * 4) + kProjWarps * (kProjTile * 32 + 32) * 2;
+}
+
 // The families move to their universes: one block per family.
 __global__ void __launch_bounds__(128) k_proj_commit(ResPtrs p) {
     const PJob q = p.pjobs[blockIdx.x];
@@ -3111,11 +3117,10 @@ int mine_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt) {
         k_proj_scan<<<(n_pj + 7) / 8, 256, 0, s>>>(P, n_pj);
         k_proj_init<<<n_pj, 256, 0, s>>>(P);
         if (by_row) {
-            const int tm_smem = (1024 * P.pj_gc + 32) * 4;
-            const int smem = ((((kProjTile * 32 + 32 * kProjWarps + 1) * P.pj_gc + 3) & ~3) * 4) +
-                             kProjWarps * (kProjTile * 32 + 32) * 2;
-            TFIM_CUDA(cudaFuncSetAttribute(k_proj_tm, cudaFuncAttributeMaxDynamicSharedMemorySize, tm_smem));
-            TFIM_CUDA(cudaFuncSetAttribute(k_proj_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+            // the limits are set for the widest chunk, the same from every thread
+            TFIM_CUDA(cudaFuncSetAttribute(k_proj_tm, cudaFuncAttributeMaxDynamicSharedMemorySize, proj_tm_smem(kProjGroups)));
+            TFIM_CUDA(cudaFuncSetAttribute(k_proj_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, proj_rows_smem(kProjGroups)));
+            const int tm_smem = proj_tm_smem(P.pj_gc), smem = proj_rows_smem(P.pj_gc);
             k_proj_tm<<<dim3((unsigned)(W / 32), (unsigned)P.pj_chunks), 32 * P.pj_gc, tm_smem, s>>>(P);
             // a short database: several blocks per tile, each for a part of the families
             const int64_t units = nt * P.pj_chunks;
