@@ -698,22 +698,18 @@ __device__ __forceinline__ void res_pack(const ResPtrs& p) {
         }
         __syncthreads();
     }
-    // a wave whose packed jobs are little work in all counts them on the CUDA cores instead
+    // a wave whose packed jobs are little work in all counts them on the CUDA cores instead.  The
+    // shared sums are only read from here on: what the decision changes stays in registers
     const bool few_pk = p.counter == TFIM_COUNTER_AUTO && s_words[1] > 0 && s_pk_work < kPkMinWork;
-    if (few_pk) {
-        if (tid == 0) {
-            s_cost += s_pk_cost;
-            s_words[1] = 0;
-        }
-        __syncthreads();
-    }
+    const int64_t pk_words = few_pk ? 0 : (int64_t)s_words[1];
+    const float l3_total = s_cost + (few_pk ? s_pk_cost : 0.f);
     // the wave's estimated CUDA-core cost over (slices per SM x SMs): the cost of one tile
     // slice; dense families are split more finely (their own target), which shortens the
     // launch's tail on large dense databases
-    const float target = fmaxf(s_cost / (p.l3_slices_per_sm * (float)p.sm_count), 1.f);
-    const float target_d = fmaxf(s_cost / (p.l3_dense_slices_per_sm * (float)p.sm_count), 1.f);
+    const float target = fmaxf(l3_total / (p.l3_slices_per_sm * (float)p.sm_count), 1.f);
+    const float target_d = fmaxf(l3_total / (p.l3_dense_slices_per_sm * (float)p.sm_count), 1.f);
     const int64_t sw_b1 = slice_words((int64_t)s_words[0], (int64_t)(p.b1_tiles_per_sm * (float)p.sm_count));
-    const int64_t sw_tc = slice_words((int64_t)s_words[1], (int64_t)(p.tc_tiles_per_sm * (float)p.sm_count));
+    const int64_t sw_tc = slice_words(pk_words, (int64_t)(p.tc_tiles_per_sm * (float)p.sm_count));
     const int64_t sw_gr = slice_words((int64_t)s_words[2], (int64_t)(p.l3_slices_per_sm * (float)p.sm_count));
     int32_t tot[kGrps] = {0, 0, 0, 0, 0, 0};
     for (int base = 0; base < (small ? 0 : nj); base += kPackThreads) {
@@ -789,7 +785,7 @@ __device__ __forceinline__ void res_pack(const ResPtrs& p) {
         }
         return run;
     };
-    if (!small && s_words[1] > 0) {
+    if (!small && pk_words > 0) {
         for (int base = 0; base < nj; base += kPackThreads) {
             const int j = base + tid;
             int32_t v[kPkClasses] = {0, 0, 0, 0, 0, 0, 0}, ex[kPkClasses], t[kPkClasses];
