@@ -337,7 +337,9 @@ typedef struct {
     double  rate_pair_incr;     /*   pair co-occurrence increments/s */
     int32_t i8_min_rows;        /* automatic choice: the tcgen05 wave counter for count jobs */
     int32_t i8_min_cols;        /*   of at least i8_min_rows x i8_min_cols (tfim_count_wave and
-                                     the empty-prefix family's bitmap Gram) */
+                                     the empty-prefix family's bitmap Gram; a wave up to two rows
+                                     earlier where the call is bound by its launches, up to four
+                                     later over long sparse rows or few items) */
     double  rate_i8_bitops;     /* cost model: tcgen05 wave counter bit-ops/s */
     int32_t tc_min_work;        /* automatic choice: the tcgen05 family counter for family jobs of
                                    at most 128 columns with rows x columns >= tc_min_work and a */

@@ -13,6 +13,7 @@
 #include <string>
 
 #include "tfim_internal.h"
+#include "wave_route.h"
 
 namespace tfim {
 int ingest_csr(tfim_ctx* c, const int64_t* off, const int32_t* items, int64_t n_rows, double thr);
@@ -96,13 +97,9 @@ int count_wave_impl(tfim_ctx* c, int32_t b, int32_t min_count, const WaveLists& 
     // host-built job/tile tables (independent of the list contents)
     const int32_t counter = c->counter_pref;
     const tfim_tuning tn = tuning();
-    // One or two rows over a long bitmap stay on the CUDA-core tiles: the tensor tiles read every
-    // column word whatever the row masks hold (1 row x 6,162 long-tail items x 1M transactions:
-    // 377 us against 130), while up to 2^14 words the call is launch-bound and the tensor tiles are
-    // the shorter launch (1 row x 69 items x 262,144 transactions: 49 us against 80).
     const bool i8 = counter == TFIM_COUNTER_I8 ||
-                    (counter == TFIM_COUNTER_AUTO && d >= tn.i8_min_cols &&
-                     (b >= tn.i8_min_rows || c->W <= (1 << 14)));
+                    (counter == TFIM_COUNTER_AUTO &&
+                     wave_on_tensor(b, d, c->W, c->empty_share, tn.i8_min_rows, tn.i8_min_cols));
     const bool b1 = !i8 && (counter == TFIM_COUNTER_TENSOR ||
                             (counter == TFIM_COUNTER_AUTO && b >= tn.b1_min_rows && d >= tn.b1_min_cols));
     std::vector<JobDesc> jobs(1, JobDesc{});

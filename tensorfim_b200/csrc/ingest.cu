@@ -20,6 +20,7 @@
 #include <atomic>
 
 #include "tfim_internal.h"
+#include "wave_route.h"
 
 namespace tfim {
 namespace {
@@ -389,6 +390,7 @@ int compute_bit_supports(tfim_ctx* c) {
         c->csr_exact = inexact == 0;
     }
     c->bit_support.assign(all.begin(), all.begin() + std::min<int32_t>(rows, c->n_counted));
+    c->empty_share = empty_pieces(c->bit_support.data(), (int64_t)c->bit_support.size(), c->sharded ? c->n_bits_total : c->n_bits);
     return TFIM_OK;
 }
 

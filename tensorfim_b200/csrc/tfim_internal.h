@@ -292,6 +292,7 @@ struct tfim_ctx {
     int64_t n_bits = 0;
     int32_t n_counted = 0;
     std::vector<int32_t> bit_support;      // popc of each counted row (bitmap supports)
+    float empty_share = 0.f;               // pieces of 128 transactions that a one-item prefix leaves empty
     std::vector<int32_t> support_order;    // the counted rows in increasing support, ties by row (or empty)
     // reduced transaction list (dense ids): row rr = red_items[red_off[rr] .. red_off[rr+1])
     int64_t* d_red_off = nullptr;
