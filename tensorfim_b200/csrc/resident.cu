@@ -2542,6 +2542,10 @@ void stash_resident(tfim_ctx* c) {
     std::lock_guard<std::mutex> lk(g_cache_mu);
     if (c->resident) {
         c->resident->graph.release();   // its launches hold this context's transaction list
+        // the projected rows, which may be many GB, go back to the device's pool: their size is this
+        // database's own
+        dev_free(c->resident->pj_pool.p, c->stream);
+        c->resident->pj_pool = Pool{};
         if (g_cached_res[dev]) free_resident(g_cached_res[dev], c->stream);
         g_cached_res[dev] = c->resident;
         c->resident = nullptr;

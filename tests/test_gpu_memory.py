@@ -1,0 +1,53 @@
+"""Mining on a GPU whose memory mostly belongs to someone else: the projected rows of the resident
+engine (csrc/resident.cu) do not outlive their database.  Each case is a process of its own, so that
+no other test's pools count."""
+import os
+import subprocess
+import sys
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+# `d` independent items in a fifth of 262,144 transactions each: every pair is frequent at 3%, no triple is
+CHILD = r'''
+import sys
+import numpy as np
+import torch
+import tensorfim_b200 as tf
+
+n, d, free, then = 262_144, int(sys.argv[1]), int(sys.argv[2]) << 20, int(sys.argv[3]) << 20
+gen = torch.Generator("cuda").manual_seed(1)
+hit = torch.cat([torch.rand(65536, d, device="cuda", generator=gen) < 0.2 for _ in range(n // 65536)])
+pair = sum(x.float().T @ x.float() for x in hit.split(65536)).round().long().cpu().numpy()
+off = np.zeros(n + 1, np.int64)
+off[1:] = hit.sum(1).cumsum(0).cpu().numpy()
+items = (hit.nonzero()[:, 1] + 1).to(torch.int32).cpu().numpy()
+del hit
+torch.cuda.empty_cache()
+with tf.Database.from_csr(off, items, 0.03) as db:
+    hog = torch.empty(torch.cuda.mem_get_info()[0] - free, dtype=torch.uint8, device="cuda")
+    for _ in range(2):
+        got = db.mine(engine="resident")
+        assert len(got) == d * (d - 1) // 2 and (np.diff(got.offsets) == 2).all()
+        a, b = got.items[0::2] - 1, got.items[1::2] - 1
+        assert (got.supports == pair[a, b]).all() and len(set(zip(a.tolist(), b.tolist()))) == len(got)
+if then:
+    rows = np.zeros((then >> 15, 1 << 13), np.uint32)
+    rows[:, 5] = 3
+    with tf.Database.from_bitmap(rows, 1 << 18, 1) as db:
+        assert db.count_wave([[], [2]], 1)[0].tolist() == [[2], [2]]
+print("mined")
+'''
+
+
+# MiB left, a little more than the search takes (3,200 measured), and a database of 1,400 MiB opened
+# where the projected rows (1,650 MiB) were.
+@pytest.mark.parametrize("items,free,then", [(500, 3400, 1400)])
+def test_little_memory_left(items, free, then):
+    r = subprocess.run([sys.executable, "-c", CHILD, str(items), str(free), str(then)], cwd=ROOT, capture_output=True, text=True,
+                       timeout=300)
+    assert r.returncode == 0 and r.stdout.strip() == "mined", r.stderr[-1500:]
