@@ -69,6 +69,22 @@ int dev_alloc(void** p, size_t bytes, cudaStream_t s) {
     return TFIM_OK;
 }
 
+size_t dev_unused(int dev) {
+    cudaMemPool_t pool = device_pool(dev);
+    uint64_t held = 0, used = 0;
+    if (!pool || cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held) != cudaSuccess ||
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return held > used ? (size_t)(held - used) : 0;
+}
+
+void dev_trim(int dev) {
+    cudaMemPool_t pool = device_pool(dev);
+    if (pool && cudaMemPoolTrimTo(pool, 0) != cudaSuccess) cudaGetLastError();
+}
+
 void dev_free(void* p, cudaStream_t s) {
     if (!p) return;
     int dev = 0;

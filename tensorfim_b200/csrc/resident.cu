@@ -2490,6 +2490,7 @@ struct ResidentState {
     Pool pk_list, loop_bar;
     Pool pjobs, pj_off, pj_pool, vrows, vitem;              // projected families
     Pool ord_keys, ord_idx, ord_meta, ord_items, ord_tmp;   // output order of the MFIs
+    size_t mem_total = 0;                                   // the device's memory (0: not asked for yet)
     HostBuf h_status, h_args, h_res, h_setup, h_first, h_tiles;
     // the database's part of the search's initial state (root flags, the top family in
     // increasing support order), computed at a context's first resident mine and its pinned
@@ -2685,7 +2686,8 @@ void finish_mfi_order(MfiSet& M, const uint64_t* key) {
 }
 }  // namespace
 
-int mine_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt) {
+namespace {
+int search_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt, bool may_project, bool* projected) {
     const auto t_entry = std::chrono::steady_clock::now();
     cudaStream_t s = c->stream;
     const int32_t d = c->n_counted;
@@ -2819,7 +2821,7 @@ int mine_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt) {
     // for a wave's counting to outweigh the extra status read (small_pools: any length, so that
     // short ones exercise it), some frequent item lies in at most half of it, and no counter that
     // reads the transaction list may be picked.
-    const bool project = (W >= (1 << 12) || small) && 2 * (int64_t)c->bit_support[F0.front()] <= c->n_bits &&
+    const bool project = may_project && (W >= (1 << 12) || small) && 2 * (int64_t)c->bit_support[F0.front()] <= c->n_bits &&
                          64 * (int64_t)minc >= c->n_bits && !may_list;
     const bool top_loop = loop && !project && o->top_counter == 0 && top_mode == 1 && n0 <= wave_rows &&
                           (double)n0 * n0 * (double)W <= kLoopTopWork;
@@ -3067,18 +3069,7 @@ int mine_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt) {
         const int32_t n_pj = hst->pj_n;
         const int64_t n_rows = hst->pj_rows, words = hst->pj_words;
         if (n_pj == 0) return TFIM_OK;
-        // the compressed rows may take an eighth of the device's memory; without room for them
-        // the families stay where they are
-        static std::atomic<size_t> total_of[64];   // device memory, asked for once (the call is slow)
-        std::atomic<size_t>& total = total_of[c->device & 63];
-        if (!total.load()) {
-            size_t mem_free = 0, mem_total = 0;
-            TFIM_CUDA(cudaMemGetInfo(&mem_free, &mem_total));
-            total.store(mem_total);
-        }
         const size_t row_bytes = (size_t)words * 4, off_bytes = (size_t)n_pj * (size_t)(nt + 1) * 4;
-        if (row_bytes + off_bytes > total.load() / 8) return TFIM_OK;
-        const size_t room = total.load() / 8 - off_bytes;
         // groups of 32 items, in chunks that shared memory holds; an odd number per chunk
         const int32_t groups = (n0 + 31) / 32;
         P.pj_chunks = (groups + kProjGroups - 1) / kProjGroups;
@@ -3086,11 +3077,28 @@ int mine_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt) {
         const int64_t n_g = (int64_t)P.pj_chunks * P.pj_gc;
         const size_t tm_bytes = (size_t)n_g * W * 128, inv_bytes = (size_t)n_pj * n_g * 64,
                      gb_bytes = (size_t)n_pj * P.pj_chunks * 4, extra = tm_bytes + inv_bytes + gb_bytes + (size_t)P.n_base * 4;
-        const bool by_row = n_rows >= kProjMinCols * hst->pj_groups && n0 <= 32767 && row_bytes + extra <= room;
-        const size_t bytes = row_bytes + (by_row ? extra : 0);
+        bool by_row = n_rows >= kProjMinCols * hst->pj_groups && n0 <= 32767;
+        size_t bytes = row_bytes + (by_row ? extra : 0);
         if (bytes > R.pj_pool.bytes) {   // its old contents are not needed
             dev_free(R.pj_pool.p, s);
             R.pj_pool = Pool{};
+            // The compressed rows may take an eighth of the device's memory, and half of what is left
+            // of it: later waves' pools grow beside them.  Without room for the transposed copy they
+            // are made word by word, without room for them the families stay where they are.  The
+            // driver is asked (slowly) only when the pool's own unused memory is not enough.
+            const size_t side = off_bytes + (size_t)n_rows * 12;
+            size_t left = dev_unused(c->device), room = left / 2;
+            if (bytes + side > room || !R.mem_total) {
+                size_t mem_free = 0;
+                TFIM_CUDA(cudaMemGetInfo(&mem_free, &R.mem_total));
+                room = (left + mem_free) / 2;
+            }
+            room = std::min(room, R.mem_total / 8);
+            if (bytes + side > room) {
+                by_row = false;
+                bytes = row_bytes;
+                if (bytes + side > room) return TFIM_OK;
+            }
             if (dev_alloc(&R.pj_pool.p, bytes, s) != TFIM_OK) {
                 R.pj_pool = Pool{};
                 cudaGetLastError();
@@ -3132,6 +3140,7 @@ int mine_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt) {
         }
         k_proj_commit<<<n_pj, 128, 0, s>>>(P);
         TFIM_CUDA(cudaGetLastError());
+        *projected = true;
         launches += by_row ? 6 : 5;
         return TFIM_OK;
     };
@@ -3481,6 +3490,25 @@ int mine_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt) {
     stt->bit_ops = stt->supports * c->n_bits;
     stt->readback_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_read0).count();
     return TFIM_OK;
+}
+}  // namespace
+
+int mine_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt) {
+    const tfim_mine_stats before = *stt;
+    bool projected = false;
+    int rc = search_resident(c, o, stt, true, &projected);
+    if (rc == TFIM_E_NOMEM && projected) {
+        // the search's pools found no room beside the projected rows: once more without these
+        TFIM_CUDA(cudaStreamSynchronize(c->stream));
+        dev_free(c->resident->pj_pool.p, c->stream);
+        c->resident->pj_pool = Pool{};
+        TFIM_CUDA(cudaStreamSynchronize(c->stream));
+        dev_trim(c->device);
+        c->mfis.clear();
+        *stt = before;
+        rc = search_resident(c, o, stt, false, &projected);
+    }
+    return rc;
 }
 
 }  // namespace tfim

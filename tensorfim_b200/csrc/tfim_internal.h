@@ -55,6 +55,8 @@ constexpr int kMaxListLen = 64;   // longest item list one counted row may AND
 // cache of blocks.
 int dev_alloc(void** p, size_t bytes, cudaStream_t s);
 void dev_free(void* p, cudaStream_t s);
+size_t dev_unused(int dev);   // bytes that the device's pool holds and nobody uses
+void dev_trim(int dev);       // gives them back to the driver
 void* pinned_alloc(size_t bytes, size_t* got);
 void pinned_free(void* p, size_t bytes);
 // Non-blocking streams of the current device from a bounded free list (creating one takes 0.3 ms);
