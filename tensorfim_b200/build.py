@@ -25,7 +25,7 @@ NVFLAGS = ["-O3", "-std=c++17", "-lineinfo", *ARCH, "-Xcompiler", "-fPIC,-fvisib
            "-I" + INCLUDE, "-I" + CSRC, "-diag-suppress", "177"]
 
 CU_SOURCES = ["common.cu", "parse.cu", "ingest.cu", "count_lop3.cu", "count_b1.cu", "count_pairs.cu", "count_proj.cu", "count_f4.cu", "count_pk.cu", "count_gram.cu", "allfi.cu", "shard.cu", "count_static.cu", "mlp.cu", "mine.cu", "resident.cu", "abi.cu"]
-HEADERS = [os.path.join(CSRC, "tfim_internal.h"), os.path.join(CSRC, "tcgen05.cuh"), os.path.join(CSRC, "wave_route.h"), os.path.join(INCLUDE, "tfim.h")]
+HEADERS = [os.path.join(CSRC, "tfim_internal.h"), os.path.join(CSRC, "tcgen05.cuh"), os.path.join(CSRC, "wave_route.h"), os.path.join(CSRC, "search_error.h"), os.path.join(INCLUDE, "tfim.h")]
 
 
 def _newer(target: str, deps: list[str]) -> bool:

@@ -24,6 +24,7 @@
 #include <cstring>
 #include <numeric>
 
+#include "search_error.h"
 #include "tfim_internal.h"
 
 namespace tfim {
@@ -1166,7 +1167,7 @@ __device__ void expand_row(const ResPtrs& p, int64_t g, int lane) {
     const int32_t t = F[i];
     const int32_t supc = crow[i];
     if (supc < minc) {   // cannot happen: t is in F(P)
-        if (lane == 0) atomicExch(&st->error, 1);
+        if (lane == 0) atomicExch(&st->error, kErrRow);
         finish_row(p, fp, lane);
         return;
     }
@@ -1698,7 +1699,7 @@ __global__ void __launch_bounds__(256) k_proj_scan(ResPtrs p, int32_t n_pj) {
         if (t <= nt) off[t] = sum + x;
         sum += __shfl_sync(0xffffffffu, x, 31);
     }
-    if (lane == 0 && sum != p.pjobs[k].sup) atomicExch(&p.st->error, 2);
+    if (lane == 0 && sum != p.pjobs[k].sup) atomicExch(&p.st->error, kErrProjected);
 }
 
 // The row table's entries, zeros in the padding, and what the chosen way of compressing needs: the
@@ -2157,7 +2158,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_res_loop(ResPtrs p, uint32_
         first = false;
         bool ok = grid_barrier(bar, arrived += gridDim.x);
         if (!ok || st->loop_go != 1) {
-            if (!ok && threadIdx.x == 0) atomicExch(&st->error, 3);
+            if (!ok && threadIdx.x == 0) atomicExch(&st->error, kErrWait);
             if (blockIdx.x == 0) publish_status(p);
             return;
         }
@@ -2168,7 +2169,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_res_loop(ResPtrs p, uint32_
             for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
                 p.counts[i] = 0;
             if (!grid_barrier(bar, arrived += gridDim.x)) {
-                if (threadIdx.x == 0) atomicExch(&st->error, 3);
+                if (threadIdx.x == 0) atomicExch(&st->error, kErrWait);
                 if (blockIdx.x == 0) publish_status(p);
                 return;
             }
@@ -2193,7 +2194,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_res_loop(ResPtrs p, uint32_
             ok = grid_barrier(bar, arrived += gridDim.x);
         }
         if (!ok) {
-            if (threadIdx.x == 0) atomicExch(&st->error, 3);
+            if (threadIdx.x == 0) atomicExch(&st->error, kErrWait);
             if (blockIdx.x == 0) publish_status(p);
             return;
         }
@@ -2687,6 +2688,12 @@ void finish_mfi_order(MfiSet& M, const uint64_t* key) {
 }  // namespace
 
 namespace {
+int check_search(int32_t error) {
+    TFIM_CHECK(error != kErrWait, search_error_status(error), "resident search: a wait of the device loop's grid barrier expired");
+    TFIM_CHECK(error == 0, search_error_status(error), "resident search invariant failed (code %d)", error);
+    return TFIM_OK;
+}
+
 int search_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt, bool may_project, bool* projected) {
     const auto t_entry = std::chrono::steady_clock::now();
     cudaStream_t s = c->stream;
@@ -3271,7 +3278,7 @@ int search_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt, 
             const double ts = std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count();
             TFIM_CUDA(cudaStreamSynchronize(s));
             sync_ms += (std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count() - ts) * 1e3;
-            TFIM_CHECK(hst->error == 0, TFIM_E_STATE, "resident search invariant failed (code %d)", hst->error);
+            TFIM_TRY(check_search(hst->error));
             if (hst->starved || hst->grow) {
                 TFIM_TRY(grow_for(*hst));
                 continue;
@@ -3307,7 +3314,7 @@ int search_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt, 
         const double ts = std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count();
         TFIM_CUDA(cudaStreamSynchronize(s));
         sync_ms += (std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count() - ts) * 1e3;
-        TFIM_CHECK(hst->error == 0, TFIM_E_STATE, "resident search invariant failed (code %d)", hst->error);
+        TFIM_TRY(check_search(hst->error));
         if (hst->starved || hst->grow) {
             TFIM_TRY(grow_for(*hst));
             continue;
