@@ -48,6 +48,7 @@ int make_ctx(int32_t device, tfim_ctx** out) {
     for (auto& b : c->d_scratch) b.stream = c->stream;
     c->d_masks.stream = c->stream;
     c->d_group.stream = c->stream;
+    c->d_status.stream = c->stream;
     *out = c;
     return TFIM_OK;
 }
@@ -88,7 +89,7 @@ int make_sharded_ctx(int32_t device, const tfim_group* g, bool args_ok, const st
 // Per-node masks + one count job over every counted row (the reference counting contract).  The
 // tables of the count job and, for lists on the host, the lists go up in one copy; one kernel
 // builds the masks and clears the counts, one counts the frequent columns and hands small
-// results and the counter's error flag to pinned host memory.
+// results and the counter's status to pinned host memory.
 int count_wave_impl(tfim_ctx* c, int32_t b, int32_t min_count, const WaveLists& L, int32_t* d_counts, int32_t* d_nfreq,
                     cudaStream_t s, int32_t* out) {
     const int32_t d = c->n_counted;
@@ -142,7 +143,9 @@ int count_wave_impl(tfim_ctx* c, int32_t b, int32_t min_count, const WaveLists& 
     const size_t o_items = o_off + (L.h_off ? (size_t)(b + 1) * 8 : 0), total = o_items + n_items * 4;
     TFIM_TRY(c->h_scratch[0].reserve(total));
     TFIM_TRY(c->d_scratch[0].reserve(total));
-    TFIM_TRY(c->h_flags.reserve(64));
+    TFIM_TRY(c->h_status.reserve(64));
+    TFIM_TRY(c->d_status.reserve(64));
+    int32_t* status = c->d_status.as<int32_t>();
     unsigned char* hp = c->h_scratch[0].as<unsigned char>();
     memcpy(hp, jobs.data(), sizeof(JobDesc));
     memcpy(hp + o_rows, rows.data(), rows.size() * sizeof(RowDesc));
@@ -161,23 +164,22 @@ int count_wave_impl(tfim_ctx* c, int32_t b, int32_t min_count, const WaveLists& 
     TFIM_CUDA(cudaMemcpyAsync(dp, hp, total, cudaMemcpyHostToDevice, s));
     TFIM_TRY(launch_wave_begin(c->d_bitmap, W, c->d_masks.as<uint32_t>(), L.d_mats,
                                L.h_off ? (const int64_t*)(dp + o_off) : L.d_off,
-                               L.h_off ? (const int32_t*)(dp + o_items) : L.d_items, b, d_counts, (int64_t)b * d, s));
+                               L.h_off ? (const int32_t*)(dp + o_items) : L.d_items, b, d_counts, (int64_t)b * d, status, s));
     CountArgs a;
     a.bitmap = c->d_bitmap; a.W = W; a.masks = c->d_masks.as<uint32_t>();
     a.jobs = (const JobDesc*)dp; a.rows = (const RowDesc*)(dp + o_rows); a.cols = (const int32_t*)(dp + o_cols);
     a.tiles = (const TileDesc*)(dp + o_tiles); a.n_tiles = (int32_t)tiles.size(); a.out = d_counts;
-    const int32_t* flag = nullptr;
-    volatile int32_t* flag_to = c->h_flags.as<int32_t>();
-    *flag_to = 0;
+    a.status = status;
+    volatile int32_t* status_to = c->h_status.as<int32_t>();
+    *status_to = 0;
     if (d > 0) {
-        if (i8) TFIM_TRY(count_f4_flag(&flag));
         TFIM_TRY(i8 ? launch_count_f4(a, wide, s) : b1 ? launch_count_b1(a, s) : launch_count_lop3(a, s));
         TFIM_TRY(group_reduce(c, d_counts, (int64_t)b * d, TFIM_DT_I32, TFIM_RED_SUM, s));
     }
-    TFIM_TRY(launch_nfreq(d_counts, b, d, min_count, d_nfreq, s, out, flag, flag ? (int32_t*)flag_to : nullptr));
+    TFIM_TRY(launch_nfreq(d_counts, b, d, min_count, d_nfreq, s, out, status, (int32_t*)status_to));
     // the host staging buffer may be reused by the next call only after its copy ran
     TFIM_CUDA(cudaStreamSynchronize(s));
-    return count_f4_status_check(*flag_to);
+    return tensor_status_check(*status_to);
 }
 
 namespace {
@@ -631,7 +633,8 @@ void tfim_close(tfim_ctx* c) {
     tfim::dev_free(c->d_red_items, c->stream);
     for (auto& b : c->d_scratch) b.release();
     for (auto& b : c->h_scratch) b.release();
-    c->h_flags.release();
+    c->h_status.release();
+    c->d_status.release();
     c->d_masks.release();
     c->d_group.release();
     if (c->stream) cudaStreamSynchronize(c->stream);

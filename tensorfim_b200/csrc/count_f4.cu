@@ -74,8 +74,6 @@ constexpr int kQAWarps = 8;                      // wide tiles: warps that expan
 constexpr int kQWideSmem = kQWideStages * kQBlocks * kQN * 128 + 1024;
 static_assert((kQM + kQN) / 8 <= kQUnits * kQExpWarps, "units fit the expansion warps");
 
-__device__ int g_f4_status;   // 0 ok, 1 an mbarrier wait expired
-
 // The expansion of one warp: U units of 8 rows (an A unit holds columns of the job, a B unit
 // rows), kQFlight / U stages of raw words ahead.  Returns false when a wait expired.
 template <int U, int NW = kQExpWarps>
@@ -313,7 +311,7 @@ __global__ void __launch_bounds__(kQThreads, 1) k_count_f4(CountArgs a) {
             }
             if (!ok) {
                 atomicExch(&s_abort, 1);
-                atomicExch(&g_f4_status, 1);
+                atomicExch(a.status, 1);
             }
             tc_commit(smem_u32(&done));   // tracks every MMA issued so far
         }
@@ -331,7 +329,7 @@ __global__ void __launch_bounds__(kQThreads, 1) k_count_f4(CountArgs a) {
         else ok = f4_expand<3>(a, t, j, units_a, units_b, rb, kc, base, S, n_st, full, empty, warp, lane);
         if (!ok && lane == 0) {
             atomicExch(&s_abort, 1);
-            atomicExch(&g_f4_status, 1);
+            atomicExch(a.status, 1);
         }
         // ---- epilogue: warp w reads lanes 32 * (w % 4) (columns of the job), accumulator columns
         // 16 * (w / 4) + 64 k (rows of the job)
@@ -340,7 +338,7 @@ __global__ void __launch_bounds__(kQThreads, 1) k_count_f4(CountArgs a) {
         const bool all_fin = __all_sync(0xffffffffu, fin);
         if (!all_fin && lane == 0) {
             atomicExch(&s_abort, 1);
-            atomicExch(&g_f4_status, 1);
+            atomicExch(a.status, 1);
         }
         if (all_fin && !*(volatile int32_t*)&s_abort && n_st > 0) {
             const int quad = warp & 3, c = t.c0 + 32 * quad + lane;
@@ -422,32 +420,8 @@ int launch_count_f4(const CountArgs& a, bool wide, cudaStream_t s) {
     return TFIM_OK;
 }
 
-int count_f4_status_fetch(int32_t* pinned, cudaStream_t s) {
-    TFIM_CUDA(cudaMemcpyFromSymbolAsync(pinned, g_f4_status, sizeof(int32_t), 0, cudaMemcpyDeviceToHost, s));
-    return TFIM_OK;
-}
-
-int count_f4_flag(const int32_t** flag) {
-    static std::atomic<const int32_t*> at[64];
-    int dev = 0;
-    TFIM_CUDA(cudaGetDevice(&dev));
-    const int32_t* p = at[dev & 63].load();
-    if (!p) {
-        void* q = nullptr;
-        TFIM_CUDA(cudaGetSymbolAddress(&q, g_f4_status));
-        p = (const int32_t*)q;
-        at[dev & 63].store(p);
-    }
-    *flag = p;
-    return TFIM_OK;
-}
-
-int count_f4_status_check(int32_t v) {
-    if (v) {
-        const int z = 0;
-        TFIM_CUDA(cudaMemcpyToSymbol(g_f4_status, &z, sizeof z));
-    }
-    TFIM_CHECK(v == 0, TFIM_E_TIMEOUT, "tensor-memory counter: an mbarrier wait expired");
+int tensor_status_check(int32_t v) {
+    TFIM_CHECK(v == 0, TFIM_E_TIMEOUT, "tensor-core counter: an mbarrier wait expired");
     return TFIM_OK;
 }
 

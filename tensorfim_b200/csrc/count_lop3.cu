@@ -348,7 +348,7 @@ __global__ void k_materialize(const uint32_t* __restrict__ B, int64_t W, uint32_
 }
 
 // The begin of a counting wave: prefix masks as in k_materialize (lists by descriptor or by
-// offset), and the count block's zeros.  grid = (nodes, word blocks of 256 U pieces): the blocks at
+// offset), the count block's zeros and the status word's.  grid = (nodes, word blocks of 256 U pieces): the blocks at
 // work share one stretch of the item rows, so that these come from L2 and memory sees each item
 // row once and each mask once.  Bound by memory then.  U pieces a thread keep the block count low.
 // Measured at 2,048 prefixes x 512 items x 8M transactions: 0.57 ms (2.7 GB, 4.7 TB/s), with
@@ -361,9 +361,10 @@ template <int U>
 __global__ void __launch_bounds__(256) k_wave_begin(const uint32_t* __restrict__ B, int64_t W, uint32_t* __restrict__ masks,
                                                     const MatDesc* __restrict__ mats, const int64_t* __restrict__ off,
                                                     const int32_t* __restrict__ items, int32_t* __restrict__ counts,
-                                                    int64_t n_zero) {
+                                                    int64_t n_zero, int32_t* status) {
     const int64_t t0 = (blockIdx.y * (int64_t)gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x;
     for (int64_t i = t0; i < n_zero; i += (int64_t)gridDim.x * gridDim.y * blockDim.x) counts[i] = 0;
+    if (t0 == 0) *status = 0;
     const int32_t node = blockIdx.x;
     const int64_t first = mats ? mats[node].off : off[node];
     const int32_t n = mats ? mats[node].n : (int32_t)(off[node + 1] - first);
@@ -387,10 +388,10 @@ __global__ void __launch_bounds__(256) k_wave_begin(const uint32_t* __restrict__
 
 // One warp per row.  `out` (pinned host memory): nfreq of every row, then the counts.
 __global__ void k_nfreq(const int32_t* __restrict__ counts, int64_t n_rows, int32_t n_cols, int32_t min_count,
-                        int32_t* __restrict__ nfreq, int32_t* __restrict__ out, const int32_t* flag, int32_t* flag_to) {
+                        int32_t* __restrict__ nfreq, int32_t* __restrict__ out, const int32_t* status, int32_t* status_to) {
     const int64_t g = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
-    if (flag_to && g == 0 && lane == 0) *flag_to = *flag;
+    if (status_to && g == 0 && lane == 0) *status_to = *status;
     if (g >= n_rows) return;
     const int32_t* row = counts + g * n_cols;
     int32_t c = 0;
@@ -483,25 +484,25 @@ int launch_materialize(const uint32_t* bitmap, int64_t W, uint32_t* masks, const
 }
 
 int launch_wave_begin(const uint32_t* bitmap, int64_t W, uint32_t* masks, const MatDesc* mats, const int64_t* off,
-                      const int32_t* items, int32_t b, int32_t* counts, int64_t n_zero, cudaStream_t s) {
+                      const int32_t* items, int32_t b, int32_t* counts, int64_t n_zero, int32_t* status, cudaStream_t s) {
     if (b <= 0) return TFIM_OK;
     const int64_t by = (W / 4 + 255) / 256;
     // four pieces a thread when that still leaves several blocks for every SM
     if (by * b >= kWaveBeginWide)
         k_wave_begin<4><<<dim3((unsigned)b, (unsigned)std::min<int64_t>((by + 3) / 4, 65535)), 256, 0, s>>>(
-            bitmap, W, masks, mats, off, items, counts, n_zero);
+            bitmap, W, masks, mats, off, items, counts, n_zero, status);
     else
         k_wave_begin<1><<<dim3((unsigned)b, (unsigned)std::max<int64_t>(1, by)), 256, 0, s>>>(
-            bitmap, W, masks, mats, off, items, counts, n_zero);
+            bitmap, W, masks, mats, off, items, counts, n_zero, status);
     TFIM_CUDA(cudaGetLastError());
     return TFIM_OK;
 }
 
 int launch_nfreq(const int32_t* counts, int64_t n_rows, int32_t n_cols, int32_t min_count, int32_t* nfreq,
-                 cudaStream_t s, int32_t* out, const int32_t* flag, int32_t* flag_to) {
+                 cudaStream_t s, int32_t* out, const int32_t* status, int32_t* status_to) {
     if (n_rows <= 0) return TFIM_OK;
     const int64_t threads = n_rows * 32;
-    k_nfreq<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(counts, n_rows, n_cols, min_count, nfreq, out, flag, flag_to);
+    k_nfreq<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(counts, n_rows, n_cols, min_count, nfreq, out, status, status_to);
     TFIM_CUDA(cudaGetLastError());
     return TFIM_OK;
 }

@@ -55,12 +55,9 @@ constexpr int kPAhead = 2;
 constexpr int kPSmem = kPStages * kPStageBytes + 1024;
 constexpr uint32_t kPScale = 256;                // accumulators at columns 0 and 128, scales from here
 
-__device__ int g_pk_status;   // 0 ok, 1 an mbarrier wait expired
-
 struct PkShared {
     uint64_t full[kPStages], empty[kPStages], acc_full[2], acc_empty[2], drain;
     uint32_t tmem;
-    int32_t abort;
 };
 
 // The units [u0, u1) that hold the tile's tail rows (whole warp; the same on every lane).
@@ -98,7 +95,6 @@ __global__ void __launch_bounds__(kPThreads, 1) k_count_pk(CountArgs a_val, cons
             }
             mbar_init(smem_u32(&sh.drain), 1);
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-            sh.abort = 0;
         }
         if (warp == kPExpWarps) tmem_alloc(smem_u32(&sh.tmem), 512);
         tc_fence_before();
@@ -263,10 +259,7 @@ __global__ void __launch_bounds__(kPThreads, 1) k_count_pk(CountArgs a_val, cons
                 if (lane == 0) mbar_arrive(smem_u32(&sh.acc_empty[i & 1]));
             }
         }
-        if (!ok && lane == 0) {
-            atomicExch(&sh.abort, 1);
-            atomicExch(&g_pk_status, 1);
-        }
+        if (!ok && lane == 0) atomicExch(a.status, 1);
         tc_fence_before();
         __syncthreads();
         if (warp == kPExpWarps) tmem_free(tmem, 512);
@@ -300,20 +293,6 @@ int launch_count_pk_persistent(const CountArgs* d_args, const int32_t* d_n_tiles
     CountArgs none;
     k_count_pk<<<grid, kPThreads, kPSmem, s>>>(none, d_args, d_n_tiles, 0);
     TFIM_CUDA(cudaGetLastError());
-    return TFIM_OK;
-}
-
-int count_pk_status_fetch(int32_t* pinned, cudaStream_t s) {
-    TFIM_CUDA(cudaMemcpyFromSymbolAsync(pinned, g_pk_status, sizeof(int32_t), 0, cudaMemcpyDeviceToHost, s));
-    return TFIM_OK;
-}
-
-int count_pk_status_check(int32_t v) {
-    if (v) {
-        const int z = 0;
-        TFIM_CUDA(cudaMemcpyToSymbol(g_pk_status, &z, sizeof z));
-    }
-    TFIM_CHECK(v == 0, TFIM_E_TIMEOUT, "tensor-memory family counter: an mbarrier wait expired");
     return TFIM_OK;
 }
 

@@ -2688,10 +2688,16 @@ void finish_mfi_order(MfiSet& M, const uint64_t* key) {
 }  // namespace
 
 namespace {
-int check_search(int32_t error) {
+// A search that a tensor-core counter left with incomplete counts reports that counter's wait.
+int check_search(tfim_ctx* c, int32_t error) {
+    if (error == 0) return TFIM_OK;
+    int32_t status = 0;
+    TFIM_CUDA(cudaMemcpyAsync(&status, c->d_status.p, 4, cudaMemcpyDeviceToHost, c->stream));
+    TFIM_CUDA(cudaStreamSynchronize(c->stream));
+    TFIM_TRY(tensor_status_check(status));
     TFIM_CHECK(error != kErrWait, search_error_status(error), "resident search: a wait of the device loop's grid barrier expired");
-    TFIM_CHECK(error == 0, search_error_status(error), "resident search invariant failed (code %d)", error);
-    return TFIM_OK;
+    set_error("resident search invariant failed (code %d)", error);
+    return search_error_status(error);
 }
 
 int search_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt, bool may_project, bool* projected) {
@@ -2910,6 +2916,7 @@ int search_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt, 
         // this mine's records: status, the top family, the stack's first entry
         const size_t o_top = (sizeof hs + 15) & ~size_t(15), o_stack = o_top + sizeof top;
         TFIM_TRY(R.h_first.reserve(o_stack + 16));
+        TFIM_TRY(c->d_status.reserve(64));
         unsigned char* hf = R.h_first.as<unsigned char>();
         memcpy(hf, &hs, sizeof hs);
         memcpy(hf + o_top, &top, sizeof top);
@@ -2917,6 +2924,7 @@ int search_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt, 
         setup.part[setup.n++] = SetupPart{(const uint4*)hf, (uint4*)R.status.p, (int64_t)o_top / 16};
         setup.part[setup.n++] = SetupPart{(const uint4*)(hf + o_top), (uint4*)R.fams.p, (int64_t)sizeof top / 16};
         setup.part[setup.n++] = SetupPart{(const uint4*)(hf + o_stack), (uint4*)R.stack.p, 1};
+        setup.part[setup.n++] = SetupPart{(const uint4*)(hf + o_stack), (uint4*)c->d_status.p, 1};   // zeros too
         static_assert(sizeof(DFam) % 16 == 0, "a family record is whole 16-byte pieces");
         k_res_setup<<<dim3((unsigned)std::min<size_t>(16, (size_t)n0 / 512 + 1), (unsigned)setup.n), 256, 0, s>>>(setup);
         TFIM_CUDA(cudaGetLastError());
@@ -2927,7 +2935,7 @@ int search_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt, 
     double sync_ms = 0, kernel_ms = 0;
     int64_t launches = 0, count_launches = 0, bytes_alg = 0, waves = 0;
     int64_t path_launches[6] = {0, 0, 0, 0, 0, 0};
-    bool used_tc = false;   // the tcgen05 family counter ran (its error flag is read at the end)
+    bool used_tc = false;   // the tcgen05 family counter ran (its status is read at the end)
     const int64_t row_bytes = (c->n_bits + 7) / 8;
     ResStatus* d_st = (ResStatus*)R.status.p;
 
@@ -3194,7 +3202,7 @@ int search_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt, 
         TFIM_CUDA(cudaMemsetAsync(R.counts.p, 0, (size_t)top_out * 4, s));
         CountArgs a;
         a.bitmap = c->d_bitmap; a.W = W; a.masks = c->d_masks.as<uint32_t>(); a.jobs = P.jobs; a.rows = P.rows;
-        a.cols = P.items; a.out = P.counts;
+        a.cols = P.items; a.out = P.counts; a.status = c->d_status.as<int32_t>();
         stt->setup_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_entry).count();
         TFIM_CUDA(cudaEventRecord(c->ev0, s));
         if (top_mode == 2) {
@@ -3252,7 +3260,7 @@ int search_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt, 
             ha->p.launch_id = ++R.launch_id;
             ha->p.wave_limit = 0x7fffffff;
             CountArgs a;
-            a.vrows = P.vrows; a.n_base = P.n_base; a.pk_list = P.pk_list;
+            a.vrows = P.vrows; a.n_base = P.n_base; a.pk_list = P.pk_list; a.status = c->d_status.as<int32_t>();
             a.bitmap = c->d_bitmap; a.W = W; a.masks = P.masks; a.jobs = P.jobs; a.rows = P.rows;
             a.cols = P.items; a.out = P.counts; a.n_tiles = 0; a.job_list = P.proj_list;
             a.tiles = P.tiles_l3;
@@ -3278,7 +3286,7 @@ int search_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt, 
             const double ts = std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count();
             TFIM_CUDA(cudaStreamSynchronize(s));
             sync_ms += (std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count() - ts) * 1e3;
-            TFIM_TRY(check_search(hst->error));
+            TFIM_TRY(check_search(c, hst->error));
             if (hst->starved || hst->grow) {
                 TFIM_TRY(grow_for(*hst));
                 continue;
@@ -3314,7 +3322,7 @@ int search_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt, 
         const double ts = std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count();
         TFIM_CUDA(cudaStreamSynchronize(s));
         sync_ms += (std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count() - ts) * 1e3;
-        TFIM_TRY(check_search(hst->error));
+        TFIM_TRY(check_search(c, hst->error));
         if (hst->starved || hst->grow) {
             TFIM_TRY(grow_for(*hst));
             continue;
@@ -3323,7 +3331,7 @@ int search_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt, 
         if (hst->jobs == 0) break;
         TFIM_CUDA(cudaMemsetAsync(R.counts.p, 0, (size_t)hst->out_total * 4, s));
         CountArgs a;
-        a.vrows = P.vrows; a.n_base = P.n_base; a.pk_list = P.pk_list;
+        a.vrows = P.vrows; a.n_base = P.n_base; a.pk_list = P.pk_list; a.status = c->d_status.as<int32_t>();
         a.bitmap = c->d_bitmap; a.W = W; a.masks = c->d_masks.as<uint32_t>(); a.jobs = P.jobs; a.rows = P.rows;
         a.cols = P.items; a.out = P.counts; a.job_list = P.proj_list;
         if (hst->tiles_l3) {
@@ -3419,14 +3427,12 @@ int search_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt, 
         TFIM_CUDA(cudaMemcpyAsync(c->la_labels.data(), R.log_label.p, (size_t)fin.log_n * 4, cudaMemcpyDeviceToHost, s));
     }
     const bool used_f4 = top_i8 && top_mode == 1 && !top_loop;
-    TFIM_TRY(c->h_flags.reserve(64));
-    int32_t* flags = c->h_flags.as<int32_t>();
-    flags[0] = flags[1] = 0;
-    if (used_f4) TFIM_TRY(count_f4_status_fetch(flags, s));
-    if (used_tc) TFIM_TRY(count_pk_status_fetch(flags + 1, s));
+    TFIM_TRY(c->h_status.reserve(64));
+    int32_t* status = c->h_status.as<int32_t>();
+    *status = 0;
+    if (used_f4 || used_tc) TFIM_CUDA(cudaMemcpyAsync(status, c->d_status.p, 4, cudaMemcpyDeviceToHost, s));
     TFIM_CUDA(cudaStreamSynchronize(s));
-    TFIM_TRY(count_f4_status_check(flags[0]));
-    TFIM_TRY(count_pk_status_check(flags[1]));
+    TFIM_TRY(tensor_status_check(*status));
     {
         MfiSet& M = c->mfis;
         const bool fresh = M.size() == 0;

@@ -149,6 +149,7 @@ struct CountArgs {
     const uint32_t* const* vrows = nullptr;
     int32_t n_base = 0x7fffffff;
     const int32_t* pk_list = nullptr;   // packed family counter: the jobs of each tile
+    int32_t* status = nullptr;          // tensor-core counters: set when an mbarrier wait expired
     // phase stamps of the launch (or nullptr): the earliest block start and the latest block
     // end, in %globaltimer nanoseconds (phase_begin / phase_end)
     unsigned long long* ph_s = nullptr;
@@ -192,14 +193,12 @@ int launch_count_proj_persistent(const CountArgs* d_args, const int32_t* d_n_job
 int persistent_occupancy(int* lop3, int* b1, int* proj);
 int configure_count_kernels();
 // tcgen05 kind::mxf4 wave counter (count_f4.cu): tiles of up to kF4Cols columns x kF4Rows rows of
-// one job without a base whose rows have one source each.  The device flag the kernel sets when
-// an mbarrier wait expired is copied to pinned memory in stream order and checked (and
-// cleared) once the stream has been waited for anyway.
+// one job without a base whose rows have one source each.  When an mbarrier wait expires, the kernel
+// sets *CountArgs::status, a word of the context that is cleared at the start of a counting wave or
+// mine, copied to pinned memory in stream order and checked by tensor_status_check.
 constexpr int kF4Cols = 128, kF4Rows = 256;
 int launch_count_f4(const CountArgs& a, bool wide, cudaStream_t s);   // wide: what tiles_f4 returned
-int count_f4_status_fetch(int32_t* pinned, cudaStream_t s);
-int count_f4_flag(const int32_t** flag);   // the flag's address on the current device
-int count_f4_status_check(int32_t v);
+int tensor_status_check(int32_t v);
 bool tiles_f4(int32_t job, int32_t nr, int32_t nc, int64_t W, int sms, std::vector<TileDesc>& out, bool upper = false);
 // Packed tcgen05 kind::mxf4 family counter (count_pk.cu): a tile holds the X rows of `nr` jobs of at
 // most kPkMaxCols columns, CountArgs::pk_list[job .. job + nr), of a class of c0 jobs per tile, over
@@ -209,8 +208,6 @@ constexpr int kPkMaxCols = 128;
 constexpr int kPkJobs = 16;         // list entries per tile
 int launch_count_pk(const CountArgs& a, int32_t sms, cudaStream_t s);
 int launch_count_pk_persistent(const CountArgs* d_args, const int32_t* d_n_tiles, int32_t grid, cudaStream_t s);
-int count_pk_status_fetch(int32_t* pinned, cudaStream_t s);
-int count_pk_status_check(int32_t v);
 int configure_pk_kernel();   // opt into its shared memory (once per device, before any capture)
 // CUDA-core Gram counter for dense family jobs (count_gram.cu): a tile is one family job of at
 // most kGramMaxCols columns and at most 128 blocks of 4 x 4 (row, column) pairs, over a word
@@ -233,14 +230,14 @@ constexpr int kProjMaxCols = 1024;  // longest column list the projected counter
 int launch_materialize(const uint32_t* bitmap, int64_t W, uint32_t* masks, const MatDesc* mats,
                        const int32_t* items, int32_t n, cudaStream_t s);
 // The begin of a counting wave: the b prefix masks (masks[i] = AND of node i's items, lists given by
-// descriptors or by offsets) and n_zero zeros in `counts`.
+// descriptors or by offsets), n_zero zeros in `counts` and the status word's zero.
 int launch_wave_begin(const uint32_t* bitmap, int64_t W, uint32_t* masks, const MatDesc* mats, const int64_t* off,
-                      const int32_t* items, int32_t b, int32_t* counts, int64_t n_zero, cudaStream_t s);
+                      const int32_t* items, int32_t b, int32_t* counts, int64_t n_zero, int32_t* status, cudaStream_t s);
 // nfreq[g] = #{c < n_cols : counts[g*n_cols + c] >= min_count} for g < n_rows.  With `out`, pinned host
-// memory takes nfreq (n_rows) and then the counts too; with flag_to, *flag_to = *flag.
+// memory takes nfreq (n_rows) and then the counts too; with status_to, *status_to = *status.
 int launch_nfreq(const int32_t* counts, int64_t n_rows, int32_t n_cols, int32_t min_count,
-                 int32_t* nfreq, cudaStream_t s, int32_t* out = nullptr, const int32_t* flag = nullptr,
-                 int32_t* flag_to = nullptr);
+                 int32_t* nfreq, cudaStream_t s, int32_t* out = nullptr, const int32_t* status = nullptr,
+                 int32_t* status_to = nullptr);
 // For each job row g (global row index over all jobs, row_job[g] = its job):
 // entries >= min_count are appended to `entries` (one atomic reservation per row) and
 // row_info[g] = (start, len).  counter[0] ends as the total entry count.
@@ -314,7 +311,8 @@ struct tfim_ctx {
     bool all_mined = false;
     bool mined = false;
     int32_t counter_pref = TFIM_COUNTER_AUTO;   // counter used by tfim_count_wave
-    tfim::HostBuf h_flags;                      // pinned copies of the tcgen05 counters' device flags
+    tfim::DevBuf d_status;                      // the tcgen05 counters' status word (CountArgs::status),
+    tfim::HostBuf h_status;                     //   and its pinned copy
     tfim_mine_stats last_stats{};
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     tfim::EngineState* engine = nullptr;

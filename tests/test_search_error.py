@@ -24,5 +24,5 @@ def test_status_of_a_failed_search(tmp_path):
     with open(os.path.join(CSRC, "resident.cu")) as f:
         s = f.read()
     # both wave loops report through it, and the barrier's expiry is recorded as such
-    assert s.count("check_search(hst->error)") == 2 and s.count("atomicExch(&st->error, kErrWait)") == 3
+    assert s.count("check_search(c, hst->error)") == 2 and s.count("atomicExch(&st->error, kErrWait)") == 3
     assert "search_error_status(error)" in s
