@@ -257,7 +257,8 @@ typedef struct {
     int32_t proj_auto;     /* resident engine, automatic counter choice may pick the projected
                               counter: -1 tuned default, 0 no, 1 yes */
     int32_t small_pools;   /* resident engine: start from minimal pool capacities so that
-                              every pool grows during the search (exercises the growth path) */
+                              every pool grows during the search, and end every launch of a wave
+                              loop after one wave (exercises growth and continuation) */
     int32_t superset;      /* resident engine: 1 drops a family whose head and whole tail lie
                               inside an MFI already found (none of its itemsets can be a new
                               maximal set), at creation and again before it leaves the stack;

@@ -2993,7 +2993,7 @@ int search_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt, 
         P.row_sum = nullptr;
         P.wave_limit = 0x7fffffff;
         P.launch_id = 0;
-        P.max_launch_ns = 2000000000ull;
+        P.max_launch_ns = small ? 1000ull : 2000000000ull;   // small_pools: every launch ends after one wave
         P.sup_index = sup_on ? (uint32_t*)R.sup_index.p : nullptr;
         P.sup_words = sup_words;
         P.sup_items = d;
