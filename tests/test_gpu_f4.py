@@ -43,3 +43,38 @@ def test_full_accumulators(n_bits):
     with tf.Database.from_bitmap(rows, n_bits, d) as db:
         counts, nfreq = db.count_wave([[i, 2 * i] for i in range(b)], n_bits, counter="i8")
     assert (counts == n_bits).all() and (nfreq == d).all()
+
+
+def _slice_words(nodes, items, words, sms=148):
+    """The words of a tile of the wave counter (tiles_f4), restated."""
+    groups = -(-nodes // 256)
+    step = (-(-nodes // groups) + 15) & ~15
+    base = -(-nodes // step) * -(-items // 128)
+    blocks = words // 64
+    best = None
+    for ks in range(1, min(blocks, max(1, 4 * sms // base) + (words >> 18) + 1) + 1):
+        per = -(-blocks // ks)
+        if per * 64 <= 1 << 18:
+            cost = -(-base * -(-blocks // per) // sms) * (per * 4 + 16)
+            if best is None or cost < best[0]:
+                best = cost, per
+    return best[1] * 64
+
+
+def test_longest_slice():
+    """37 row groups x 4 column tiles fill the 148 SMs once, so a tile takes all of 2^23 transactions:
+    its FP32 sums reach 2^23.  Items hold every transaction but some of the first 4,096."""
+    n, d, b = 1 << 23, 512, 37 * 256
+    assert _slice_words(b, d, n // 32) == n // 32
+    rng = np.random.Generator(np.random.PCG64(3))
+    head = rng.random((d, 4096)) < rng.random((d, 1))
+    head[:3] = True
+    rows = np.full((d, n // 32), 0xFFFFFFFF, np.uint32)
+    rows[:, :128] = np.packbits(head, axis=1, bitorder="little").view(np.uint32)
+    lists = [[k % d, (k * 7 + k // d) % d] for k in range(b)]
+    both = np.array([head[i] & head[j] for i, j in lists], np.float32)
+    expected = (both @ head.T.astype(np.float32)).astype(np.int64) + n - 4096
+    with tf.Database.from_bitmap(rows, n, d) as db:
+        counts, nfreq = db.count_wave(lists, n, counter="i8")
+    assert (counts == expected).all() and (nfreq == (expected >= n).sum(1)).all()
+    assert counts.max() == n
