@@ -65,6 +65,7 @@ struct B1Shared {
 };
 
 // Block: 256 threads (8 warps as 2 x 4; each warp owns 32 rows x 16 columns).
+template <bool V>
 __device__ void b1_tile(const CountArgs& a, const TileDesc t, unsigned char* smem, B1Shared& sh) {
     const uint32_t** row_src = sh.row_src;
     const uint32_t** col_src = sh.col_src;
@@ -78,7 +79,7 @@ __device__ void b1_tile(const CountArgs& a, const TileDesc t, unsigned char* sme
         if (r < t.nr) {
             const RowDesc rd = a.rows[j.row_off + t.r0 + r];
             if (rd.slot >= 0) { row_src[r] = a.masks + (int64_t)rd.slot * W; row_kind[r] = 0; }
-            else if (rd.item >= 0) { row_src[r] = item_row(a, rd.item); row_kind[r] = 0; }
+            else if (rd.item >= 0) { row_src[r] = item_row<V>(a, rd.item); row_kind[r] = 0; }
             else { row_src[r] = nullptr; row_kind[r] = 1; }
         } else {
             row_src[r] = nullptr;
@@ -88,7 +89,7 @@ __device__ void b1_tile(const CountArgs& a, const TileDesc t, unsigned char* sme
         const int c = tid - 64;
         if (t.c0 + c < t.c1) {
             const int32_t col = (t.c0 + c) == j.self_col ? -1 : a.cols[j.col_off + t.c0 + c];
-            if (col >= 0) { col_src[c] = item_row(a, col); col_kind[c] = 0; }
+            if (col >= 0) { col_src[c] = item_row<V>(a, col); col_kind[c] = 0; }
             else { col_src[c] = nullptr; col_kind[c] = 1; }
         } else {
             col_src[c] = nullptr;
@@ -96,7 +97,7 @@ __device__ void b1_tile(const CountArgs& a, const TileDesc t, unsigned char* sme
         }
     }
     const uint32_t* base_m = j.base_slot >= 0 ? a.masks + (int64_t)j.base_slot * W : nullptr;
-    const uint32_t* base_i = j.base_item >= 0 ? item_row(a, j.base_item) : nullptr;
+    const uint32_t* base_i = j.base_item >= 0 ? item_row<V>(a, j.base_item) : nullptr;
     const bool has_base = base_m || base_i;
     __syncthreads();
 
@@ -207,11 +208,12 @@ __device__ void b1_tile(const CountArgs& a, const TileDesc t, unsigned char* sme
     __syncthreads();   // the block's next tile reuses the staging and the source tables
 }
 
+template <bool V>
 __global__ void __launch_bounds__(256) k_count_b1(CountArgs a) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ B1Shared sh;
     phase_begin(a.ph_s);
-    b1_tile(a, a.tiles[blockIdx.x], smem, sh);
+    b1_tile<V>(a, a.tiles[blockIdx.x], smem, sh);
     phase_end(a.ph_e);
 }
 
@@ -229,7 +231,7 @@ __global__ void __launch_bounds__(256) k_count_b1_persistent(const CountArgs* __
         const int32_t t = s_t;
         __syncthreads();
         if (t >= n) break;
-        b1_tile(a, a.tiles[t], smem, sh);
+        b1_tile<true>(a, a.tiles[t], smem, sh);
     }
     phase_end(a.ph_e);
 }
@@ -243,7 +245,8 @@ int configure_count_kernels() {
     TFIM_CUDA(cudaGetDevice(&dev));
     if (dev >= 0 && dev < 64 && done[dev].load()) return TFIM_OK;
     const size_t smem = (size_t)kStages * kStageBytes;
-    TFIM_CUDA(cudaFuncSetAttribute(k_count_b1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    TFIM_CUDA(cudaFuncSetAttribute(k_count_b1<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    TFIM_CUDA(cudaFuncSetAttribute(k_count_b1<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     TFIM_CUDA(cudaFuncSetAttribute(k_count_b1_persistent, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     if (dev >= 0 && dev < 64) done[dev].store(true);
     return TFIM_OK;
@@ -253,7 +256,8 @@ int launch_count_b1(const CountArgs& a, cudaStream_t s) {
     if (a.n_tiles <= 0) return TFIM_OK;
     TFIM_TRY(configure_count_kernels());
     const size_t smem = (size_t)kStages * kStageBytes;
-    k_count_b1<<<a.n_tiles, 256, smem, s>>>(a);
+    if (a.vrows) k_count_b1<true><<<a.n_tiles, 256, smem, s>>>(a);
+    else k_count_b1<false><<<a.n_tiles, 256, smem, s>>>(a);
     TFIM_CUDA(cudaGetLastError());
     return TFIM_OK;
 }

@@ -43,7 +43,7 @@ struct Lop3Shared {
 
 __device__ __forceinline__ bool nonzero4(uint4 v) { return (v.x | v.y | v.z | v.w) != 0u; }
 
-template <bool WIDE>
+template <bool WIDE, bool V>
 __device__ void lop3_tile_impl(const CountArgs& a, const TileDesc t, Lop3Shared& sh) {
     const JobDesc j = a.jobs[t.job];
     const int64_t W = a.W;
@@ -53,11 +53,11 @@ __device__ void lop3_tile_impl(const CountArgs& a, const TileDesc t, Lop3Shared&
     if (tid < kLop3Rows && tid < nr) {
         const RowDesc rd = a.rows[j.row_off + t.r0 + tid];
         sh.rsrc[tid][0] = rd.slot >= 0 ? reinterpret_cast<const uint4*>(a.masks + (int64_t)rd.slot * W) : nullptr;
-        sh.rsrc[tid][1] = rd.item >= 0 ? reinterpret_cast<const uint4*>(item_row(a, rd.item)) : nullptr;
+        sh.rsrc[tid][1] = rd.item >= 0 ? reinterpret_cast<const uint4*>(item_row<V>(a, rd.item)) : nullptr;
     }
     for (int q = tid; q < kLop3Rows * 64; q += blockDim.x) sh.acc[q] = 0;
     const uint4* base_m = j.base_slot >= 0 ? reinterpret_cast<const uint4*>(a.masks + (int64_t)j.base_slot * W) : nullptr;
-    const uint4* base_i = j.base_item >= 0 ? reinterpret_cast<const uint4*>(item_row(a, j.base_item)) : nullptr;
+    const uint4* base_i = j.base_item >= 0 ? reinterpret_cast<const uint4*>(item_row<V>(a, j.base_item)) : nullptr;
     // flush layout: G staged positions per pass, lane -> (position offset, column(s))
     constexpr bool wide = WIDE;
     constexpr int NC = WIDE ? 2 : 1;   // columns per lane
@@ -77,7 +77,7 @@ __device__ void lop3_tile_impl(const CountArgs& a, const TileDesc t, Lop3Shared&
             if (col < 0) ck[ci] = 1;   // the all-ones column
             else {
                 ck[ci] = 0;
-                cp[ci] = reinterpret_cast<const uint4*>(item_row(a, col));
+                cp[ci] = reinterpret_cast<const uint4*>(item_row<V>(a, col));
             }
         }
     }
@@ -201,7 +201,7 @@ __device__ void lop3_tile_impl(const CountArgs& a, const TileDesc t, Lop3Shared&
 // columns straight from L2 (16-byte loads, consecutive positions on consecutive lanes) and
 // adds BR x BC popcounts held in registers -- (2 + BR + BC) loads per BR * BC popc4 instead of
 // about 1 + nr per nr.  The G threads of a block meet in shared memory at the end, as above.
-template <int BR>
+template <int BR, bool V>
 __device__ void lop3_dense_impl(const CountArgs& a, const TileDesc t, int32_t* sacc) {
     constexpr int BC = BR == 1 ? 16 : BR == 2 ? 8 : BR == 3 ? 5 : 4;
     const JobDesc j = a.jobs[t.job];
@@ -215,7 +215,7 @@ __device__ void lop3_dense_impl(const CountArgs& a, const TileDesc t, int32_t* s
     const int br = busy ? (b / cb) * BR : 0, bc = busy ? (b % cb) * BC : 0;
     for (int q = tid; q < kLop3Rows * 64; q += blockDim.x) sacc[q] = 0;
     const uint4* base_m = j.base_slot >= 0 ? reinterpret_cast<const uint4*>(a.masks + (int64_t)j.base_slot * W) : nullptr;
-    const uint4* base_i = j.base_item >= 0 ? reinterpret_cast<const uint4*>(item_row(a, j.base_item)) : nullptr;
+    const uint4* base_i = j.base_item >= 0 ? reinterpret_cast<const uint4*>(item_row<V>(a, j.base_item)) : nullptr;
     // sources of the block's rows and columns, clamped to the tile's last row / column (pairs
     // outside the tile are computed on valid rows and discarded); a null source is all ones
     const uint4* rsl[BR];
@@ -225,13 +225,13 @@ __device__ void lop3_dense_impl(const CountArgs& a, const TileDesc t, int32_t* s
     for (int x = 0; x < BR; x++) {
         const RowDesc rd = a.rows[j.row_off + t.r0 + min(br + x, nr - 1)];
         rsl[x] = rd.slot >= 0 ? reinterpret_cast<const uint4*>(a.masks + (int64_t)rd.slot * W) : nullptr;
-        rit[x] = rd.item >= 0 ? reinterpret_cast<const uint4*>(item_row(a, rd.item)) : nullptr;
+        rit[x] = rd.item >= 0 ? reinterpret_cast<const uint4*>(item_row<V>(a, rd.item)) : nullptr;
     }
 #pragma unroll
     for (int y = 0; y < BC; y++) {
         const int c = t.c0 + min(bc + y, nc - 1);
         const int32_t col = c == j.self_col ? -1 : a.cols[j.col_off + c];
-        csrc[y] = col >= 0 ? reinterpret_cast<const uint4*>(item_row(a, col)) : nullptr;
+        csrc[y] = col >= 0 ? reinterpret_cast<const uint4*>(item_row<V>(a, col)) : nullptr;
     }
     uint32_t acc[BR][BC];
 #pragma unroll
@@ -277,37 +277,40 @@ __device__ void lop3_dense_impl(const CountArgs& a, const TileDesc t, int32_t* s
 }
 
 // Row blocks by the tile's rows: 1, 2, 3 (also 5, 6 as two blocks) or 4 (also 7, 8).
+template <bool V>
 __device__ __forceinline__ void lop3_dense_tile(const CountArgs& a, const TileDesc t, int32_t* sacc) {
     switch (t.nr) {
-        case 1: lop3_dense_impl<1>(a, t, sacc); break;
-        case 2: lop3_dense_impl<2>(a, t, sacc); break;
-        case 3: case 5: case 6: lop3_dense_impl<3>(a, t, sacc); break;
-        default: lop3_dense_impl<4>(a, t, sacc); break;
+        case 1: lop3_dense_impl<1, V>(a, t, sacc); break;
+        case 2: lop3_dense_impl<2, V>(a, t, sacc); break;
+        case 3: case 5: case 6: lop3_dense_impl<3, V>(a, t, sacc); break;
+        default: lop3_dense_impl<4, V>(a, t, sacc); break;
     }
 }
 
 // Tiles of more than 32 columns give each lane two columns.  DENSE: the launch may hold
 // dense tiles too (the persistent form); the plain launches hold one kind each.
-template <bool DENSE>
+template <bool DENSE, bool V>
 __device__ __forceinline__ void lop3_tile(const CountArgs& a, const TileDesc t, Lop3Shared& sh) {
-    if (DENSE && (t.pad & 1)) lop3_dense_tile(a, t, sh.acc);
-    else if (t.c1 - t.c0 > 32) lop3_tile_impl<true>(a, t, sh);
-    else lop3_tile_impl<false>(a, t, sh);
+    if (DENSE && (t.pad & 1)) lop3_dense_tile<V>(a, t, sh.acc);
+    else if (t.c1 - t.c0 > 32) lop3_tile_impl<true, V>(a, t, sh);
+    else lop3_tile_impl<false, V>(a, t, sh);
 }
 
+template <bool V>
 __global__ void __launch_bounds__(256, 4) k_count_lop3(CountArgs a) {
     __shared__ Lop3Shared sh;
     phase_begin(a.ph_s);
-    lop3_tile<false>(a, a.tiles[blockIdx.x], sh);
+    lop3_tile<false, V>(a, a.tiles[blockIdx.x], sh);
     phase_end(a.ph_e);
 }
 
 // Dense tiles only (a separate launch, so that the register budget of the skipping tiles
 // above stays as it is).
+template <bool V>
 __global__ void __launch_bounds__(256, 4) k_count_lop3_dense(CountArgs a) {
     __shared__ int32_t sacc[kLop3Rows * 64];
     phase_begin(a.ph_s);
-    lop3_dense_tile(a, a.tiles[blockIdx.x], sacc);
+    lop3_dense_tile<V>(a, a.tiles[blockIdx.x], sacc);
     phase_end(a.ph_e);
 }
 
@@ -327,7 +330,7 @@ __global__ void __launch_bounds__(256, 4) k_count_lop3_persistent(const CountArg
         const int32_t t = s_t;
         __syncthreads();
         if (t >= n) break;
-        lop3_tile<true>(a, a.tiles[t], sh);
+        lop3_tile<true, true>(a, a.tiles[t], sh);
     }
     phase_end(a.ph_e);
 }
@@ -448,14 +451,16 @@ __global__ void k_compact(const int32_t* __restrict__ counts, const JobDesc* __r
 
 int launch_count_lop3(const CountArgs& a, cudaStream_t s) {
     if (a.n_tiles <= 0) return TFIM_OK;
-    k_count_lop3<<<a.n_tiles, 256, 0, s>>>(a);
+    if (a.vrows) k_count_lop3<true><<<a.n_tiles, 256, 0, s>>>(a);
+    else k_count_lop3<false><<<a.n_tiles, 256, 0, s>>>(a);
     TFIM_CUDA(cudaGetLastError());
     return TFIM_OK;
 }
 
 int launch_count_lop3_dense(const CountArgs& a, cudaStream_t s) {
     if (a.n_tiles <= 0) return TFIM_OK;
-    k_count_lop3_dense<<<a.n_tiles, 256, 0, s>>>(a);
+    if (a.vrows) k_count_lop3_dense<true><<<a.n_tiles, 256, 0, s>>>(a);
+    else k_count_lop3_dense<false><<<a.n_tiles, 256, 0, s>>>(a);
     TFIM_CUDA(cudaGetLastError());
     return TFIM_OK;
 }

@@ -3331,7 +3331,8 @@ int search_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt, 
         if (hst->jobs == 0) break;
         TFIM_CUDA(cudaMemsetAsync(R.counts.p, 0, (size_t)hst->out_total * 4, s));
         CountArgs a;
-        a.vrows = P.vrows; a.n_base = P.n_base; a.pk_list = P.pk_list; a.status = c->d_status.as<int32_t>();
+        if (*projected) a.vrows = P.vrows, a.n_base = P.n_base;
+        a.pk_list = P.pk_list; a.status = c->d_status.as<int32_t>();
         a.bitmap = c->d_bitmap; a.W = W; a.masks = c->d_masks.as<uint32_t>(); a.jobs = P.jobs; a.rows = P.rows;
         a.cols = P.items; a.out = P.counts; a.job_list = P.proj_list;
         if (hst->tiles_l3) {
@@ -3519,6 +3520,7 @@ int mine_resident(tfim_ctx* c, const tfim_mine_opts* o, tfim_mine_stats* stt) {
         dev_trim(c->device);
         c->mfis.clear();
         *stt = before;
+        projected = false;
         rc = search_resident(c, o, stt, false, &projected);
     }
     return rc;
