@@ -285,7 +285,8 @@ typedef struct {
     double  host_ms;           /* host time spent building waves and processing results */
     double  sync_ms;           /* host time blocked on device results */
     int64_t lookaheads_skipped;/* lookaheads ruled out because a tail pair is infrequent */
-    double  top_ms;            /* CUDA-event time of counting the empty-prefix family (resident) */
+    double  top_ms;            /* CUDA-event time of counting the empty-prefix family (resident; 0
+                                  when the device loop counts it with the other waves) */
     int64_t pruned_superset;   /* families dropped by the superset check (resident) */
     /* per counting path (index TFIM_PATH_*): device time of its launches, algorithmic bytes
        (every operand row read once as a dense row, every count written once), bit-ops

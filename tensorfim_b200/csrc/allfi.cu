@@ -6,7 +6,7 @@
 // and the extensions j > its last item with support >= minsup are the frequent k-itemsets
 // (canonical extension, each itemset generated once).  This is the same search on the
 // library's counting pipeline: prefix masks from the item lists, the automatically chosen
-// counter (LOP3 / b1 / tcgen05 kind::i8), and a device-side compaction that returns only the
+// counter (LOP3 / b1 / tcgen05 kind::mxf4), and a device-side compaction that returns only the
 // frequent extensions of each prefix.
 #include <algorithm>
 #include <chrono>

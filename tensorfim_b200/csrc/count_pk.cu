@@ -21,7 +21,7 @@
 // memory, the loads return 1 KiB and the MMA reads 4 KiB and the window, about 110 cycles of the
 // shared-memory pipe whatever the number of tail rows (128 measured), while AND + popc spends
 // rows x columns / 8 cycles: the two meet near eight tail rows per job.  Measured on the
-// 6.3M-row dense database (267 items, minsup 6%): the families this kernel takes need 10.6 ms
+// 6.3M-row dense database (267 items, minsup 6%): the families this kernel takes need 10.3 ms
 // of a mine; the byte-expanding kind::i8 tiles of one family each that it replaces and the
 // CUDA-core tiles needed 16.9 ms for the same.
 //

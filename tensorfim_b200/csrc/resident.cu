@@ -256,9 +256,9 @@ constexpr int kPkMinRows = 8, kPkMinWords = 1024;
 // than they save (a 1M-row sparse mine 1.69 / 1.72 ms with its one packed wave on the CUDA cores /
 // packed; a 49,000-row dense one 2.62 / 2.56 ms with its waves below 2e8 / 5e7 on the CUDA cores).
 constexpr float kPkMinWork = 1e8f;
-// Narrow dense families of short rows stay with the Gram counter: 49,000 / 98,000 / 196,000 rows of
-// the dense database mine in 2.57 / 3.27 / 3.50 ms with it and 2.56 / 3.25 / 3.49 ms with their jobs in
-// packed tiles, the same within a launch.
+// Narrow dense families of short rows stay with the Gram counter.  It neither gains nor costs much: 49,000 /
+// 98,000 / 196,000 rows of the dense database mine in 2.28 / 2.93 / 2.89 ms with it and in 2.26 / 2.90 / 2.87 ms
+// with their jobs in packed tiles or CUDA-core tiles.
 constexpr int kGramMaxWords = 4096;
 
 constexpr int kPackThreads = 1024;
@@ -292,9 +292,9 @@ __device__ __forceinline__ int pk_class(int cols) {
 __device__ __forceinline__ int pk_per(int cls) { return cls <= 3 ? 16 / (cls + 1) : cls == 4 ? 3 : cls == 5 ? 2 : 1; }
 
 // The CUDA-core Gram counter takes a dense family job of at most kGramMaxCols columns (and at
-// most 128 blocks of 4 x 4 pairs) that the packed tiles leave: a dense prefix has no zero word for the general tiles to
-// skip, and at these widths the register-tiled Gram block (86-91% of the POPC ceiling at 32
-// and 64 columns) beats the tensor tiles, whose narrow MMAs cost about 50 cycles each.
+// most 128 blocks of 4 x 4 pairs) over rows of fewer than kGramMaxWords words: a dense prefix has no
+// zero word for the general tiles to skip, and the columns are read once per job instead of once per
+// eight rows.
 __device__ __forceinline__ bool use_gram(const ResPtrs& p, const JobDesc& jd, int32_t sup, int32_t n) {
     // tails of 1 or 2 rows are memory-bound in any kernel (8 bit-ops per byte and row); the
     // general tiles handle them as well, and measured faster on the dense benchmark
@@ -1604,8 +1604,12 @@ __global__ void __launch_bounds__(256) k_top_finish(int32_t* __restrict__ M, int
 // base, over sup(t) instead of N transactions.  Supports do not change.  It pays from a few tail
 // rows on: a family reads its rows again for every one of them.
 // Measured on the 6.3M-row dense database (267 items, minsup 6%): counting of the later waves
-// 62 -> 25 ms, masks 1.8 -> 0.6 ms, compression 2.4 ms; the mine 64.8 -> 29.7 ms.  Lines at
+// 62 -> 25 ms and masks 1.8 -> 0.6 ms, for 2.2 ms of compression.  Lines at
 // 3/4 and 19/20 of N instead of 1/2 moved the mine by less than its noise, as did 2 tail rows.
+// The plan is made once, after the first wave, and leaves out the families that wait on a lookahead then
+// (state 1): these and their subtrees count over all transactions.  With the learned proposal they are
+// few (72 lookaheads in all at 12.5M rows, 42 ms a mine), with the tail-pair filter alone
+// many (3,321, 100 ms).
 constexpr int kProjMinTail = 4;        // tail rows from which a family is projected
 constexpr int kProjTile = 64;          // words of a row per tile; rows are padded to this
 constexpr int kProjGroups = 13;        // most groups of 32 items in a transposed chunk (odd)
@@ -2051,8 +2055,8 @@ __global__ void __launch_bounds__(256) k_res_setup(SetupParts s) {   // blockIdx
 // and a host wait, 85 us.  This kernel runs such waves back to back with its whole grid resident
 // (cooperative launch): block 0 packs, then all blocks count, expand and build masks, with a grid
 // barrier after each.  A wave of more than kLoopMaxWork, and one that needs larger pools, is left
-// to the host.  Measured: 10,000-row dense mine 0.70 -> 0.43 ms (31 us a wave), 2M-row one 0.43 ->
-// 0.31 ms, 500,000 rows at 82% 0.53 -> 0.33 ms.
+// to the host.  Measured, a call: 10,000-row dense mine 0.70 -> 0.48 ms (31 us a wave), 2M-row one 0.45 ->
+// 0.35 ms.
 constexpr int kLoopThreads = 512;
 constexpr int kLoopMaxWords = 4096;     // rows of the databases that take it;
 constexpr int kLoopDenseWords = 1 << 16; // of dense ones (minimum support at least 1/64 of the transactions)
